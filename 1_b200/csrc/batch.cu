@@ -16,62 +16,15 @@
 #include <string.h>
 #include <vector>
 
-#include "fft_fixed_kernels.cuh"
+#include "fx_dispatch.cuh"
 #include "solver_state.cuh"
 
-__device__ __forceinline__ int find_seg(const int* __restrict__ starts, int nseg, int b) {
-  int lo = 0, hi = nseg - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (__ldg(&starts[mid]) <= b) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
-
-struct BCol {
-  const float2* src;
-  float2* dst;
-  ColPass cp;
-};
-struct BZr2c {
-  const float* src;
-  float2* dst;
-  ZPass z;
-  ZComb cb;
-  int vec2;
-};
 struct BFin {
   float* m;
   const float* mnew;
   int64_t n;
 };
 
-template <int L, int TK, int T, bool INV, bool HALF>
-__global__ void __launch_bounds__(T) kb_col(const BCol* __restrict__ a, const int* __restrict__ starts, int nseg) {
-  int s = find_seg(starts, nseg, blockIdx.x);
-  int t = blockIdx.x - starts[s];
-  const BCol& c = a[s];
-  col_body<L, TK, T, INV, HALF>(c.src, c.dst, c.cp, t);
-}
-template <int L, int TK, int T, bool D2, bool HALF>
-__global__ void __launch_bounds__(T) kb_conv(const ConvArgs* __restrict__ a, const int* __restrict__ starts,
-                                             int nseg) {
-  int s = find_seg(starts, nseg, blockIdx.x);
-  conv_body<L, TK, T, D2, HALF>(a[s], blockIdx.x - starts[s]);
-}
-template <int M, int RT, int T, bool COMB>
-__global__ void __launch_bounds__(T) kb_zr2c(const BZr2c* __restrict__ a, const int* __restrict__ starts, int nseg) {
-  int s = find_seg(starts, nseg, blockIdx.x);
-  const BZr2c& c = a[s];
-  zr2c_body<M, RT, T, COMB>(c.src, c.dst, c.z, c.cb, c.vec2, blockIdx.x - starts[s]);
-}
-template <int M, int RT, int T, int MODE>
-__global__ void __launch_bounds__(T) kb_zinv(const ZinvArgs* __restrict__ a, const int* __restrict__ starts,
-                                             int nseg) {
-  int s = find_seg(starts, nseg, blockIdx.x);
-  zinv_body<M, RT, T, MODE>(a[s], blockIdx.x - starts[s]);
-}
 // m <- normalize(m_new) for every instance (rk.go:444)
 __global__ void kb_finalize(const BFin* __restrict__ a, const int* __restrict__ starts, int nseg) {
   int s = find_seg(starts, nseg, blockIdx.x);
@@ -95,7 +48,7 @@ struct Launch {
   void* args;     // device array of per-instance argument structs
   int* starts;    // device array of tile offsets
   int variant = 0;  // tile shape (column passes: 0 = fx_col_tk, 1 = col_tk_alt)
-  int half = 0;     // column passes: every instance's data fill half the line
+  int half = 0;     // column and convolution passes: every instance's data fill half the line
   std::vector<int> inst;  // instances this launch reads or writes (graph dependencies)
   size_t args_off = 0, starts_off = 0;  // offsets into the batch's table block
 };
@@ -133,131 +86,24 @@ __global__ void kb_clear(float** p, int n) {
   if (i < n) *p[i] = 0.f;
 }
 
-// ---------------------------------------------------------------------
-// launch dispatch over the compiled line lengths
-// ---------------------------------------------------------------------
-template <typename K>
-static void set_smem(K kern, size_t bytes) {
-  if (bytes > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
-// The autotuner's alternative column-tile width: half the default where
-// that leaves >= 8 columns (more, smaller blocks), else double (fewer,
-// larger blocks).
-__host__ __device__ constexpr int col_tk_alt(int L) { return fx_col_tk(L) >= 16 ? fx_col_tk(L) / 2 : 2 * fx_col_tk(L); }
-__host__ __device__ constexpr int col_tk_variant(int L, int v) { return v ? col_tk_alt(L) : fx_col_tk(L); }
-
-template <int L, int TK>
-static cudaError_t run_col_tk(const Launch& l, cudaStream_t st) {
-  constexpr int T = fx_threads(TK * L);
-  size_t smem = sizeof(float2) * (size_t)odd_pitch(TK) * L;
-#define KB_COL_(INV, HALF)                                                                        \
-  set_smem(kb_col<L, TK, T, INV, HALF>, smem);                                                    \
-  kb_col<L, TK, T, INV, HALF><<<l.blocks, T, smem, st>>>((const BCol*)l.args, l.starts, l.nseg);
-  if (l.flag) {
-    if (l.half) { KB_COL_(true, true) } else { KB_COL_(true, false) }
-  } else {
-    if (l.half) { KB_COL_(false, true) } else { KB_COL_(false, false) }
-  }
-#undef KB_COL_
-  return cudaGetLastError();
-}
-template <int L>
-static cudaError_t run_col(const Launch& l, cudaStream_t st) {
-  return l.variant ? run_col_tk<L, col_tk_alt(L)>(l, st) : run_col_tk<L, fx_col_tk(L)>(l, st);
-}
-template <int L>
-static int conv_tk() {
-  return conv_tkp_narrow(L);
-}
-template <int L>
-static cudaError_t run_conv(const Launch& l, cudaStream_t st) {
-  constexpr int TKP = conv_tkp_narrow(L);
-  constexpr int NBF = TKP * (L / fwd_radix(L, n_stages(L) - 1));
-  constexpr int T = NBF < 64 ? 64 : (NBF > 512 ? 512 : ((NBF + 31) / 32) * 32);
-  size_t smem = conv_smem_tk(L, TKP);
-  // variant 1: every instance of the launch has its data in the lower half
-#define KB_CONV_(D2, HALF)                                                                              \
-  set_smem(kb_conv<L, TKP, T, D2, HALF>, smem);                                                         \
-  kb_conv<L, TKP, T, D2, HALF><<<l.blocks, T, smem, st>>>((const ConvArgs*)l.args, l.starts, l.nseg);
-  if (l.flag) {
-    if (l.variant) { KB_CONV_(true, true) } else { KB_CONV_(true, false) }
-  } else {
-    if (l.variant) { KB_CONV_(false, true) } else { KB_CONV_(false, false) }
-  }
-#undef KB_CONV_
-  return cudaGetLastError();
-}
-template <int M>
-static cudaError_t run_zr2c(const Launch& l, cudaStream_t st) {
-  constexpr int RT = fx_rows(M, 1);
-  constexpr int T = fx_threads(RT * M);
-  size_t smem = sizeof(float2) * (size_t)RT * row_pitch(M);
-  if (l.flag) {
-    set_smem(kb_zr2c<M, RT, T, true>, smem);
-    kb_zr2c<M, RT, T, true><<<l.blocks, T, smem, st>>>((const BZr2c*)l.args, l.starts, l.nseg);
-  } else {
-    set_smem(kb_zr2c<M, RT, T, false>, smem);
-    kb_zr2c<M, RT, T, false><<<l.blocks, T, smem, st>>>((const BZr2c*)l.args, l.starts, l.nseg);
-  }
-  return cudaGetLastError();
-}
-template <int M, int MODE>
-static cudaError_t run_zinv_mode(const Launch& l, cudaStream_t st) {
-  constexpr int RT = fx_rows(M, 3);
-  constexpr int T = fx_threads(3 * RT * M);
-  size_t smem = sizeof(float2) * (size_t)3 * RT * row_pitch(M);
-  set_smem(kb_zinv<M, RT, T, MODE>, smem);
-  kb_zinv<M, RT, T, MODE><<<l.blocks, T, smem, st>>>((const ZinvArgs*)l.args, l.starts, l.nseg);
-  return cudaGetLastError();
-}
-template <int M>
-static cudaError_t run_zinv(const Launch& l, cudaStream_t st) {
-  switch (l.flag) {
-    case EPI_HEUN1: return run_zinv_mode<M, EPI_HEUN1>(l, st);
-    case EPI_HEUN2: return run_zinv_mode<M, EPI_HEUN2>(l, st);
-    case EPI_TORQUE: return run_zinv_mode<M, EPI_TORQUE>(l, st);
-    default: return run_zinv_mode<M, EPI_RK>(l, st);
-  }
-}
-
 static cudaError_t run_launch(const Launch& l, cudaStream_t st) {
+  BatchLaunch b;
+  b.L = l.L;
+  b.nseg = l.nseg;
+  b.blocks = l.blocks;
+  b.half = l.half;
+  b.variant = l.variant;
+  b.flag = l.flag;
+  b.args = l.args;
+  b.starts = l.starts;
   switch (l.kind) {
     case L_FIN:
       kb_finalize<<<l.blocks, 256, 0, st>>>((const BFin*)l.args, l.starts, l.nseg);
       return cudaGetLastError();
-    case L_COL:
-      switch (l.L) {
-#define C_(LL) \
-  case LL: return run_col<LL>(l, st);
-        FX_SIZES(C_)
-#undef C_
-      }
-      break;
-    case L_CONV:
-      switch (l.L) {
-#define C_(LL) \
-  case LL: return run_conv<LL>(l, st);
-        FX_SIZES(C_)
-#undef C_
-      }
-      break;
-    case L_ZR2C:
-      switch (l.L) {
-#define C_(LL) \
-  case LL: return run_zr2c<LL>(l, st);
-        FX_SIZES(C_)
-#undef C_
-      }
-      break;
-    case L_ZINV:
-      switch (l.L) {
-#define C_(LL) \
-  case LL: return run_zinv<LL>(l, st);
-        FX_SIZES(C_)
-#undef C_
-      }
-      break;
+    case L_COL: return bx_col(b, st);
+    case L_CONV: return l.flag ? bx_conv_1(b, st) : bx_conv_0(b, st);
+    case L_ZR2C: return bx_zr2c(b, st);
+    case L_ZINV: return bx_zinv(l.flag, b, false, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -360,7 +206,7 @@ static int conv_tiles(int L, int ncols) {
   int tk = 1;
   switch (L) {
 #define C_(LL) \
-  case LL: tk = conv_tk<LL>(); break;
+  case LL: tk = conv_tkp_narrow(LL); break;
     FX_SIZES(C_)
 #undef C_
   }
@@ -579,7 +425,7 @@ static int build_eval(mmx_batch* b, std::vector<Launch>& out, int mode, bool com
       out.back().inst = g.second;
       bool half = true;
       for (const ConvArgs& c : a) half = half && 2 * c.n_data == g.first;
-      out.back().variant = half ? 1 : 0;
+      out.back().half = half ? 1 : 0;
     }
   }
   // Y inverse (3D)
@@ -689,30 +535,18 @@ static int batch_build(mmx_batch* b) {
         ea.dtg = f32_div(1.f, f32_add(1.f, f32_mul(s->p.alpha, s->p.alpha)));
         ea.m_in = st == 0 ? s->m : s->m1;
         ea.dt_dev = s->scratch + 2;
-        for (int j = 0; j < s->stages; j++) ea.kbuf[j] = s->kb[j];
-        ea.stage = st;
         ea.out0 = s->kb[st];
         if (st == 0) ea.err = s->scratch + 1;  // max |k0|, the torque the relax loop stops on
         if (st == 3) {
           ea.aux0 = s->m;
           ea.out1 = s->mnew;
-          ea.rk.nk = s->stages;
-          for (int j = 0; j < s->stages; j++) ea.rk.a[j] = s->b[j];
-          ea.rk.final_stage = 1;
-          ea.rk.adaptive = 0;
+          ea.rk = solver_rk_final(s);
         }
         return ea;
       };
       auto comb = [&](int i) {
         mmx_solver* s = b->inst[i];
-        ZComb c;
-        memset(&c, 0, sizeof(c));
-        c.m0 = s->m;
-        for (int j = 0; j < s->stages; j++) { c.k[j] = s->kb[j]; c.a[j] = s->a[st][j]; }
-        c.nk = s->stages;
-        c.dt = s->scratch + 2;
-        c.out = s->m1;
-        return c;
+        return solver_rk_comb(s, st, s->scratch + 2);
       };
       auto src_m = [&](int i) { return (const float*)b->inst[i]->m; };
       rc = build_eval(b, b->stage[st], st == 3 ? EPI_RK : EPI_TORQUE, st > 0, epi, comb, src_m);

@@ -11,12 +11,18 @@ enum { EPI_FIELD = 0, EPI_HEUN1 = 1, EPI_HEUN2 = 2, EPI_TORQUE = 3, EPI_RK = 4, 
 __host__ __device__ constexpr bool epi_rk(int mode) { return mode == EPI_RK || mode == EPI_RK64; }
 
 #define RK_MAXS 7
+// The combination a Runge-Kutta epilogue forms from the stage torques:
+// m0 + sum_j (dt a_j) k_j over the np earlier stages with a non-zero weight
+// (in stage order), then this stage's own torque (weight a_own).  Weights
+// are zero where only the other combination of a pair uses the stage.
 struct RKCoef {
-  float a[RK_MAXS];   // row a[i+1][0..i] (next stage input), or b for the final stage
-  float b2[RK_MAXS];  // lower-order weights (final stage, adaptive)
-  int nk;             // number of k's combined
-  int final_stage;    // 1: produce m_high / m_low / error
-  int adaptive;
+  const float* kp[RK_MAXS - 1];  // earlier stage torques
+  float a[RK_MAXS - 1];          // next stage's row of the tableau, or b for the final stage
+  float b2[RK_MAXS - 1];         // lower-order weights (final stage, adaptive)
+  float a_own, b2_own;
+  int np;
+  int adaptive;  // final stage: form the error as well and leave m_high to the controller
+  int norm;      // final stage of a fixed step: out1 takes normalize(m_high)
 };
 
 struct EpiArgs {
@@ -33,33 +39,39 @@ struct EpiArgs {
   double* energy;       // RK stages: device accumulator of the total energy
                         // density sum (Relax's energy, relax.go:14-23), may be null
   const float* dt_dev;  // RK: device dt
-  float* kbuf[RK_MAXS]; // RK: stage torques
-  int stage;            // RK: index of this stage's k
   RKCoef rk;
 };
 
 
 // Per-cell inputs an epilogue reads besides the field: m at which the field
 // was evaluated, and for Heun's corrector t0 and m (aux0, aux1), for an RK
-// stage the step-start m (aux0).  Loaded ahead of the transform so that
-// their latency overlaps it.
-template <int MODE>
+// stage that forms a combination the step-start m (aux0, or m itself where
+// aux0 is null).  Loaded ahead of their use so that the latencies overlap.
+template <int MODE, bool NEXT>
 struct EpiIn {
+  static constexpr bool A0 = MODE == EPI_HEUN2 || epi_rk(MODE) || (MODE == EPI_TORQUE && NEXT);
   float m[3];
-  float a0[(MODE == EPI_HEUN2 || epi_rk(MODE)) ? 3 : 1];
+  float a0[A0 ? 3 : 1];
   float a1[MODE == EPI_HEUN2 ? 3 : 1];
 };
 
-template <int MODE>
-__device__ __forceinline__ void epi_load(const EpiArgs& ea, int64_t g, EpiIn<MODE>& in) {
+template <int MODE, bool NEXT>
+__device__ __forceinline__ void epi_load(const EpiArgs& ea, int64_t g, EpiIn<MODE, NEXT>& in) {
   const int64_t n = ea.n;
   in.m[0] = ea.m_in[g];
   in.m[1] = ea.m_in[n + g];
   in.m[2] = ea.m_in[2 * n + g];
-  if (MODE == EPI_HEUN2 || epi_rk(MODE)) {
-    in.a0[0] = ea.aux0[g];
-    in.a0[1] = ea.aux0[n + g];
-    in.a0[2] = ea.aux0[2 * n + g];
+  if constexpr (EpiIn<MODE, NEXT>::A0) {
+    const float* a0 = ea.aux0;
+    if (MODE == EPI_HEUN2 || a0) {
+      in.a0[0] = a0[g];
+      in.a0[1] = a0[n + g];
+      in.a0[2] = a0[2 * n + g];
+    } else {
+      in.a0[0] = in.m[0];
+      in.a0[1] = in.m[1];
+      in.a0[2] = in.m[2];
+    }
   }
   if (MODE == EPI_HEUN2) {
     in.a1[0] = ea.aux1[g];
@@ -68,152 +80,150 @@ __device__ __forceinline__ void epi_load(const EpiArgs& ea, int64_t g, EpiIn<MOD
   }
 }
 
-// next: if not null, receives the cell's next stage input (Heun: m1est
-// after the predictor, m after the corrector)
-// eacc: the thread's energy-density sum (RK stages with ea.energy set)
+// The local fields of one cell and, except for EPI_FIELD, the torque:
+// (hx,hy,hz) comes in as the convolution's field and leaves as the torque.
 template <int MODE>
-__device__ __forceinline__ void epi_cell_in(const EpiArgs& ea, int64_t g, float hx, float hy, float hz,
-                                            const EpiIn<MODE>& in, float& lmax, float* next = nullptr,
-                                            double* eacc = nullptr);
-
-// cell g (index into one component), field (hx,hy,hz) from the convolution
-template <int MODE>
-__device__ __forceinline__ void epi_cell(const EpiArgs& ea, int64_t g, float hx, float hy, float hz, float& lmax,
-                                         double* eacc = nullptr) {
-  EpiIn<MODE> in;
-  epi_load<MODE>(ea, g, in);
-  epi_cell_in<MODE>(ea, g, hx, hy, hz, in, lmax, nullptr, eacc);
+__device__ __forceinline__ void epi_torque(const EpiArgs& ea, int64_t g, float mx, float my, float mz, float& hx,
+                                           float& hy, float& hz, double& eacc) {
+  llg_local(ea.lf, mx, my, mz, hx, hy, hz);
+  if constexpr (epi_rk(MODE) || MODE == EPI_TORQUE) {
+    // energy density of the stage's m: -1/2 m.h_conv - m.Hext - 1/2 K (m.u)^2
+    // = -1/2 m.(h + Hext) with h the full field (the anisotropy terms
+    // cancel), summed in float64
+    if (ea.energy) {
+      float s = FA(FA(FM(mx, FA(hx, ea.lf.hext[0])), FM(my, FA(hy, ea.lf.hext[1]))), FM(mz, FA(hz, ea.lf.hext[2])));
+      eacc += (double)FM(-0.5f, s);
+    }
+    // the thermal field, added after the energy density (field.go:64-80)
+    if (ea.lf.sigma != 0.f) {
+      float nrm[3];
+      thermal_normals(ea.lf, g, nrm);
+      hx = FA(hx, FM(ea.lf.sigma, nrm[0]));
+      hy = FA(hy, FM(ea.lf.sigma, nrm[1]));
+      hz = FA(hz, FM(ea.lf.sigma, nrm[2]));
+    }
+  }
+  if constexpr (MODE != EPI_FIELD) llg_delta_m(mx, my, mz, hx, hy, hz, ea.alpha, ea.dtg);
 }
 
-template <int MODE>
-__device__ __forceinline__ void epi_cell_in(const EpiArgs& ea, int64_t g, float hx, float hy, float hz,
-                                            const EpiIn<MODE>& in, float& lmax, float* next, double* eacc) {
-    const int64_t n = ea.n;
-    float mx = in.m[0], my = in.m[1], mz = in.m[2];
-    llg_local(ea.lf, mx, my, mz, hx, hy, hz);
-    if constexpr (epi_rk(MODE) || MODE == EPI_TORQUE) {
-      // energy density of the stage's m: -1/2 m.h_conv - m.Hext - 1/2 K (m.u)^2
-      // = -1/2 m.(h + Hext) with h the full field (the anisotropy terms
-      // cancel), summed in float64
-      if (ea.energy && eacc) {
-        float s = FA(FA(FM(mx, FA(hx, ea.lf.hext[0])), FM(my, FA(hy, ea.lf.hext[1]))), FM(mz, FA(hz, ea.lf.hext[2])));
-        *eacc += (double)FM(-0.5f, s);
-      }
-      // the thermal field, added after the energy density (field.go:64-80)
-      if (ea.lf.sigma != 0.f) {
-        float nrm[3];
-        thermal_normals(ea.lf, g, nrm);
-        hx = FA(hx, FM(ea.lf.sigma, nrm[0]));
-        hy = FA(hy, FM(ea.lf.sigma, nrm[1]));
-        hz = FA(hz, FM(ea.lf.sigma, nrm[2]));
-      }
-    }
-    if (MODE == EPI_FIELD) {
-      ea.out0[g] = hx;
-      ea.out0[n + g] = hy;
-      ea.out0[2 * n + g] = hz;
-      return;
-    }
-    llg_delta_m(mx, my, mz, hx, hy, hz, ea.alpha, ea.dtg);
-    if (MODE == EPI_TORQUE) {
-      ea.out0[g] = hx;
-      ea.out0[n + g] = hy;
-      ea.out0[2 * n + g] = hz;
-      if (ea.err) lmax = fmaxf(lmax, fmaxf(fabsf(hx), fmaxf(fabsf(hy), fabsf(hz))));
-    } else if (MODE == EPI_HEUN1) {
+// The solver update of C cells of one thread: cell indices g (into one
+// component), h the convolution's field, in the other inputs; cells with
+// g < 0 are skipped.  With NEXT, h receives the next stage's input (Heun:
+// the predicted and the corrected m; RK: the combination).
+//
+// An RK combination reads up to six earlier torques.  They are read stage
+// by stage, all 3C values of a stage in flight together: one cell after the
+// other with the stages inside, as this loop was first written, each load
+// waited for the one before it (three-stage RK23 on a 512 x 512 film: final
+// stage 27.7 us against 9.5 us for a stage without a combination).
+template <int MODE, bool NEXT, int C>
+__device__ __forceinline__ void epi_cells(const EpiArgs& ea, const int64_t (&g)[C], float (&h)[C][3],
+                                          const EpiIn<MODE, NEXT> (&in)[C], float& lmax, double& eacc) {
+  const int64_t n = ea.n;
+#pragma unroll
+  for (int i = 0; i < C; i++) {
+    if (g[i] < 0) continue;
+    const float mx = in[i].m[0], my = in[i].m[1], mz = in[i].m[2];
+    epi_torque<MODE>(ea, g[i], mx, my, mz, h[i][0], h[i][1], h[i][2], eacc);
+    if constexpr (MODE == EPI_HEUN1) {
       // t0 = torque*dt; m1est = normalize(m + t0)   (adaptive_heun.go:39-44)
-      ea.out0[g] = hx;
-      ea.out0[n + g] = hy;
-      ea.out0[2 * n + g] = hz;
-      float ex = FA(mx, hx), ey = FA(my, hy), ez = FA(mz, hz);
+      float ex = FA(mx, h[i][0]), ey = FA(my, h[i][1]), ez = FA(mz, h[i][2]);
       llg_normalize(ex, ey, ez);
-      ea.out1[g] = ex;
-      ea.out1[n + g] = ey;
-      ea.out1[2 * n + g] = ez;
-      if (next) { next[0] = ex; next[1] = ey; next[2] = ez; }
-    } else if (MODE == EPI_HEUN2) {
+#pragma unroll
+      for (int c = 0; c < 3; c++) ea.out0[c * n + g[i]] = h[i][c];
+      h[i][0] = ex;
+      h[i][1] = ey;
+      h[i][2] = ez;
+#pragma unroll
+      for (int c = 0; c < 3; c++) ea.out1[c * n + g[i]] = h[i][c];
+    } else if constexpr (MODE == EPI_HEUN2) {
       // t = 0.5 t1 + 0.5 t0; m = normalize(m + t)   (adaptive_heun.go:46-52)
-      float tx = FA(FM(0.5f, hx), FM(0.5f, in.a0[0]));
-      float ty = FA(FM(0.5f, hy), FM(0.5f, in.a0[1]));
-      float tz = FA(FM(0.5f, hz), FM(0.5f, in.a0[2]));
-      float nx = FA(in.a1[0], tx), ny = FA(in.a1[1], ty), nz = FA(in.a1[2], tz);
-      llg_normalize(nx, ny, nz);
-      ea.out0[g] = nx;
-      ea.out0[n + g] = ny;
-      ea.out0[2 * n + g] = nz;
-      if (next) { next[0] = nx; next[1] = ny; next[2] = nz; }
+#pragma unroll
+      for (int c = 0; c < 3; c++) h[i][c] = FA(in[i].a1[c], FA(FM(0.5f, h[i][c]), FM(0.5f, in[i].a0[c])));
+      llg_normalize(h[i][0], h[i][1], h[i][2]);
+#pragma unroll
+      for (int c = 0; c < 3; c++) ea.out0[c * n + g[i]] = h[i][c];
       if (ea.err) {
         // error = maxabs(m1est - m)   (adaptive_heun.go:56-59)
-        float d0 = fabsf(FA(mx, FM(-1.f, nx)));
-        float d1 = fabsf(FA(my, FM(-1.f, ny)));
-        float d2 = fabsf(FA(mz, FM(-1.f, nz)));
-        lmax = fmaxf(lmax, fmaxf(d0, fmaxf(d1, d2)));
-      }
-    } else if (epi_rk(MODE)) {
-      float kx = hx, ky = hy, kz = hz;
-      float* kd = ea.out0;
-      kd[g] = kx;
-      kd[n + g] = ky;
-      kd[2 * n + g] = kz;
-      const float dt = *ea.dt_dev;
-      // in.a0: the step-start magnetisation
-      float q[3] = {in.a0[0], in.a0[1], in.a0[2]};
-      // next stage input (or m_high): m0 + sum_j (dt a_j) k_j, j in order
 #pragma unroll
-      for (int j = 0; j < RK_MAXS; j++) {
-        if (j >= ea.rk.nk) break;
-        float a = ea.rk.a[j];
-        if (a == 0.f) continue;
-        float c = FM(dt, a);
-        float k0, k1, k2;
-        if (j == ea.stage) { k0 = kx; k1 = ky; k2 = kz; }
-        else { k0 = ea.kbuf[j][g]; k1 = ea.kbuf[j][n + g]; k2 = ea.kbuf[j][2 * n + g]; }
-        q[0] = FA(q[0], FM(c, k0));
-        q[1] = FA(q[1], FM(c, k1));
-        q[2] = FA(q[2], FM(c, k2));
+        for (int c = 0; c < 3; c++) lmax = fmaxf(lmax, fabsf(FA(in[i].m[c], FM(-1.f, h[i][c]))));
       }
-      if (MODE == EPI_RK64 && ea.rk.final_stage && ea.rk.adaptive) {
+    } else {
+      // the field (EPI_FIELD) or the stage torque
+      if (ea.out0) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) ea.out0[c * n + g[i]] = h[i][c];
+      }
+      if (MODE == EPI_TORQUE && ea.err) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) lmax = fmaxf(lmax, fabsf(h[i][c]));
+      }
+    }
+  }
+  if constexpr (epi_rk(MODE) || (MODE == EPI_TORQUE && NEXT)) {
+    const float dt = *ea.dt_dev;
+    const bool low = MODE == EPI_RK && ea.rk.adaptive;
+    const bool low64 = MODE == EPI_RK64 && ea.rk.adaptive;
+    float q[C][3], lo[MODE == EPI_RK ? C : 1][3];
+    double e64[MODE == EPI_RK64 ? C : 1][3];
+#pragma unroll
+    for (int i = 0; i < C; i++) {
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        q[i][c] = in[i].a0[c];
+        if constexpr (MODE == EPI_RK) lo[i][c] = in[i].a0[c];
+        if constexpr (MODE == EPI_RK64) e64[i][c] = 0.0;
+      }
+    }
+    auto add = [&](int i, int c, float a, float b, float k) {
+      if (a != 0.f) q[i][c] = FA(q[i][c], FM(FM(dt, a), k));
+      if constexpr (MODE == EPI_RK) {
+        if (low && b != 0.f) lo[i][c] = FA(lo[i][c], FM(FM(b, dt), k));
+      }
+      if constexpr (MODE == EPI_RK64) {
         // the embedded error vector sum_j (b_j - b*_j) dt k_j formed and
         // normed in float64 from the float32 stage torques
-        double e0 = 0.0, e1 = 0.0, e2 = 0.0;
-#pragma unroll
-        for (int j = 0; j < RK_MAXS; j++) {
-          if (j >= ea.rk.nk) break;
-          const double w = ((double)ea.rk.a[j] - (double)ea.rk.b2[j]) * (double)dt;
-          if (w == 0.0) continue;
-          float k0, k1, k2;
-          if (j == ea.stage) { k0 = kx; k1 = ky; k2 = kz; }
-          else { k0 = ea.kbuf[j][g]; k1 = ea.kbuf[j][n + g]; k2 = ea.kbuf[j][2 * n + g]; }
-          e0 = fma(w, (double)k0, e0);
-          e1 = fma(w, (double)k1, e1);
-          e2 = fma(w, (double)k2, e2);
-        }
-        lmax = fmaxf(lmax, (float)fmax(fabs(e0), fmax(fabs(e1), fabs(e2))));
-      } else if (ea.rk.final_stage && ea.rk.adaptive) {
-        float lo[3] = {in.a0[0], in.a0[1], in.a0[2]};
-#pragma unroll
-        for (int j = 0; j < RK_MAXS; j++) {
-          if (j >= ea.rk.nk) break;
-          float b = ea.rk.b2[j];
-          if (b == 0.f) continue;
-          float c = FM(b, dt);
-          float k0, k1, k2;
-          if (j == ea.stage) { k0 = kx; k1 = ky; k2 = kz; }
-          else { k0 = ea.kbuf[j][g]; k1 = ea.kbuf[j][n + g]; k2 = ea.kbuf[j][2 * n + g]; }
-          lo[0] = FA(lo[0], FM(c, k0));
-          lo[1] = FA(lo[1], FM(c, k1));
-          lo[2] = FA(lo[2], FM(c, k2));
-        }
-        float d0 = fabsf(FA(lo[0], FM(-1.f, q[0])));
-        float d1 = fabsf(FA(lo[1], FM(-1.f, q[1])));
-        float d2 = fabsf(FA(lo[2], FM(-1.f, q[2])));
-        lmax = fmaxf(lmax, fmaxf(d0, fmaxf(d1, d2)));
+        const double w = ((double)a - (double)b) * (double)dt;
+        if (low64 && w != 0.0) e64[i][c] = fma(w, (double)k, e64[i][c]);
       }
-      ea.out1[g] = q[0];
-      ea.out1[n + g] = q[1];
-      ea.out1[2 * n + g] = q[2];
+    };
+    const int np = ea.rk.np;
+#pragma unroll 1
+    for (int j = 0; j < np; j++) {
+      const float* kj = ea.rk.kp[j];
+      const float a = ea.rk.a[j], b = ea.rk.b2[j];
+      float v[C][3];
+#pragma unroll
+      for (int i = 0; i < C; i++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) v[i][c] = g[i] >= 0 ? kj[c * n + g[i]] : 0.f;
+#pragma unroll
+      for (int i = 0; i < C; i++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) add(i, c, a, b, v[i][c]);
     }
-  
+#pragma unroll
+    for (int i = 0; i < C; i++) {
+      if (g[i] < 0) continue;
+#pragma unroll
+      for (int c = 0; c < 3; c++) add(i, c, ea.rk.a_own, ea.rk.b2_own, h[i][c]);
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        if constexpr (MODE == EPI_RK) {
+          if (low) lmax = fmaxf(lmax, fabsf(FA(lo[i][c], FM(-1.f, q[i][c]))));
+        }
+        if constexpr (MODE == EPI_RK64) {
+          if (low64) lmax = fmaxf(lmax, (float)fabs(e64[i][c]));
+        }
+      }
+      if (epi_rk(MODE) && ea.rk.norm) llg_normalize(q[i][0], q[i][1], q[i][2]);
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        ea.out1[c * n + g[i]] = q[i][c];
+        h[i][c] = q[i][c];
+      }
+    }
+  }
 }
 
 // block-wide maximum of lmax into *ea.err (non-negative float atomics) and,

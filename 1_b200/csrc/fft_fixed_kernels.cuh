@@ -314,14 +314,6 @@ __device__ __forceinline__ void conv_body(const ConvArgs& a, int bx) {
   }
 }
 
-template <int L, int TK, int T, bool D2, bool HALF>
-// at least 768 resident threads per SM (6 blocks of 128 for L = 64):
-// measured faster than the unconstrained 96-register build (5 blocks) and
-// than 7 or 8 blocks (register spills)
-__global__ void __launch_bounds__(T, (768 / T) > 0 ? (768 / T) : 1) k_conv_fx(ConvArgs a) {
-  conv_body<L, TK, T, D2, HALF, !D2>(a, blockIdx.x);
-}
-
 // ---------------------------------------------------------------------
 // Z rows.  Tile index-major with an odd row pitch: element n of line l at
 // sm[n * SIP + l]; global accesses walk the row (coalesced), stages walk
@@ -359,31 +351,59 @@ __device__ __forceinline__ void zr2c_body(const float* __restrict__ src, float2*
     int l, j;
     S0::lj(i, l, j);
     float2 v[R0];
+    const int64_t roff = l < nl ? roff_s[l] : 0;
+    if (COMB && vec2 && l < nl) {
+      // the stage combination, each term's pairs loaded together
 #pragma unroll
-    for (int q = 0; q < R0; q++) {
-      const int n = S0::in_idx(j, q);
-      float a = 0.f, b = 0.f;
-      if (l < nl) {
-        const int64_t roff = roff_s[l];
-        const int i0 = 2 * n;
-        if (COMB && vec2 && i0 + 1 < nreal) {
-          const float2 p = zcomb_value2(cb, dt, roff + i0);
-          *reinterpret_cast<float2*>(cb.out + roff + i0) = p;
-          a = p.x;
-          b = p.y;
-        } else if (COMB) {
-          if (i0 < nreal) { a = zcomb_value(cb, dt, roff + i0); cb.out[roff + i0] = a; }
-          if (i0 + 1 < nreal) { b = zcomb_value(cb, dt, roff + i0 + 1); cb.out[roff + i0 + 1] = b; }
-        } else if (vec2 && i0 + 1 < nreal) {
-          float2 p = __ldg(reinterpret_cast<const float2*>(src + roff + i0));
-          a = p.x;
-          b = p.y;
-        } else {
-          if (i0 < nreal) a = src[roff + i0];
-          if (i0 + 1 < nreal) b = src[roff + i0 + 1];
+      for (int q = 0; q < R0; q++) {
+        const int i0 = 2 * S0::in_idx(j, q);
+        v[q] = i0 + 1 < nreal ? __ldg(reinterpret_cast<const float2*>(cb.m0 + roff + i0)) : make_float2(0.f, 0.f);
+        // the last value of an odd row
+        if (i0 + 1 == nreal) v[q].x = cb.m0[roff + i0];
+      }
+#pragma unroll 1
+      for (int t = 0; t < cb.nk; t++) {
+        const float* kt = cb.k[t] + roff;
+        const float f = __fmul_rn(dt, cb.a[t]);
+        float2 kk[R0];
+#pragma unroll
+        for (int q = 0; q < R0; q++) {
+          const int i0 = 2 * S0::in_idx(j, q);
+          kk[q] = i0 + 1 < nreal ? __ldg(reinterpret_cast<const float2*>(kt + i0)) : make_float2(0.f, 0.f);
+          if (i0 + 1 == nreal) kk[q].x = kt[i0];
+        }
+#pragma unroll
+        for (int q = 0; q < R0; q++) {
+          v[q].x = __fadd_rn(v[q].x, __fmul_rn(f, kk[q].x));
+          v[q].y = __fadd_rn(v[q].y, __fmul_rn(f, kk[q].y));
         }
       }
-      v[q] = make_float2(a, b);
+#pragma unroll
+      for (int q = 0; q < R0; q++) {
+        const int i0 = 2 * S0::in_idx(j, q);
+        if (i0 + 1 < nreal) *reinterpret_cast<float2*>(cb.out + roff + i0) = v[q];
+        else if (i0 + 1 == nreal) cb.out[roff + i0] = v[q].x;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < R0; q++) {
+        const int i0 = 2 * S0::in_idx(j, q);
+        float a = 0.f, b = 0.f;
+        if (l < nl) {
+          if (COMB) {
+            if (i0 < nreal) { a = zcomb_value(cb, dt, roff + i0); cb.out[roff + i0] = a; }
+            if (i0 + 1 < nreal) { b = zcomb_value(cb, dt, roff + i0 + 1); cb.out[roff + i0 + 1] = b; }
+          } else if (vec2 && i0 + 1 < nreal) {
+            const float2 p = __ldg(reinterpret_cast<const float2*>(src + roff + i0));
+            a = p.x;
+            b = p.y;
+          } else {
+            if (i0 < nreal) a = src[roff + i0];
+            if (i0 + 1 < nreal) b = src[roff + i0 + 1];
+          }
+        }
+        v[q] = make_float2(a, b);
+      }
     }
     // open boundary (n_real = M): the upper half of the pairs is padding
     if (nreal == M) dft_half<R0>(v, false);
@@ -538,35 +558,39 @@ __device__ __forceinline__ void zinv_body(const ZinvArgs& za, int bx) {
     // input of this thread's cells is loaded before any is used, so the
     // loads are in flight together.
     constexpr int CPT = (RT * M + T - 1) / T;
-    EpiIn<MODE> in[CPT];
+    EpiIn<MODE, FUSE> in[CPT];
+    int64_t g[CPT];
+    float h[CPT][3];
 #pragma unroll
     for (int i = 0; i < CPT; i++) {
-      int e = threadIdx.x + i * T;
-      if (e < nr * M) epi_load<MODE>(ea, g0 + e, in[i]);
+      const int e = threadIdx.x + i * T;
+      g[i] = e < nr * M ? g0 + e : -1;
+      if (g[i] >= 0) epi_load<MODE, FUSE>(ea, g[i], in[i]);
     }
 #pragma unroll
     for (int i = 0; i < CPT; i++) {
-      int e = threadIdx.x + i * T;
+      const int e = threadIdx.x + i * T;
       if (e >= nr * M) continue;
-      int r = e / M, zz = e % M;
-      float2* base = sm + 3 * r * PITCH + padi(zz >> 1);
-      float hx = (zz & 1) ? base[0].y : base[0].x;
-      float hy = (zz & 1) ? base[PITCH].y : base[PITCH].x;
-      float hz = (zz & 1) ? base[2 * PITCH].y : base[2 * PITCH].x;
-      if constexpr (FUSE) {
-        // the same 4-byte word that held this cell's field takes its new m
-        float nm[3];
-        epi_cell_in<MODE>(ea, g0 + e, hx, hy, hz, in[i], lmax, nm);
-        float* w = reinterpret_cast<float*>(base) + (zz & 1);
-        w[0] = nm[0];
-        w[2 * PITCH] = nm[1];
-        w[4 * PITCH] = nm[2];
-      } else {
-        epi_cell_in<MODE>(ea, g0 + e, hx, hy, hz, in[i], lmax, nullptr, &eacc);
+      const int r = e / M, zz = e % M;
+      const float* base = reinterpret_cast<const float*>(sm + 3 * r * PITCH + padi(zz >> 1)) + (zz & 1);
+#pragma unroll
+      for (int c = 0; c < 3; c++) h[i][c] = base[2 * c * PITCH];
+    }
+    epi_cells<MODE, FUSE, CPT>(ea, g, h, in, lmax, eacc);
+    if constexpr (FUSE) {
+      // the same 4-byte word that held a cell's field takes its new m
+#pragma unroll
+      for (int i = 0; i < CPT; i++) {
+        const int e = threadIdx.x + i * T;
+        if (e >= nr * M) continue;
+        const int r = e / M, zz = e % M;
+        float* base = reinterpret_cast<float*>(sm + 3 * r * PITCH + padi(zz >> 1)) + (zz & 1);
+#pragma unroll
+        for (int c = 0; c < 3; c++) base[2 * c * PITCH] = h[i][c];
       }
     }
     if constexpr (FUSE) {
-      epi_flush_max<MODE>(ea, lmax);
+      epi_flush_max<MODE>(ea, lmax, eacc);
       __syncthreads();
       // forward Z of the new rows: pairs n < M/2 hold the data, the rest of
       // each line is padding (zero); then the R2C split into the spectrum
@@ -612,25 +636,26 @@ __device__ __forceinline__ void zinv_body(const ZinvArgs& za, int bx) {
       return;
     }
   } else {
-    for (int e = threadIdx.x; e < nr * N2; e += T) {
-      int r = e / N2, zz = e - r * N2;
-      const float2* base = sm + 3 * r * PITCH + padi(zz >> 1);
-      float hx = (zz & 1) ? base[0].y : base[0].x;
-      float hy = (zz & 1) ? base[PITCH].y : base[PITCH].x;
-      float hz = (zz & 1) ? base[2 * PITCH].y : base[2 * PITCH].x;
-      epi_cell<MODE>(ea, g0 + e, hx, hy, hz, lmax, &eacc);
+    constexpr int C = 4;
+    for (int e0 = threadIdx.x; e0 < nr * N2; e0 += C * T) {
+      EpiIn<MODE, false> in[C];
+      int64_t g[C];
+      float h[C][3];
+#pragma unroll
+      for (int i = 0; i < C; i++) {
+        const int e = e0 + i * T;
+        g[i] = e < nr * N2 ? g0 + e : -1;
+        if (g[i] < 0) continue;
+        epi_load<MODE, false>(ea, g[i], in[i]);
+        const int r = e / N2, zz = e - r * N2;
+        const float* base = reinterpret_cast<const float*>(sm + 3 * r * PITCH + padi(zz >> 1)) + (zz & 1);
+#pragma unroll
+        for (int c = 0; c < 3; c++) h[i][c] = base[2 * c * PITCH];
+      }
+      epi_cells<MODE, false, C>(ea, g, h, in, lmax, eacc);
     }
   }
   epi_flush_max<MODE>(ea, lmax, eacc);
-}
-
-template <int M, int RT, int T, int MODE>
-__global__ void __launch_bounds__(T) k_zinv_fx(ZinvArgs za) {
-  zinv_body<M, RT, T, MODE>(za, blockIdx.x);
-}
-template <int M, int RT, int T, int MODE>
-__global__ void __launch_bounds__(T) k_zinv_fwd_fx(ZinvArgs za) {
-  zinv_body<M, RT, T, MODE, true>(za, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------
@@ -712,25 +737,6 @@ cudaError_t fx_launch_col(const float2* src, float2* dst, const ColPass& cp, cud
   return cudaGetLastError();
 }
 
-template <int L, bool D2>
-cudaError_t fx_launch_conv(const ConvArgs& a, cudaStream_t st) {
-  constexpr int TKP = conv_tkp(L);
-  // one thread per (column, radix-8 butterfly): it owns the three components
-  constexpr int NBF = TKP * (L / fwd_radix(L, n_stages(L) - 1));
-  constexpr int T = NBF < 64 ? 64 : (NBF > 512 ? 512 : ((NBF + 31) / 32) * 32);
-  size_t smem = conv_smem(L);
-  if (2 * a.n_data == L) {
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(k_conv_fx<L, TKP, T, D2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_conv_fx<L, TKP, T, D2, true><<<div_up(a.ncols, TKP), T, smem, st>>>(a);
-  } else {
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(k_conv_fx<L, TKP, T, D2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_conv_fx<L, TKP, T, D2, false><<<div_up(a.ncols, TKP), T, smem, st>>>(a);
-  }
-  return cudaGetLastError();
-}
-
 // rows per Z tile: 2048 elements for the forward pass (smaller blocks, more
 // of them resident), 4096 for the three-component inverse pass
 __host__ __device__ constexpr int fx_rows(int M, int lines_per_row) {
@@ -757,46 +763,5 @@ cudaError_t fx_launch_zc2r(const float2* src, float* dst, const ZPass& z, cudaSt
   size_t smem = sizeof(float2) * (size_t)odd_pitch(RT) * M;
   if (smem > 48 * 1024) cudaFuncSetAttribute(k_zc2r_fx<M, RT, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   k_zc2r_fx<M, RT, T><<<div_up(z.nrows, RT), T, smem, st>>>(src, dst, z);
-  return cudaGetLastError();
-}
-
-template <int M, int MODE>
-cudaError_t fx_launch_zinv(const float2* S, const float2* twz, const float2* twP, int P1, int HZ, int64_t CS, int nrows,
-                           const EpiArgs& ea, cudaStream_t st) {
-  constexpr int RT = fx_rows(M, 3);
-  constexpr int T = fx_threads(3 * RT * M);
-  size_t smem = sizeof(float2) * (size_t)3 * RT * row_pitch(M);
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k_zinv_fx<M, RT, T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  ZinvArgs za;
-  za.S = const_cast<float2*>(S);
-  za.twz = twz;
-  za.twP = twP;
-  za.P1 = P1;
-  za.HZ = HZ;
-  za.CS = CS;
-  za.nrows = nrows;
-  za.ea = ea;
-  k_zinv_fx<M, RT, T, MODE><<<div_up(nrows, RT), T, smem, st>>>(za);
-  return cudaGetLastError();
-}
-
-// inverse Z + Heun epilogue + the next evaluation's forward Z (k_zinv_fwd_fx)
-template <int M, int MODE>
-cudaError_t fx_launch_zinv_fwd(float2* S, const float2* twz, const float2* twP, int P1, int HZ, int64_t CS, int nrows,
-                               const EpiArgs& ea, cudaStream_t st) {
-  constexpr int RT = fx_rows(M, 3);
-  constexpr int T = fx_threads(3 * RT * M);
-  size_t smem = sizeof(float2) * (size_t)3 * RT * row_pitch(M);
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k_zinv_fwd_fx<M, RT, T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  ZinvArgs za;
-  za.S = S;
-  za.twz = twz;
-  za.twP = twP;
-  za.P1 = P1;
-  za.HZ = HZ;
-  za.CS = CS;
-  za.nrows = nrows;
-  za.ea = ea;
-  k_zinv_fwd_fx<M, RT, T, MODE><<<div_up(nrows, RT), T, smem, st>>>(za);
   return cudaGetLastError();
 }

@@ -51,8 +51,9 @@ __device__ __forceinline__ void zrow_offsets(const ZPass& z, int r, int64_t* rof
 }
 
 // Optional stage combination applied while loading a row: the value
-// transformed is  m0 + sum_j (dt a_j) k_j  (the Runge-Kutta stage input of
-// src/go/sim/rk.go:316-322, same operation order), also stored to 'out'.
+// transformed is  m0 + sum_j (dt a_j) k_j  over the nk stages with a non-zero
+// weight (the Runge-Kutta stage input of src/go/sim/rk.go:316-322, same
+// operation order), also stored to 'out'.
 #define ZCOMB_MAXK 7
 struct ZComb {
   const float* m0;
@@ -65,28 +66,8 @@ struct ZComb {
 
 __device__ __forceinline__ float zcomb_value(const ZComb& cb, float dt, int64_t gi) {
   float q = cb.m0[gi];
-#pragma unroll
-  for (int j = 0; j < ZCOMB_MAXK; j++) {
-    if (j >= cb.nk) break;
-    if (cb.a[j] == 0.f) continue;
-    q = __fadd_rn(q, __fmul_rn(__fmul_rn(dt, cb.a[j]), cb.k[j][gi]));
-  }
-  return q;
-}
-
-// The same for the two adjacent elements gi, gi + 1 (gi even, 8-byte
-// aligned rows): 8-byte loads, each component rounded as above.
-__device__ __forceinline__ float2 zcomb_value2(const ZComb& cb, float dt, int64_t gi) {
-  float2 q = __ldg(reinterpret_cast<const float2*>(cb.m0 + gi));
-#pragma unroll
-  for (int j = 0; j < ZCOMB_MAXK; j++) {
-    if (j >= cb.nk) break;
-    if (cb.a[j] == 0.f) continue;
-    const float f = __fmul_rn(dt, cb.a[j]);
-    const float2 kk = __ldg(reinterpret_cast<const float2*>(cb.k[j] + gi));
-    q.x = __fadd_rn(q.x, __fmul_rn(f, kk.x));
-    q.y = __fadd_rn(q.y, __fmul_rn(f, kk.y));
-  }
+#pragma unroll 1
+  for (int j = 0; j < cb.nk; j++) q = __fadd_rn(q, __fmul_rn(__fmul_rn(dt, cb.a[j]), cb.k[j][gi]));
   return q;
 }
 

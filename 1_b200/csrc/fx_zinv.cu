@@ -1,0 +1,75 @@
+// The inverse Z passes with one epilogue each (FX_MODE, an EPI_* value):
+// plain and followed by the next evaluation's forward Z, single grid and batch.
+#include "fx_dispatch.cuh"
+
+template <int M, int RT, int T, int MODE>
+__global__ void __launch_bounds__(T) k_zinv_fx(ZinvArgs za) {
+  zinv_body<M, RT, T, MODE>(za, blockIdx.x);
+}
+template <int M, int RT, int T, int MODE>
+__global__ void __launch_bounds__(T) k_zinv_fwd_fx(ZinvArgs za) {
+  zinv_body<M, RT, T, MODE, true>(za, blockIdx.x);
+}
+
+template <int M, int RT, int T, int MODE, bool FUSE>
+__global__ void __launch_bounds__(T) kb_zinv(const ZinvArgs* __restrict__ a, const int* __restrict__ starts,
+                                             int nseg) {
+  int s = find_seg(starts, nseg, blockIdx.x);
+  zinv_body<M, RT, T, MODE, FUSE>(a[s], blockIdx.x - starts[s]);
+}
+
+// epilogues that can be followed by the next forward Z: the Heun stages (and, in later
+// stages of a step, the Runge-Kutta ones)
+static constexpr bool CAN_FUSE = FX_MODE == EPI_HEUN1 || FX_MODE == EPI_HEUN2;
+static constexpr bool IN_BATCH = FX_MODE >= EPI_HEUN1 && FX_MODE <= EPI_RK;
+
+template <int M>
+static cudaError_t launch(const ZinvArgs& za, bool fuse, cudaStream_t st) {
+  constexpr int RT = fx_rows(M, 3);
+  constexpr int T = fx_threads(3 * RT * M);
+  size_t smem = sizeof(float2) * (size_t)3 * RT * row_pitch(M);
+  auto go = [&](auto kern) {
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kern<<<div_up(za.nrows, RT), T, smem, st>>>(za);
+    return cudaGetLastError();
+  };
+  if (!fuse) return go(k_zinv_fx<M, RT, T, FX_MODE>);
+  if constexpr (CAN_FUSE) return go(k_zinv_fwd_fx<M, RT, T, FX_MODE>);
+  return cudaErrorInvalidValue;
+}
+template <int M>
+static cudaError_t launch_batch(const BatchLaunch& l, bool fuse, cudaStream_t st) {
+  constexpr int RT = fx_rows(M, 3);
+  constexpr int T = fx_threads(3 * RT * M);
+  size_t smem = sizeof(float2) * (size_t)3 * RT * row_pitch(M);
+  auto go = [&](auto kern) {
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    kern<<<l.blocks, T, smem, st>>>((const ZinvArgs*)l.args, l.starts, l.nseg);
+    return cudaGetLastError();
+  };
+  if constexpr (IN_BATCH) {
+    if (!fuse) return go(kb_zinv<M, RT, T, FX_MODE, false>);
+  }
+  return cudaErrorInvalidValue;
+}
+
+#define CAT2_(a, b) a##b
+#define CAT_(a, b) CAT2_(a, b)
+cudaError_t CAT_(fx_zinv_, FX_MODE)(int M, const ZinvArgs& za, bool fuse, cudaStream_t st) {
+  switch (M) {
+#define C_(LL) \
+  case LL: return launch<LL>(za, fuse, st);
+    FX_SIZES(C_)
+#undef C_
+  }
+  return cudaErrorInvalidValue;
+}
+cudaError_t CAT_(bx_zinv_, FX_MODE)(const BatchLaunch& l, bool fuse, cudaStream_t st) {
+  switch (l.L) {
+#define C_(LL) \
+  case LL: return launch_batch<LL>(l, fuse, st);
+    FX_SIZES(C_)
+#undef C_
+  }
+  return cudaErrorInvalidValue;
+}

@@ -30,7 +30,7 @@
 #include "llg_ops.cuh"
 #include "epilogue.cuh"
 #include "kernmul.cuh"
-#include "fft_fixed_kernels.cuh"
+#include "fx_dispatch.cuh"
 #include "solver_state.cuh"
 #include "../../include/mmx.h"
 
@@ -208,14 +208,23 @@ __global__ void FFT_BOUNDS(THREADS) k_zinv_epi(const float2* __restrict__ S, Lin
 
   float lmax = 0.f;
   double eacc = 0.0;
-  for (int e = threadIdx.x; e < nr * N2; e += nt) {
-    int r = e / N2, z = e - r * N2;
-    int64_t g = (int64_t)(r0 + r) * N2 + z;
-    const float2* base = sm + (r * 3) * ld + (z >> 1);
-    float hx = (z & 1) ? base[0].y : base[0].x;
-    float hy = (z & 1) ? base[ld].y : base[ld].x;
-    float hz = (z & 1) ? base[2 * ld].y : base[2 * ld].x;
-    epi_cell<MODE>(ea, g, hx, hy, hz, lmax, &eacc);
+  constexpr int C = 4;
+  for (int e0 = threadIdx.x; e0 < nr * N2; e0 += C * nt) {
+    EpiIn<MODE, false> in[C];
+    int64_t g[C];
+    float h[C][3];
+#pragma unroll
+    for (int i = 0; i < C; i++) {
+      const int e = e0 + i * nt;
+      g[i] = e < nr * N2 ? (int64_t)r0 * N2 + e : -1;
+      if (g[i] < 0) continue;
+      epi_load<MODE, false>(ea, g[i], in[i]);
+      const int r = e / N2, z = e - r * N2;
+      const float* base = reinterpret_cast<const float*>(sm + (r * 3) * ld + (z >> 1)) + (z & 1);
+#pragma unroll
+      for (int c = 0; c < 3; c++) h[i][c] = base[2 * c * ld];
+    }
+    epi_cells<MODE, false, C>(ea, g, h, in, lmax, eacc);
   }
   epi_flush_max<MODE>(ea, lmax, eacc);
 }
@@ -388,12 +397,7 @@ static cudaError_t launch_xconv(mmx_solver* s, cudaStream_t st) {
     a.tw = s->bp.fx.tw;
     a.tws = s->bp.fx.tws;
     ScopedPass sp(s, "xconv", st);
-    switch (P0) {
-#define C_(L) \
-  case L: return fx_launch_conv<L, false>(a, st);
-      FX_SIZES(C_)
-#undef C_
-    }
+    return fx_conv_0(P0, a, st);
   }
   int tk = 1;
   while (tk < 32 && P0 * 3 * tk * 2 <= (is_pow2(P0) ? 4096 : 2048)) tk *= 2;
@@ -431,12 +435,7 @@ static cudaError_t launch_yconv2d(mmx_solver* s, cudaStream_t st) {
     a.tw = s->bp.fy.tw;
     a.tws = s->bp.fy.tws;
     ScopedPass sp(s, "yconv2d", st);
-    switch (P1) {
-#define C_(L) \
-  case L: return fx_launch_conv<L, true>(a, st);
-      FX_SIZES(C_)
-#undef C_
-    }
+    return fx_conv_1(P1, a, st);
   }
   int tk = 1;
   while (tk < 32 && P1 * 3 * tk * 2 <= (is_pow2(P1) ? 4096 : 2048) && tk * 2 <= s->HZ) tk *= 2;
@@ -449,23 +448,28 @@ static cudaError_t launch_yconv2d(mmx_solver* s, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+static ZinvArgs zinv_args(mmx_solver* s, const EpiArgs& ea) {
+  ZinvArgs za;
+  za.S = s->S;
+  za.twz = s->bp.twz;
+  za.twP = s->bp.twz;
+  za.P1 = s->P[1];
+  za.HZ = s->HZ;
+  za.CS = s->CS;
+  za.nrows = s->N[0] * s->N[1];
+  za.ea = ea;
+  return za;
+}
+
 template <int MODE>
 static cudaError_t launch_zinv(mmx_solver* s, const EpiArgs& ea, cudaStream_t st) {
   int M = s->P[2] / 2;
   int nrows = s->N[0] * s->N[1];
-  if (fx_ok(M)) {
-    ScopedPass sp(s, "zinv_epi", st);
-    switch (M) {
-#define C_(L) \
-  case L: return fx_launch_zinv<L, MODE>(s->S, s->bp.twz, s->bp.twz, s->P[1], s->HZ, s->CS, nrows, ea, st);
-      FX_SIZES(C_)
-#undef C_
-    }
-  }
+  ScopedPass sp(s, "zinv_epi", st);
+  if (fx_ok(M)) return fx_zinv(MODE, M, zinv_args(s, ea), false, st);
   int rows = 1;
   while (3 * (rows * 2) * (M + 1) <= (is_pow2(M) ? 4096 : 2048) && rows * 2 <= nrows) rows *= 2;
   size_t smem = sizeof(float2) * (size_t)3 * rows * (M + 1);
-  ScopedPass sp(s, "zinv_epi", st);
   SHAPE_DISPATCH(3 * rows * (M + 1), is_pow2(M), {
     allow_smem(k_zinv_epi<T, E, P2, MODE>, smem);
     k_zinv_epi<T, E, P2, MODE><<<div_up(nrows, rows), T, smem, st>>>(s->S, s->bp.fz, s->bp.twz, s->N[0], s->P[1],
@@ -477,16 +481,8 @@ static cudaError_t launch_zinv(mmx_solver* s, const EpiArgs& ea, cudaStream_t st
 // inverse Z + Heun epilogue + the next evaluation's forward Z in one pass
 template <int MODE>
 static cudaError_t launch_zinv_fwd(mmx_solver* s, const EpiArgs& ea, cudaStream_t st) {
-  int M = s->P[2] / 2;
-  int nrows = s->N[0] * s->N[1];
   ScopedPass sp(s, "zinv_epi_zfwd", st);
-  switch (M) {
-#define C_(L) \
-  case L: return fx_launch_zinv_fwd<L, MODE>(s->S, s->bp.twz, s->bp.twz, s->P[1], s->HZ, s->CS, nrows, ea, st);
-    FX_SIZES(C_)
-#undef C_
-  }
-  return cudaErrorInvalidValue;
+  return fx_zinv(MODE, s->P[2] / 2, zinv_args(s, ea), true, st);
 }
 
 // Fixed-step Heun with an open Z boundary and a compiled Z length: each
@@ -607,24 +603,46 @@ static cudaError_t heun_step(mmx_solver* s, cudaStream_t st) {
   return e;
 }
 
+// The input of RK stage i: m + dt sum_j a_ij k_j over the non-zero weights.
+ZComb solver_rk_comb(mmx_solver* s, int i, const float* dt_dev) {
+  ZComb c;
+  memset(&c, 0, sizeof(c));
+  c.m0 = s->m;
+  c.dt = dt_dev;
+  c.out = s->m1;
+  for (int j = 0; j < s->stages; j++) {
+    if (s->a[i][j] == 0.f) continue;
+    c.k[c.nk] = s->kb[j];
+    c.a[c.nk++] = s->a[i][j];
+  }
+  return c;
+}
+
+// The combinations of the last stage: m_high (b) and, if adaptive, m_low (b2).
+RKCoef solver_rk_final(mmx_solver* s) {
+  RKCoef r;
+  memset(&r, 0, sizeof(r));
+  const int last = s->stages - 1;
+  for (int j = 0; j < last; j++) {
+    if (s->b[j] == 0.f && (!s->adaptive || s->b2[j] == 0.f)) continue;
+    r.kp[r.np] = s->kb[j];
+    r.a[r.np] = s->b[j];
+    r.b2[r.np++] = s->b2[j];
+  }
+  r.a_own = s->b[last];
+  r.b2_own = s->b2[last];
+  r.adaptive = s->adaptive;
+  return r;
+}
+
 // RK stage i: combine the stage input, transform, torque epilogue.
 static cudaError_t rk_stage(mmx_solver* s, int i, cudaStream_t st, float* dt_dev) {
   cudaError_t e;
   const float* src = s->m;
-  ZComb cb;
-  memset(&cb, 0, sizeof(cb));
-  bool comb = false;
-  for (int j = 0; j < s->stages; j++)
-    if (s->a[i][j] != 0.f) comb = true;
+  const ZComb cb = solver_rk_comb(s, i, dt_dev);
+  const bool comb = cb.nk > 0;
   ZPass z = box_zpass(&s->bp, 3, s->N[0], s->n, s->CS);
-  if (comb) {
-    cb.m0 = s->m;
-    for (int j = 0; j < s->stages; j++) { cb.k[j] = s->kb[j]; cb.a[j] = s->a[i][j]; }
-    cb.nk = s->stages;
-    cb.dt = dt_dev;
-    cb.out = s->m1;
-    src = s->m1;
-  }
+  if (comb) src = s->m1;
   {
     ScopedPass sp(s, "zfwd", st);
     e = launch_z_r2c(s->m, s->S, z, st, comb ? &cb : nullptr);
@@ -663,8 +681,6 @@ static cudaError_t rk_stage(mmx_solver* s, int i, cudaStream_t st, float* dt_dev
   ea.dtg = f32_div(1.f, f32_add(1.f, f32_mul(s->p.alpha, s->p.alpha)));  // Torque = DeltaM(dt=1)
   ea.m_in = src;
   ea.dt_dev = dt_dev;
-  for (int j = 0; j < s->stages; j++) ea.kbuf[j] = s->kb[j];
-  ea.stage = i;
   if (s->noise_sigma != 0.f) {
     ea.lf.sigma = s->noise_sigma;
     ea.lf.seed = s->p.thermal_seed;
@@ -678,10 +694,7 @@ static cudaError_t rk_stage(mmx_solver* s, int i, cudaStream_t st, float* dt_dev
     ea.out0 = s->kb[i];
     ea.aux0 = s->m;
     ea.out1 = s->mnew;
-    ea.rk.nk = s->stages;
-    for (int j = 0; j < s->stages; j++) { ea.rk.a[j] = s->b[j]; ea.rk.b2[j] = s->b2[j]; }
-    ea.rk.final_stage = 1;
-    ea.rk.adaptive = s->adaptive;
+    ea.rk = solver_rk_final(s);
     ea.err = s->adaptive ? s->scratch : nullptr;
     // the precision form keeps float64 for the embedded error norm
     if (s->p.precision && s->adaptive) return launch_zinv<EPI_RK64>(s, ea, st);

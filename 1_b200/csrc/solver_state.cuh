@@ -103,6 +103,9 @@ static inline float f32_add(float a, float b) { volatile float r = a + b; return
 EpiArgs solver_base_args(mmx_solver* s);
 // Device launch grid for a 1D element-wise kernel over n items.
 int solver_grid_1d(int64_t n);
+// Runge-Kutta combinations: the input of stage i, and the last stage's.
+ZComb solver_rk_comb(mmx_solver* s, int i, const float* dt_dev);
+RKCoef solver_rk_final(mmx_solver* s);
 // h = demag + exchange field of the device array m (no local fields).
 int solver_field_conv(mmx_solver* s, const float* m, float* h, cudaStream_t st);
 // One trial of the device-controlled adaptive RK step (first: no FSAL
