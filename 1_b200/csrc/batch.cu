@@ -19,25 +19,6 @@
 #include "fx_dispatch.cuh"
 #include "solver_state.cuh"
 
-struct BFin {
-  float* m;
-  const float* mnew;
-  int64_t n;
-};
-
-// m <- normalize(m_new) for every instance (rk.go:444)
-__global__ void kb_finalize(const BFin* __restrict__ a, const int* __restrict__ starts, int nseg) {
-  int s = find_seg(starts, nseg, blockIdx.x);
-  const BFin& f = a[s];
-  int64_t i = (int64_t)(blockIdx.x - starts[s]) * blockDim.x + threadIdx.x;
-  if (i >= f.n) return;
-  float x = f.mnew[i], y = f.mnew[f.n + i], z = f.mnew[2 * f.n + i];
-  llg_normalize(x, y, z);
-  f.m[i] = x;
-  f.m[f.n + i] = y;
-  f.m[2 * f.n + i] = z;
-}
-
 // One launch: a kernel family, a line length, and device tables.
 struct Launch {
   int kind;       // see enum below
@@ -49,21 +30,30 @@ struct Launch {
   int* starts;    // device array of tile offsets
   int variant = 0;  // tile shape (column passes: 0 = fx_col_tk, 1 = col_tk_alt)
   int half = 0;     // column and convolution passes: every instance's data fill half the line
+  int fuse = 0;     // inverse Z passes: followed by the next forward Z
   std::vector<int> inst;  // instances this launch reads or writes (graph dependencies)
   size_t args_off = 0, starts_off = 0;  // offsets into the batch's table block
 };
-enum { L_ZR2C = 0, L_COL = 1, L_CONV = 2, L_ZINV = 3, L_FIN = 4 };
+enum { L_ZR2C = 0, L_COL = 1, L_CONV = 2, L_ZINV = 3 };
 
 struct mmx_batch {
   std::vector<mmx_solver*> inst;
   bool owns = true;  // false: a view over solvers owned by the caller
   int solver = 0;
-  std::vector<std::vector<Launch>> stage;  // launches of each field evaluation (stage)
-  std::vector<Launch> finalize;
+  // A step: the forward Z of m (z0), then the launches of each field
+  // evaluation (stage).  Instances with an open Z boundary go on from each
+  // inverse Z to the next evaluation's forward Z; the others run the forward
+  // Z of every later evaluation as launches of its stage.  last_z holds the
+  // last stage's inverse Z passes, last_z_carry the same going on to the
+  // forward Z of the new m, for a step that another one of the same call follows.
+  std::vector<Launch> z0;
+  std::vector<std::vector<Launch>> stage;
+  std::vector<Launch> last_z, last_z_carry;
   std::vector<void*> owned;
   int use_graph = 0;
-  cudaGraphExec_t gexec = nullptr;
-  cudaStream_t gstream = nullptr;
+  // step graphs: [0] self-contained, [1] starting and ending with zfwd(m) in the spectrum buffers
+  cudaGraphExec_t gexec[2] = {nullptr, nullptr};
+  cudaStream_t gstream[2] = {nullptr, nullptr};
   long long cells = 0;
   int launches_per_step = 0;
   float** torque_ptrs = nullptr;  // RK4: per-instance max |k0| slots, cleared each step
@@ -97,13 +87,10 @@ static cudaError_t run_launch(const Launch& l, cudaStream_t st) {
   b.args = l.args;
   b.starts = l.starts;
   switch (l.kind) {
-    case L_FIN:
-      kb_finalize<<<l.blocks, 256, 0, st>>>((const BFin*)l.args, l.starts, l.nseg);
-      return cudaGetLastError();
     case L_COL: return bx_col(b, st);
     case L_CONV: return l.flag ? bx_conv_1(b, st) : bx_conv_0(b, st);
     case L_ZR2C: return bx_zr2c(b, st);
-    case L_ZINV: return bx_zinv(l.flag, b, false, st);
+    case L_ZINV: return bx_zinv(l.flag, b, l.fuse != 0, st);
   }
   return cudaErrorInvalidValue;
 }
@@ -157,7 +144,9 @@ static int batch_upload(mmx_batch* b) {
     }
   };
   for (auto& st : b->stage) patch(st);
-  patch(b->finalize);
+  patch(b->z0);
+  patch(b->last_z);
+  patch(b->last_z_carry);
   return MMX_OK;
 }
 
@@ -353,17 +342,42 @@ extern "C" int mmx_batch_tuning(int max, int* rows, float* ms, int* n) {
   return MMX_OK;
 }
 
-// Builds the launches of one field evaluation: zfwd (optionally with the
-// stage combination), yfwd / conv / yinv, zinv with the given epilogue.
-// stage_args(i) returns the epilogue arguments, comb_for(i) the combination.
+// Adds the forward Z passes of the instances 'ids' with line length M.
+template <typename CombF, typename SrcF>
+static int add_zfwd(mmx_batch* b, std::vector<Launch>& out, int M, const std::vector<int>& ids, bool comb,
+                    CombF comb_for, SrcF src_for) {
+  std::vector<BZr2c> a;
+  std::vector<int> t;
+  for (int i : ids) {
+    mmx_solver* s = b->inst[i];
+    BZr2c z;
+    memset(&z, 0, sizeof(z));
+    z.z = box_zpass(&s->bp, 3, s->N[0], s->n, s->CS);
+    z.dst = s->S;
+    z.src = src_for(i);
+    if (comb) z.cb = comb_for(i);
+    z.vec2 = (z.z.ld_real % 2 == 0) && (s->n % 2 == 0);
+    a.push_back(z);
+    t.push_back(div_up(z.z.nrows, zrows_per_tile(M, 1)));
+  }
+  int rc = add_launch(b, out, L_ZR2C, M, comb ? 1 : 0, a, t);
+  if (rc == MMX_OK && !a.empty()) out.back().inst = ids;
+  return rc;
+}
+
+// Builds the launches of one field evaluation: the forward Z where the
+// evaluation before did not go on to it (first: into z0), yfwd / conv / yinv,
+// and zinv with the given epilogue.  epi_for(i, chain) returns the epilogue
+// arguments, comb_for(i) the stage combination, src_for(i) the input.
 template <typename EpiF, typename CombF, typename SrcF>
-static int build_eval(mmx_batch* b, std::vector<Launch>& out, int mode, bool comb, EpiF epi_for, CombF comb_for,
-                      SrcF src_for) {
+static int build_eval(mmx_batch* b, std::vector<Launch>& out, int mode, bool first, bool last, bool comb, EpiF epi_for,
+                      CombF comb_for, SrcF src_for) {
   int rc;
-  std::map<int, std::vector<int>> byM, byP1_3d, byP0, byP1_2d;
+  std::map<std::pair<int, int>, std::vector<int>> byM;  // (line length, chained)
+  std::map<int, std::vector<int>> byP1_3d, byP0, byP1_2d;
   for (int i = 0; i < (int)b->inst.size(); i++) {
     mmx_solver* s = b->inst[i];
-    byM[s->P[2] / 2].push_back(i);
+    byM[std::make_pair(s->P[2] / 2, solver_z_chain(s) ? 1 : 0)].push_back(i);
     if (s->is2d) byP1_2d[s->P[1]].push_back(i);
     else {
       byP1_3d[s->P[1]].push_back(i);
@@ -372,22 +386,10 @@ static int build_eval(mmx_batch* b, std::vector<Launch>& out, int mode, bool com
   }
   // zfwd
   for (auto& g : byM) {
-    std::vector<BZr2c> a;
-    std::vector<int> t;
-    for (int i : g.second) {
-      mmx_solver* s = b->inst[i];
-      BZr2c z;
-      memset(&z, 0, sizeof(z));
-      z.z = box_zpass(&s->bp, 3, s->N[0], s->n, s->CS);
-      z.dst = s->S;
-      z.src = src_for(i);
-      if (comb) z.cb = comb_for(i);
-      z.vec2 = (z.z.ld_real % 2 == 0) && (s->n % 2 == 0);
-      a.push_back(z);
-      t.push_back(div_up(z.z.nrows, zrows_per_tile(g.first, 1)));
-    }
-    if ((rc = add_launch(b, out, L_ZR2C, g.first, comb ? 1 : 0, a, t)) != MMX_OK) return rc;
-    out.back().inst = g.second;
+    const bool chained = g.first.second != 0;
+    if (chained && !first) continue;
+    if ((rc = add_zfwd(b, chained ? b->z0 : out, g.first.first, g.second, comb, comb_for, src_for)) != MMX_OK)
+      return rc;
   }
   // Y forward (3D)
   for (auto& g : byP1_3d)
@@ -432,10 +434,11 @@ static int build_eval(mmx_batch* b, std::vector<Launch>& out, int mode, bool com
   for (auto& g : byP1_3d)
     if ((rc = add_col_launch(b, out, g.first, 1, g.second)) != MMX_OK) return rc;
   // Z inverse + epilogue
-  for (auto& g : byM) {
+  auto add_zinv = [&](std::vector<Launch>& to, const std::pair<int, int>& key, const std::vector<int>& ids,
+                      bool fuse) -> int {
     std::vector<ZinvArgs> a;
     std::vector<int> t;
-    for (int i : g.second) {
+    for (int i : ids) {
       mmx_solver* s = b->inst[i];
       ZinvArgs z;
       z.S = s->S;
@@ -445,22 +448,35 @@ static int build_eval(mmx_batch* b, std::vector<Launch>& out, int mode, bool com
       z.HZ = s->HZ;
       z.CS = s->CS;
       z.nrows = s->N[0] * s->N[1];
-      z.ea = epi_for(i);
+      z.ea = epi_for(i, fuse);
       a.push_back(z);
-      t.push_back(div_up(z.nrows, zrows_per_tile(g.first, 3)));
+      t.push_back(div_up(z.nrows, zrows_per_tile(key.first, 3)));
     }
-    if ((rc = add_launch(b, out, L_ZINV, g.first, mode, a, t)) != MMX_OK) return rc;
-    out.back().inst = g.second;
-    for (size_t k = 0; k < g.second.size(); k++)
-      b->hext_off[g.second[k]].push_back(out.back().args_off + k * sizeof(ZinvArgs) + offsetof(ZinvArgs, ea) +
-                                         offsetof(EpiArgs, lf) + offsetof(LocalField, hext));
+    int r = add_launch(b, to, L_ZINV, key.first, mode, a, t);
+    if (r != MMX_OK) return r;
+    to.back().inst = ids;
+    to.back().fuse = fuse ? 1 : 0;
+    for (size_t k = 0; k < ids.size(); k++)
+      b->hext_off[ids[k]].push_back(to.back().args_off + k * sizeof(ZinvArgs) + offsetof(ZinvArgs, ea) +
+                                    offsetof(EpiArgs, lf) + offsetof(LocalField, hext));
+    return MMX_OK;
+  };
+  for (auto& g : byM) {
+    const bool chained = g.first.second != 0;
+    if (last) {
+      if ((rc = add_zinv(b->last_z, g.first, g.second, false)) != MMX_OK) return rc;
+      if ((rc = add_zinv(b->last_z_carry, g.first, g.second, chained)) != MMX_OK) return rc;
+    } else if ((rc = add_zinv(out, g.first, g.second, chained)) != MMX_OK) {
+      return rc;
+    }
   }
   return MMX_OK;
 }
 
 static void batch_free(mmx_batch* b) {
   if (!b) return;
-  if (b->gexec) cudaGraphExecDestroy(b->gexec);
+  for (cudaGraphExec_t g : b->gexec)
+    if (g) cudaGraphExecDestroy(g);
   for (cudaStream_t q : b->par) cudaStreamDestroy(q);
   for (cudaEvent_t e : b->ev_join) cudaEventDestroy(e);
   for (void* p : b->owned) cudaFree(p);
@@ -502,7 +518,7 @@ static int batch_build(mmx_batch* b) {
   }
   if (b->solver == MMX_SOLVER_HEUN) {
     b->stage.resize(2);
-    auto epi1 = [&](int i) {
+    auto epi1 = [&](int i, bool) {
       mmx_solver* s = b->inst[i];
       EpiArgs ea = solver_base_args(s);
       ea.dtg = f32_div(s->dt, f32_add(1.f, f32_mul(s->p.alpha, s->p.alpha)));
@@ -511,7 +527,7 @@ static int batch_build(mmx_batch* b) {
       ea.out1 = s->m1;
       return ea;
     };
-    auto epi2 = [&](int i) {
+    auto epi2 = [&](int i, bool) {
       mmx_solver* s = b->inst[i];
       EpiArgs ea = solver_base_args(s);
       ea.dtg = f32_div(s->dt, f32_add(1.f, f32_mul(s->p.alpha, s->p.alpha)));
@@ -524,12 +540,12 @@ static int batch_build(mmx_batch* b) {
     auto nocomb = [&](int) { ZComb c; memset(&c, 0, sizeof(c)); return c; };
     auto src_m = [&](int i) { return (const float*)b->inst[i]->m; };
     auto src_m1 = [&](int i) { return (const float*)b->inst[i]->m1; };  // the normalised Euler estimate
-    rc = build_eval(b, b->stage[0], EPI_HEUN1, false, epi1, nocomb, src_m);
-    if (rc == MMX_OK) rc = build_eval(b, b->stage[1], EPI_HEUN2, false, epi2, nocomb, src_m1);
+    rc = build_eval(b, b->stage[0], EPI_HEUN1, true, false, false, epi1, nocomb, src_m);
+    if (rc == MMX_OK) rc = build_eval(b, b->stage[1], EPI_HEUN2, false, true, false, epi2, nocomb, src_m1);
   } else {
     b->stage.resize(4);
     for (int st = 0; st < 4 && rc == MMX_OK; st++) {
-      auto epi = [&](int i) {
+      auto epi = [&](int i, bool chain) {
         mmx_solver* s = b->inst[i];
         EpiArgs ea = solver_base_args(s);
         ea.dtg = f32_div(1.f, f32_add(1.f, f32_mul(s->p.alpha, s->p.alpha)));
@@ -538,9 +554,15 @@ static int batch_build(mmx_batch* b) {
         ea.out0 = s->kb[st];
         if (st == 0) ea.err = s->scratch + 1;  // max |k0|, the torque the relax loop stops on
         if (st == 3) {
+          ea.out0 = nullptr;
           ea.aux0 = s->m;
-          ea.out1 = s->mnew;
+          ea.out1 = s->m;  // normalize(m_high) (rk.go:444)
           ea.rk = solver_rk_final(s);
+          ea.rk.norm = 1;
+        } else if (chain) {
+          ea.rk = solver_rk_next(s, st);
+          ea.aux0 = st == 0 ? nullptr : s->m;
+          ea.out1 = s->m1;
         }
         return ea;
       };
@@ -549,37 +571,23 @@ static int batch_build(mmx_batch* b) {
         return solver_rk_comb(s, st, s->scratch + 2);
       };
       auto src_m = [&](int i) { return (const float*)b->inst[i]->m; };
-      rc = build_eval(b, b->stage[st], st == 3 ? EPI_RK : EPI_TORQUE, st > 0, epi, comb, src_m);
+      rc = build_eval(b, b->stage[st], st == 3 ? EPI_RK : EPI_TORQUE, st == 0, st == 3, st > 0, epi, comb, src_m);
     }
     if (rc == MMX_OK) {
-      std::vector<BFin> a;
-      std::vector<int> t;
-      for (mmx_solver* s : b->inst) {
-        BFin f;
-        f.m = s->m;
-        f.mnew = s->mnew;
-        f.n = s->n;
-        a.push_back(f);
-        t.push_back(div_up(s->n, 256));
-      }
-      rc = add_launch(b, b->finalize, L_FIN, 0, 0, a, t);
-      if (rc == MMX_OK) {
-        for (int i = 0; i < (int)b->inst.size(); i++) b->finalize.back().inst.push_back(i);
-        // clear the per-instance torque maxima before the step
-        std::vector<float*> tq;
-        for (mmx_solver* s : b->inst) tq.push_back(s->scratch + 1);
-        void* d = nullptr;
-        if (cudaMalloc(&d, sizeof(float*) * tq.size()) != cudaSuccess) return MMX_ERR_MEM;
-        b->owned.push_back(d);
-        cudaMemcpy(d, tq.data(), sizeof(float*) * tq.size(), cudaMemcpyHostToDevice);
-        b->torque_ptrs = (float**)d;
-      }
+      // clear the per-instance torque maxima before the step
+      std::vector<float*> tq;
+      for (mmx_solver* s : b->inst) tq.push_back(s->scratch + 1);
+      void* d = nullptr;
+      if (cudaMalloc(&d, sizeof(float*) * tq.size()) != cudaSuccess) return MMX_ERR_MEM;
+      b->owned.push_back(d);
+      cudaMemcpy(d, tq.data(), sizeof(float*) * tq.size(), cudaMemcpyHostToDevice);
+      b->torque_ptrs = (float**)d;
     }
   }
   if (rc != MMX_OK) return rc;
   if ((rc = batch_upload(b)) != MMX_OK) return rc;
   for (auto& st : b->stage) b->launches_per_step += (int)st.size();
-  b->launches_per_step += (int)b->finalize.size() + (b->torque_ptrs ? 1 : 0);
+  b->launches_per_step += (int)(b->z0.size() + b->last_z.size()) + (b->torque_ptrs ? 1 : 0);
   return MMX_OK;
 }
 
@@ -646,10 +654,10 @@ extern "C" mmx_solver* mmx_batch_instance(mmx_batch* b, int i) {
 // Launches are spread round-robin over BATCH_DAG_STREAMS streams; events
 // carry the per-instance dependencies.
 #define BATCH_DAG_STREAMS 16
-static cudaError_t batch_step_dag(mmx_batch* b, cudaStream_t st) {
+static cudaError_t batch_step_dag(mmx_batch* b, cudaStream_t st, bool carry) {
   cudaError_t e;
   const int ninst = (int)b->inst.size();
-  size_t nl = 4 + b->finalize.size();
+  size_t nl = 4 + b->z0.size() + b->last_z.size();
   for (auto& stage : b->stage) nl += stage.size();
   while ((int)b->par.size() < BATCH_DAG_STREAMS) {
     cudaStream_t q;
@@ -688,10 +696,13 @@ static cudaError_t batch_step_dag(mmx_batch* b, cudaStream_t st) {
     for (int i : l.inst) last[i] = done;
     return cudaSuccess;
   };
+  if (!carry)
+    for (const Launch& l : b->z0)
+      if ((e = run(l)) != cudaSuccess) return e;
   for (auto& stage : b->stage)
     for (const Launch& l : stage)
       if ((e = run(l)) != cudaSuccess) return e;
-  for (const Launch& l : b->finalize)
+  for (const Launch& l : carry ? b->last_z_carry : b->last_z)
     if ((e = run(l)) != cudaSuccess) return e;
   // join: the capturing stream waits for every instance's last launch
   std::vector<cudaEvent_t> tails;
@@ -705,51 +716,62 @@ static cudaError_t batch_step_dag(mmx_batch* b, cudaStream_t st) {
   return cudaSuccess;
 }
 
-static cudaError_t batch_step_launches(mmx_batch* b, cudaStream_t st, bool parallel) {
-  if (parallel) return batch_step_dag(b, st);
-  if (b->torque_ptrs) {
-    int n = (int)b->inst.size();
-    kb_clear<<<(n + 255) / 256, 256, 0, st>>>(b->torque_ptrs, n);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  for (auto& stage : b->stage)
-    for (const Launch& l : stage) {
-      cudaError_t e = run_launch(l, st);
-      if (e != cudaSuccess) return e;
-    }
-  for (const Launch& l : b->finalize) {
+static cudaError_t run_all(const std::vector<Launch>& ls, cudaStream_t st) {
+  for (const Launch& l : ls) {
     cudaError_t e = run_launch(l, st);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
 
+// one step as plain launches; have_z: the spectrum buffers hold the forward
+// Z of m, carry: leave them so
+static cudaError_t batch_step_launches(mmx_batch* b, cudaStream_t st, bool have_z, bool carry) {
+  cudaError_t e;
+  if (b->torque_ptrs) {
+    int n = (int)b->inst.size();
+    kb_clear<<<(n + 255) / 256, 256, 0, st>>>(b->torque_ptrs, n);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  if (!have_z && (e = run_all(b->z0, st)) != cudaSuccess) return e;
+  for (auto& stage : b->stage)
+    if ((e = run_all(stage, st)) != cudaSuccess) return e;
+  return run_all(carry ? b->last_z_carry : b->last_z, st);
+}
+
 extern "C" int mmx_batch_step(mmx_batch* b, int nsteps, cudaStream_t st) {
   if (!b || nsteps < 0) { mmx_set_error("bad argument"); return MMX_ERR_ARG; }
+  // several steps in one call hand the forward Z of m from step to step;
+  // each call starts from the instances' m itself
+  const int v = nsteps > 1 ? 1 : 0;
   for (int k = 0; k < nsteps; k++) {
     if (b->use_graph) {
-      if (!b->gexec || b->gstream != st) {
-        if (b->gexec) { cudaGraphExecDestroy(b->gexec); b->gexec = nullptr; }
+      if (v && k == 0) {
+        cudaError_t e = run_all(b->z0, st);
+        if (e != cudaSuccess) { mmx_set_error(cudaGetErrorString(e)); return MMX_ERR_CUDA; }
+      }
+      if (!b->gexec[v] || b->gstream[v] != st) {
+        if (b->gexec[v]) { cudaGraphExecDestroy(b->gexec[v]); b->gexec[v] = nullptr; }
         cudaStream_t cap = st;
         bool own = false;
         if (cap == 0) { MMX_TRY(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking)); own = true; }
         cudaGraph_t g;
         MMX_TRY(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e = batch_step_launches(b, cap, true);
+        cudaError_t e = batch_step_dag(b, cap, v != 0);
         cudaError_t e2 = cudaStreamEndCapture(cap, &g);
         if (own) cudaStreamDestroy(cap);
         if (e != cudaSuccess || e2 != cudaSuccess) { mmx_set_error("batch graph capture failed"); return MMX_ERR_CUDA; }
-        MMX_TRY(cudaGraphInstantiate(&b->gexec, g, 0));
+        MMX_TRY(cudaGraphInstantiate(&b->gexec[v], g, 0));
         cudaGraphDestroy(g);
-        b->gstream = st;
+        b->gstream[v] = st;
       }
-      MMX_TRY(cudaGraphLaunch(b->gexec, st));
+      MMX_TRY(cudaGraphLaunch(b->gexec[v], st));
     } else {
-      cudaError_t e = batch_step_launches(b, st, false);
+      cudaError_t e = batch_step_launches(b, st, k > 0, k + 1 < nsteps);
       if (e != cudaSuccess) { mmx_set_error(cudaGetErrorString(e)); return MMX_ERR_CUDA; }
     }
     for (mmx_solver* s : b->inst) {
+      s->spec_ready = 0;
       s->time += (double)s->dt;
       s->steps++;
     }
@@ -790,6 +812,10 @@ extern "C" int mmx_batch_set_hext(mmx_batch* b, int i, const float hext[3]) {
 extern "C" int mmx_batch_use_graph(mmx_batch* b, int on) {
   if (!b) { mmx_set_error("null argument"); return MMX_ERR_ARG; }
   b->use_graph = on;
-  if (!on && b->gexec) { cudaGraphExecDestroy(b->gexec); b->gexec = nullptr; }
+  if (!on)
+    for (cudaGraphExec_t& g : b->gexec) {
+      if (g) cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
   return MMX_OK;
 }

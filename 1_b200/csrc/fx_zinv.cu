@@ -18,10 +18,8 @@ __global__ void __launch_bounds__(T) kb_zinv(const ZinvArgs* __restrict__ a, con
   zinv_body<M, RT, T, MODE, FUSE>(a[s], blockIdx.x - starts[s]);
 }
 
-// epilogues that can be followed by the next forward Z: the Heun stages (and, in later
-// stages of a step, the Runge-Kutta ones)
-static constexpr bool CAN_FUSE = FX_MODE == EPI_HEUN1 || FX_MODE == EPI_HEUN2;
-static constexpr bool IN_BATCH = FX_MODE >= EPI_HEUN1 && FX_MODE <= EPI_RK;
+// epilogues that a step can follow with the next forward Z, and that a batch runs
+static constexpr bool IN_STEP = FX_MODE >= EPI_HEUN1 && FX_MODE <= EPI_RK;
 
 template <int M>
 static cudaError_t launch(const ZinvArgs& za, bool fuse, cudaStream_t st) {
@@ -34,7 +32,7 @@ static cudaError_t launch(const ZinvArgs& za, bool fuse, cudaStream_t st) {
     return cudaGetLastError();
   };
   if (!fuse) return go(k_zinv_fx<M, RT, T, FX_MODE>);
-  if constexpr (CAN_FUSE) return go(k_zinv_fwd_fx<M, RT, T, FX_MODE>);
+  if constexpr (IN_STEP) return go(k_zinv_fwd_fx<M, RT, T, FX_MODE>);
   return cudaErrorInvalidValue;
 }
 template <int M>
@@ -47,9 +45,7 @@ static cudaError_t launch_batch(const BatchLaunch& l, bool fuse, cudaStream_t st
     kern<<<l.blocks, T, smem, st>>>((const ZinvArgs*)l.args, l.starts, l.nseg);
     return cudaGetLastError();
   };
-  if constexpr (IN_BATCH) {
-    if (!fuse) return go(kb_zinv<M, RT, T, FX_MODE, false>);
-  }
+  if constexpr (IN_STEP) return fuse ? go(kb_zinv<M, RT, T, FX_MODE, true>) : go(kb_zinv<M, RT, T, FX_MODE, false>);
   return cudaErrorInvalidValue;
 }
 

@@ -478,20 +478,24 @@ static cudaError_t launch_zinv(mmx_solver* s, const EpiArgs& ea, cudaStream_t st
   return cudaGetLastError();
 }
 
-// inverse Z + Heun epilogue + the next evaluation's forward Z in one pass
+// inverse Z + epilogue + the next evaluation's forward Z in one pass
 template <int MODE>
 static cudaError_t launch_zinv_fwd(mmx_solver* s, const EpiArgs& ea, cudaStream_t st) {
   ScopedPass sp(s, "zinv_epi_zfwd", st);
   return fx_zinv(MODE, s->P[2] / 2, zinv_args(s, ea), true, st);
 }
 
-// Fixed-step Heun with an open Z boundary and a compiled Z length: each
-// inverse-Z epilogue also produces the next evaluation's forward Z, so the
-// spectrum buffer holds zfwd(m) between steps (spec_ready).
-static bool heun_fused(const mmx_solver* s) {
+// With an open Z boundary and a compiled Z length the inverse-Z pass can go
+// on to the forward Z of the magnetisation it has just produced (the next
+// evaluation's input is in its tile): the forward Z pass, its reads of m and
+// of the stage torques, and one launch per evaluation go away.
+bool solver_z_chain(const mmx_solver* s) {
   int M = s->P[2] / 2;
-  return s->p.solver == MMX_SOLVER_HEUN && s->p.max_error == 0.f && s->N[2] == M && s->p.periodic[2] == 0 &&
-         fx_ok(M);
+  return s->N[2] == M && s->p.periodic[2] == 0 && fx_ok(M);
+}
+// Fixed-step Heun: the spectrum buffer holds zfwd(m) between steps (spec_ready).
+static bool heun_fused(const mmx_solver* s) {
+  return s->p.solver == MMX_SOLVER_HEUN && s->p.max_error == 0.f && solver_z_chain(s);
 }
 
 static cudaError_t conv_rest(mmx_solver* s, cudaStream_t st);
@@ -635,47 +639,38 @@ RKCoef solver_rk_final(mmx_solver* s) {
   return r;
 }
 
-// RK stage i: combine the stage input, transform, torque epilogue.
-static cudaError_t rk_stage(mmx_solver* s, int i, cudaStream_t st, float* dt_dev) {
+// What stage i's epilogue forms when it goes on to the next stage: the input
+// of stage i + 1.
+RKCoef solver_rk_next(mmx_solver* s, int i) {
+  RKCoef r;
+  memset(&r, 0, sizeof(r));
+  for (int j = 0; j < i; j++) {
+    if (s->a[i + 1][j] == 0.f) continue;
+    r.kp[r.np] = s->kb[j];
+    r.a[r.np++] = s->a[i + 1][j];
+  }
+  r.a_own = s->a[i + 1][i];
+  return r;
+}
+
+// RK stage i: the stage input and its forward Z (have_z: already done by the
+// stage before), the rest of the field evaluation, the torque epilogue.
+// chain: the epilogue goes on to the next stage's input, or after the last
+// stage of a fixed step to the new m, and its forward Z.
+static cudaError_t rk_stage(mmx_solver* s, int i, cudaStream_t st, float* dt_dev, bool have_z = false,
+                            bool chain = false) {
   cudaError_t e;
   const float* src = s->m;
   const ZComb cb = solver_rk_comb(s, i, dt_dev);
   const bool comb = cb.nk > 0;
   ZPass z = box_zpass(&s->bp, 3, s->N[0], s->n, s->CS);
   if (comb) src = s->m1;
-  {
+  if (!have_z) {
     ScopedPass sp(s, "zfwd", st);
     e = launch_z_r2c(s->m, s->S, z, st, comb ? &cb : nullptr);
     if (e != cudaSuccess) return e;
   }
-  // remaining passes of the field evaluation
-  if (s->is2d) {
-    e = launch_yconv2d(s, st);
-  } else {
-    ColPass y;
-    y.f = s->bp.fy;
-    y.nplanes = 3 * s->N[0];
-    y.plane_stride = (int64_t)s->P[1] * s->HZ;
-    y.ncols = s->HZ;
-    y.stride_i = s->HZ;
-    y.n_in = s->N[1];
-    y.n_out = s->P[1];
-    y.inv = 0;
-    {
-      ScopedPass sp(s, "yfwd", st);
-      e = launch_col(s->S, s->S, y, st);
-    }
-    if (e != cudaSuccess) return e;
-    e = launch_xconv(s, st);
-    if (e != cudaSuccess) return e;
-    y.n_in = s->P[1];
-    y.n_out = s->N[1];
-    y.inv = 1;
-    {
-      ScopedPass sp(s, "yinv", st);
-      e = launch_col(s->S, s->S, y, st);
-    }
-  }
+  e = conv_rest(s, st);
   if (e != cudaSuccess) return e;
   EpiArgs ea = solver_base_args(s);
   ea.dtg = f32_div(1.f, f32_add(1.f, f32_mul(s->p.alpha, s->p.alpha)));  // Torque = DeltaM(dt=1)
@@ -690,19 +685,26 @@ static cudaError_t rk_stage(mmx_solver* s, int i, cudaStream_t st, float* dt_dev
   // calcHeffEnergy at the last stage (FSAL) or the first (rk.go:321-337)
   if (s->want_energy && s->eacc && (s->fsal ? i == s->stages - 1 : i == 0)) ea.energy = s->eacc;
   if (i == s->stages - 1) {
-    // last stage: k_last, then m_high (b) and, if adaptive, m_low (b2)
-    ea.out0 = s->kb[i];
+    // last stage: m_high (b) and, if adaptive, m_low (b2); a fixed step
+    // always takes m_high, so its epilogue writes normalize(m_high) into m
+    // (rk.go:444).  k_last is read by the next step's FSAL copy only.
+    ea.out0 = s->fsal ? s->kb[i] : nullptr;
     ea.aux0 = s->m;
-    ea.out1 = s->mnew;
     ea.rk = solver_rk_final(s);
+    ea.rk.norm = !s->adaptive;
+    ea.out1 = s->adaptive ? s->mnew : s->m;
     ea.err = s->adaptive ? s->scratch : nullptr;
     // the precision form keeps float64 for the embedded error norm
     if (s->p.precision && s->adaptive) return launch_zinv<EPI_RK64>(s, ea, st);
-    return launch_zinv<EPI_RK>(s, ea, st);
+    return chain ? launch_zinv_fwd<EPI_RK>(s, ea, st) : launch_zinv<EPI_RK>(s, ea, st);
   }
   ea.out0 = s->kb[i];
   if (i == 0) ea.err = s->scratch + 1;  // max |k0|: the reference's 'torque'
-  return launch_zinv<EPI_TORQUE>(s, ea, st);
+  if (!chain) return launch_zinv<EPI_TORQUE>(s, ea, st);
+  ea.rk = solver_rk_next(s, i);
+  ea.aux0 = i == 0 ? nullptr : s->m;
+  ea.out1 = s->m1;
+  return launch_zinv_fwd<EPI_TORQUE>(s, ea, st);
 }
 
 // renorm_reject: normalise m also when the step was rejected (the host
@@ -790,6 +792,12 @@ static int rk_step(mmx_solver* s, cudaStream_t st) {
   // the thermal noise, fixed for the step's trials (updateTempNoise at the
   // step start, rk.go:289-292; temperature.go:27-36)
   const bool thermal = s->p.thermal_k != 0.f;
+  // each stage goes on to the next one's input; not stage 0 when the dt
+  // bounds may still change dt after it.  The last stage of a fixed step
+  // goes on to the next step's when the caller takes more steps.
+  const bool zc = solver_z_chain(s);
+  bool have_z = s->spec_ready != 0;
+  s->spec_ready = 0;
   s->noise_sigma = thermal ? (float)sqrt((double)f32_div(s->p.thermal_k, s->dt)) : 0.f;
   s->noise_step = s->steps;
   // energy must not rise when it is wanted (rk.go:297-301,425)
@@ -816,8 +824,11 @@ static int rk_step(mmx_solver* s, cudaStream_t st) {
         if (i == 0) MMX_TRY(cudaMemsetAsync(s->scratch + 1, 0, sizeof(float), st));
         if (i == last && s->adaptive) MMX_TRY(cudaMemsetAsync(s->scratch, 0, sizeof(float), st));
         MMX_TRY(cudaMemcpyAsync(dt_dev, &s->dt, sizeof(float), cudaMemcpyHostToDevice, st));
-        cudaError_t e = rk_stage(s, i, st, dt_dev);
+        const bool chain = zc && (i == last ? !s->adaptive && s->more_steps : i > 0 || !(bounds && !thermal));
+        cudaError_t e = rk_stage(s, i, st, dt_dev, have_z, chain);
         if (e != cudaSuccess) { mmx_set_error(cudaGetErrorString(e)); return MMX_ERR_CUDA; }
+        have_z = chain && i < last;
+        if (chain && i == last) s->spec_ready = 1;
         s->fsal_init = 1;
       }
       if (i == 0 && bounds && !thermal) {
@@ -840,8 +851,6 @@ static int rk_step(mmx_solver* s, cudaStream_t st) {
     if (want_e) MMX_TRY(cudaMemcpyAsync(&esum, s->eacc, sizeof(double), cudaMemcpyDeviceToHost, st));
     if (!s->adaptive) {
       good = 1;
-      int one = 1;
-      MMX_TRY(cudaMemcpyAsync(acc_dev, &one, sizeof(int), cudaMemcpyHostToDevice, st));
       if (want_e) {
         MMX_TRY(cudaStreamSynchronize(st));
         s->energy = (float)(esum * (double)solver_cell_volume(s));
@@ -870,6 +879,7 @@ static int rk_step(mmx_solver* s, cudaStream_t st) {
     int accv = good;
     MMX_TRY(cudaMemcpyAsync(acc_dev, &accv, sizeof(int), cudaMemcpyHostToDevice, st));
   }
+  if (!s->adaptive) return MMX_OK;  // the last stage wrote m
   // m <- normalize(m_high) if accepted, else normalize(m)   (rk.go:444)
   k_finalize_accept<<<solver_grid_1d(s->n), 256, 0, st>>>(s->m, s->mnew, s->n, acc_dev);
   MMX_TRY(cudaGetLastError());
@@ -922,12 +932,17 @@ extern "C" int mmx_face_kernel6(const int P[3], const int periodic[3], const flo
   return MMX_OK;
 }
 
+static void free_step_graphs(mmx_solver* s) {
+  if (s->gexec) cudaGraphExecDestroy(s->gexec);
+  if (s->gexec_carry) cudaGraphExecDestroy(s->gexec_carry);
+  s->gexec = s->gexec_carry = nullptr;
+}
 static void free_profile_graph(mmx_solver* s);
 static void solver_free(mmx_solver* s) {
   if (!s) return;
   solver_run_free(s);
   free_profile_graph(s);
-  if (s->gexec) cudaGraphExecDestroy(s->gexec);
+  free_step_graphs(s);
   for (int g = 0; g < 2; g++)
     if (s->dgraph[g]) cudaGraphExecDestroy(s->dgraph[g]);
   cudaFree(s->rkdev);
@@ -1218,6 +1233,8 @@ static cudaError_t rk_device_trial(mmx_solver* s, cudaStream_t st, bool first) {
   RkDev* dev = reinterpret_cast<RkDev*>(s->rkdev);
   const RkCtl c = rk_ctl(s);
   const int last = s->stages - 1;
+  const bool zc = solver_z_chain(s);
+  bool have_z = false;
   cudaError_t e;
   for (int i = 0; i < s->stages; i++) {
     if (i == 0) {
@@ -1226,8 +1243,9 @@ static cudaError_t rk_device_trial(mmx_solver* s, cudaStream_t st, bool first) {
         k_fsal_copy<<<solver_grid_1d(3 * s->n), 256, 0, st>>>(s->kb[0], s->kb[last], 3 * s->n, dev, s->p.faithful,
                                                               s->scratch + 1);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-      } else if ((e = rk_stage(s, 0, st, dt_dev)) != cudaSuccess) {
-        return e;
+      } else {
+        have_z = zc && !c.bounds;
+        if ((e = rk_stage(s, 0, st, dt_dev, false, have_z)) != cudaSuccess) return e;
       }
       if (c.bounds) {
         k_rk_bounds<<<1, 1, 0, st>>>(s->scratch, dev, c);
@@ -1236,7 +1254,8 @@ static cudaError_t rk_device_trial(mmx_solver* s, cudaStream_t st, bool first) {
       continue;
     }
     if (i == last && (e = cudaMemsetAsync(s->scratch, 0, sizeof(float), st)) != cudaSuccess) return e;
-    if ((e = rk_stage(s, i, st, dt_dev)) != cudaSuccess) return e;
+    if ((e = rk_stage(s, i, st, dt_dev, have_z, zc && i < last)) != cudaSuccess) return e;
+    have_z = zc;
   }
   k_rk_control<<<1, 1, 0, st>>>(s->scratch, dev, c);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -1325,24 +1344,19 @@ static bool rk_fixed(const mmx_solver* s) {
 }
 
 // One fixed-step RK step as pure launches (no host traffic), for graph
-// capture: the device dt and accept flag are uploaded beforehand.
-static cudaError_t rk_fixed_launches(mmx_solver* s, cudaStream_t st) {
+// capture: the device dt is uploaded beforehand.  carry: the step starts
+// from the forward Z of m in the spectrum buffer and leaves that of the new m.
+static cudaError_t rk_fixed_launches(mmx_solver* s, cudaStream_t st, bool carry) {
   float* dt_dev = s->scratch + 2;
-  const int* acc_dev = reinterpret_cast<const int*>(s->scratch + 3);
-  for (int i = 0; i < s->stages; i++) {
-    if (i == 0) {
-      cudaError_t e = cudaMemsetAsync(s->scratch + 1, 0, sizeof(float), st);
-      if (e != cudaSuccess) return e;
-    }
-    cudaError_t e = rk_stage(s, i, st, dt_dev);
-    if (e != cudaSuccess) return e;
-  }
-  k_finalize_accept<<<solver_grid_1d(s->n), 256, 0, st>>>(s->m, s->mnew, s->n, acc_dev);
-  return cudaGetLastError();
+  const bool zc = solver_z_chain(s);
+  cudaError_t e = cudaMemsetAsync(s->scratch + 1, 0, sizeof(float), st);
+  for (int i = 0; i < s->stages && e == cudaSuccess; i++)
+    e = rk_stage(s, i, st, dt_dev, i == 0 ? carry : zc, i == s->stages - 1 ? carry : zc);
+  return e;
 }
 
-static cudaError_t step_launches(mmx_solver* s, cudaStream_t st) {
-  return s->p.solver == MMX_SOLVER_HEUN ? heun_step(s, st) : rk_fixed_launches(s, st);
+static cudaError_t step_launches(mmx_solver* s, cudaStream_t st, bool carry = false) {
+  return s->p.solver == MMX_SOLVER_HEUN ? heun_step(s, st) : rk_fixed_launches(s, st, carry);
 }
 
 static void free_profile_graph(mmx_solver* s) {
@@ -1404,55 +1418,59 @@ extern "C" int mmx_solver_step(mmx_solver* s, int nsteps, cudaStream_t st) {
       ((s->p.solver == MMX_SOLVER_HEUN && s->p.max_error == 0.f) || rk_fixed(s)) && s->p.thermal_k == 0.f;
   if (s->profile == 2 && fixed_graphable && !s->want_energy) {
     if (s->p.solver != MMX_SOLVER_HEUN && s->dt_uploaded != s->dt) {
-      float v[2] = {s->dt, 0.f};
-      int one = 1;
-      memcpy(&v[1], &one, sizeof(int));
-      MMX_TRY(cudaMemcpyAsync(s->scratch + 2, v, sizeof(v), cudaMemcpyHostToDevice, st));
+      MMX_TRY(cudaMemcpyAsync(s->scratch + 2, &s->dt, sizeof(float), cudaMemcpyHostToDevice, st));
       MMX_TRY(cudaStreamSynchronize(st));
       s->dt_uploaded = s->dt;
     }
     return profiled_graph_steps(s, nsteps, st);
   }
   bool graphable = s->use_graph && !s->profile && !s->want_energy && fixed_graphable;
-  if (graphable && s->p.solver != MMX_SOLVER_HEUN && s->dt_uploaded != s->dt) {
-    float v[2] = {s->dt, 0.f};
-    int one = 1;
-    memcpy(&v[1], &one, sizeof(int));
-    MMX_TRY(cudaMemcpyAsync(s->scratch + 2, v, sizeof(v), cudaMemcpyHostToDevice, st));
+  const bool rk = s->p.solver != MMX_SOLVER_HEUN;
+  if (graphable && rk && s->dt_uploaded != s->dt) {
+    MMX_TRY(cudaMemcpyAsync(s->scratch + 2, &s->dt, sizeof(float), cudaMemcpyHostToDevice, st));
     MMX_TRY(cudaStreamSynchronize(st));
     s->dt_uploaded = s->dt;
   }
+  // several Runge-Kutta steps in one call hand the forward Z of m from step
+  // to step; each call starts from m itself
+  if (rk) s->spec_ready = 0;
+  const bool carry = rk && graphable && nsteps > 1 && solver_z_chain(s);
+  cudaGraphExec_t& gexec = carry ? s->gexec_carry : s->gexec;
+  cudaStream_t& gstream = carry ? s->gstream_carry : s->gstream;
   for (int k = 0; k < nsteps; k++) {
-    if (graphable && heun_fused(s) && !s->spec_ready) {
+    if (graphable && (heun_fused(s) || carry) && !s->spec_ready) {
       // the captured step expects the forward Z spectrum of m in S
       cudaError_t e = zfwd_only(s, s->m, st);
       if (e != cudaSuccess) { mmx_set_error(cudaGetErrorString(e)); return MMX_ERR_CUDA; }
       s->spec_ready = 1;
     }
     if (graphable) {
-      if (!s->gexec || s->gstream != st) {
-        if (s->gexec) { cudaGraphExecDestroy(s->gexec); s->gexec = nullptr; }
+      if (!gexec || gstream != st) {
+        if (gexec) { cudaGraphExecDestroy(gexec); gexec = nullptr; }
         cudaStream_t cap = st;
         bool own = false;
         if (cap == 0) { MMX_TRY(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking)); own = true; }
         cudaGraph_t g;
         MMX_TRY(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e = step_launches(s, cap);
+        cudaError_t e = step_launches(s, cap, carry);
         cudaError_t e2 = cudaStreamEndCapture(cap, &g);
         if (own) cudaStreamDestroy(cap);
         if (e != cudaSuccess || e2 != cudaSuccess) { mmx_set_error("graph capture failed"); return MMX_ERR_CUDA; }
-        MMX_TRY(cudaGraphInstantiate(&s->gexec, g, 0));
+        MMX_TRY(cudaGraphInstantiate(&gexec, g, 0));
         cudaGraphDestroy(g);
-        s->gstream = st;
+        gstream = st;
       }
-      MMX_TRY(cudaGraphLaunch(s->gexec, st));
+      MMX_TRY(cudaGraphLaunch(gexec, st));
       s->time += (double)s->dt;
     } else {
+      s->more_steps = k + 1 < nsteps;
       int rc = step_once(s, st);
+      s->more_steps = 0;
       if (rc != MMX_OK) return rc;
     }
     s->steps++;
   }
+  if (rk) s->spec_ready = 0;
   if (s->profile) flush_timers(s);
   return MMX_OK;
 }
@@ -1503,7 +1521,7 @@ extern "C" int mmx_solver_state(mmx_solver* s, double* time, float* dt, float* m
 extern "C" int mmx_solver_set_hext(mmx_solver* s, const float hext[3]) {
   if (!s || !hext) { mmx_set_error("null argument"); return MMX_ERR_ARG; }
   for (int d = 0; d < 3; d++) s->p.hext[d] = hext[d];
-  if (s->gexec) { cudaGraphExecDestroy(s->gexec); s->gexec = nullptr; }
+  free_step_graphs(s);
   return MMX_OK;
 }
 
@@ -1513,7 +1531,7 @@ extern "C" float* mmx_solver_torque_device(mmx_solver* s) { return s ? s->scratc
 extern "C" int mmx_solver_use_graph(mmx_solver* s, int on) {
   if (!s) { mmx_set_error("null argument"); return MMX_ERR_ARG; }
   s->use_graph = on;
-  if (!on && s->gexec) { cudaGraphExecDestroy(s->gexec); s->gexec = nullptr; }
+  if (!on) free_step_graphs(s);
   return MMX_OK;
 }
 

@@ -49,7 +49,8 @@ struct mmx_solver {
   float torque = 0, step_error = 0;
   long long steps = 0;
   int fsal_init = 0;
-  int spec_ready = 0;  // S holds the forward Z spectrum of m (fused Heun steps)
+  int spec_ready = 0;  // S holds the forward Z spectrum of m (between Heun steps; RK: within one call)
+  int more_steps = 0;  // the caller takes another step right after this one
   float dt_uploaded = -1.f;  // dt last written to the device scalar by the graph path
   // tableau
   int stages = 0, fsal = 0, adaptive = 0;
@@ -65,6 +66,8 @@ struct mmx_solver {
   int use_graph = 0;
   cudaGraphExec_t gexec = nullptr;
   cudaStream_t gstream = nullptr;
+  cudaGraphExec_t gexec_carry = nullptr;  // fixed RK step that starts and ends with zfwd(m) in S
+  cudaStream_t gstream_carry = nullptr;
   // run loop with table output (run.cu)
   void* runbuf = nullptr;                 // RunDev on the device
   float* rows_dev = nullptr;              // device table rows
@@ -106,6 +109,9 @@ int solver_grid_1d(int64_t n);
 // Runge-Kutta combinations: the input of stage i, and the last stage's.
 ZComb solver_rk_comb(mmx_solver* s, int i, const float* dt_dev);
 RKCoef solver_rk_final(mmx_solver* s);
+RKCoef solver_rk_next(mmx_solver* s, int i);
+// The inverse-Z pass can go on to the next evaluation's forward Z.
+bool solver_z_chain(const mmx_solver* s);
 // h = demag + exchange field of the device array m (no local fields).
 int solver_field_conv(mmx_solver* s, const float* m, float* h, cudaStream_t st);
 // One trial of the device-controlled adaptive RK step (first: no FSAL
