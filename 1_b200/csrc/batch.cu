@@ -442,7 +442,7 @@ static int build_eval(mmx_batch* b, std::vector<Launch>& out, int mode, bool fir
       mmx_solver* s = b->inst[i];
       ZinvArgs z;
       z.S = s->S;
-      z.twz = s->bp.twz;
+      z.fz = s->bp.fz;
       z.twP = s->bp.twz;
       z.P1 = s->P[1];
       z.HZ = s->HZ;

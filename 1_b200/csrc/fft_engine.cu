@@ -23,24 +23,44 @@
 #include "fft_engine.cuh"
 #include "fft_passes.cuh"
 #include "fft_fixed_kernels.cuh"
+#include "fft_mixed.cuh"
+
+// Plans are searched over non-increasing radices: the fewest stages, among
+// those the smallest first radix (more butterflies for the block's threads).
+static void plan_search(int m, int most, int last_max, int depth, int* cur, int* best, int* nbest) {
+  static const int radices[15] = {25, 20, 16, 15, 14, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+  if (m == 1) {
+    if (depth && cur[depth - 1] > last_max) return;
+    if (*nbest < 0 || depth < *nbest || (depth == *nbest && depth && cur[0] < best[0])) {
+      for (int i = 0; i < depth; i++) best[i] = cur[i];
+      *nbest = depth;
+    }
+    return;
+  }
+  if (depth == 8 || (*nbest >= 0 && depth >= *nbest)) return;
+  for (int r : radices) {
+    if (r > most || m % r) continue;
+    cur[depth] = r;
+    plan_search(m / r, r, last_max, depth + 1, cur, best, nbest);
+  }
+}
 
 bool fft_factor(int L, LineFFT* f) {
-  f->L = L;
-  f->nst = 0;
-  f->code = 0;
   int m = L;
-  const int order[6] = {8, 4, 2, 3, 5, 7};
-  const int codes[6] = {5, 2, 0, 1, 3, 4};
-  for (int oi = 0; oi < 6; oi++) {
-    int r = order[oi];
-    while (m % r == 0) {
-      if (f->nst >= FFT_MAX_STAGES) return false;
-      f->code |= (unsigned long long)codes[oi] << (3 * f->nst);
-      f->nst++;
-      m /= r;
-    }
+  for (int p : {2, 3, 5, 7})
+    while (m % p == 0) m /= p;
+  if (m != 1) return false;
+  f->L = L;
+  for (int conv = 0; conv < 2; conv++) {
+    int cur[8], best[8], n = -1;
+    plan_search(L, 25, conv ? 10 : 25, 0, cur, best, &n);
+    if (n < 0) return false;
+    unsigned long long code = 0;
+    for (int i = 0; i < n; i++) code |= (unsigned long long)best[i] << (8 * i);
+    (conv ? f->conv_nst : f->nst) = n;
+    (conv ? f->conv_code : f->code) = code;
   }
-  return m == 1;
+  return true;
 }
 
 static std::mutex g_tw_mu;
@@ -88,22 +108,10 @@ cudaError_t launch_z_r2c(const float* src, float2* dst, const ZPass& zp, cudaStr
 #undef C_
     }
   }
-  int lines = 1;
-  while (M * lines * 2 <= (is_pow2(M) ? 4096 : 2048) && lines * 2 <= zp.nrows) lines *= 2;
-  size_t smem = sizeof(float2) * (size_t)M * lines;
-  dim3 grid(div_up(zp.nrows, lines));
+  if (M > 8192) return cudaErrorInvalidValue;
   ZComb none;
   memset(&none, 0, sizeof(none));
-  SHAPE_DISPATCH(M * lines, is_pow2(M), {
-    if (cb) {
-      allow_smem(k_z_r2c<T, E, P2, true>, smem);
-      k_z_r2c<T, E, P2, true><<<grid, T, smem, st>>>(src, dst, zp, lines, *cb);
-    } else {
-      allow_smem(k_z_r2c<T, E, P2, false>, smem);
-      k_z_r2c<T, E, P2, false><<<grid, T, smem, st>>>(src, dst, zp, lines, none);
-    }
-  });
-  return cudaGetLastError();
+  return cb ? mix::launch_zr2c_mix<true>(src, dst, zp, *cb, st) : mix::launch_zr2c_mix<false>(src, dst, zp, none, st);
 }
 
 cudaError_t launch_z_c2r(const float2* src, float* dst, const ZPass& zp, cudaStream_t st) {
@@ -116,15 +124,7 @@ cudaError_t launch_z_c2r(const float2* src, float* dst, const ZPass& zp, cudaStr
 #undef C_
     }
   }
-  int lines = 1;
-  while ((M + 1) * lines * 2 <= (is_pow2(M) ? 4096 : 2048) && lines * 2 <= zp.nrows) lines *= 2;
-  size_t smem = sizeof(float2) * (size_t)(M + 1) * lines;
-  dim3 grid(div_up(zp.nrows, lines));
-  SHAPE_DISPATCH((M + 1) * lines, is_pow2(M), {
-    allow_smem(k_z_c2r<T, E, P2>, smem);
-    k_z_c2r<T, E, P2><<<grid, T, smem, st>>>(src, dst, zp, lines);
-  });
-  return cudaGetLastError();
+  return M < 8192 ? mix::launch_zc2r_mix(src, dst, zp, st) : cudaErrorInvalidValue;
 }
 
 cudaError_t launch_col(const float2* src, float2* dst, const ColPass& cp, cudaStream_t st) {
@@ -137,15 +137,7 @@ cudaError_t launch_col(const float2* src, float2* dst, const ColPass& cp, cudaSt
 #undef C_
     }
   }
-  int tk = 1;
-  while (tk < 32 && L * tk * 2 <= (is_pow2(L) ? 4096 : 2048) && tk * 2 <= cp.ncols) tk *= 2;
-  size_t smem = sizeof(float2) * (size_t)L * tk;
-  dim3 grid(div_up(cp.ncols, tk), cp.nplanes);
-  SHAPE_DISPATCH(L * tk, is_pow2(L), {
-    allow_smem(k_col<T, E, P2>, smem);
-    k_col<T, E, P2><<<grid, T, smem, st>>>(src, dst, cp, tk);
-  });
-  return cudaGetLastError();
+  return L <= 8192 ? mix::launch_col_mix(src, dst, cp, st) : cudaErrorInvalidValue;
 }
 
 // ---------------------------------------------------------------------

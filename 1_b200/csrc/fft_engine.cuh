@@ -1,12 +1,5 @@
-// Shared-memory mixed-radix Stockham FFT used by every transform of the
-// LLG engine.  A CTA owns a tile of lines in shared memory; each stage
-// reads all of its butterfly inputs into registers, synchronises, applies
-// twiddles and the radix-R DFT, and writes the outputs in Stockham (self
-// sorting) order, so the tile is transformed in place and the result is in
-// natural order.
-//
-// Radices 2, 4, 8 have specialised butterflies; 3, 5, 7 use a constant
-// table DFT.  A line length is any product of these.
+// Line transforms of the LLG engine: the run-time plan of a line and the
+// butterflies the compiled passes (fft_fixed.cuh) use.
 //
 // Twiddles come from a per-length table tw[t] = exp(-2 pi i t / Lt) in
 // float, computed in double on the host; a stage of radix R at span ns
@@ -14,16 +7,13 @@
 #pragma once
 #include "mmx_common.cuh"
 
-#define FFT_MAX_STAGES 16
-
-// Radix codes, 3 bits per stage (kernel parameters must not be indexed
-// with a runtime index, which would copy them to local memory).
-#define FFT_RADIX_OF(code) ((code) == 0 ? 2 : (code) == 1 ? 3 : (code) == 2 ? 4 : (code) == 3 ? 5 : (code) == 4 ? 7 : 8)
-
+// A line length is any product of 2, 3, 5 and 7.  The radix of stage s is
+// byte s of 'code'; the second plan, for the fused convolution, ends with a
+// radix of at most 10.
 struct LineFFT {
   int L;                       // complex length of the line
-  int nst;                     // number of stages
-  unsigned long long code;     // radix code of stage s in bits [3s, 3s+3)
+  int nst, conv_nst;           // number of stages
+  unsigned long long code, conv_code;
   const float2* tw;            // twiddle table, length L * tws
   int tws;                     // table stride (table built for a multiple of L)
 };
@@ -201,127 +191,11 @@ __device__ __forceinline__ void Radix<7>::dft(float2* v, bool inv) {
   odd_dft<7>(v, inv, c, s);
 }
 
-// Division by a runtime constant d through a multiply-high
-// (round-up method; exact for n < 2^31).
-struct FDiv {
-  unsigned d, m, s;
-};
-__host__ __device__ inline FDiv make_fdiv(unsigned d) {
-  FDiv f;
-  f.d = d;
-  unsigned l = 0;
-  while ((1ull << l) < d) l++;
-  f.s = l;
-  f.m = (unsigned)((((1ull << 32) * ((1ull << l) - d)) / d) + 1);
-  return f;
-}
-__device__ __forceinline__ unsigned fdiv(const FDiv& f, unsigned n) { return (__umulhi(f.m, n) + n) >> f.s; }
-
-// Tile addressing: element i of line l lives at s[i * si + l * sl].
-// 'lfast' selects the thread mapping: consecutive threads walk lines
-// (index-major tiles, sl == 1) or indices (line-major tiles, si == 1).
-// POW2: the line length and the line count are powers of two and every
-// radix is 2, 4 or 8, so index arithmetic reduces to shifts and masks
-// (lgL = log2 L, lgl = log2 nlines).
-template <int R, int EPT, bool POW2>
-__device__ __forceinline__ void fft_stage(float2* s, int L, int lgL, int ns, int lgns, int nlines, const FDiv& fl,
-                                          int si, int sl, bool lfast, const float2* __restrict__ tw, int tws,
-                                          bool inv) {
-  constexpr int IT = (EPT + R - 1) / R;
-  constexpr int LGR = R == 2 ? 1 : R == 4 ? 2 : R == 8 ? 3 : 0;
-  const int m = POW2 ? (L >> LGR) : L / R;
-  const int lgm = lgL - LGR;
-  const int total = m * nlines;
-  const int nt = blockDim.x;
-  const int tid = threadIdx.x;
-  float2 v[IT][R];
-  const int tstep = POW2 ? (L >> (lgns + LGR)) : L / (ns * R);
-#pragma unroll
-  for (int it = 0; it < IT; it++) {
-    int item = it * nt + tid;
-    if (item < total) {
-      int l, j;
-      if (lfast) { j = (int)fdiv(fl, (unsigned)item); l = item - j * nlines; }
-      else if (POW2) { j = item & (m - 1); l = item >> lgm; }
-      else { j = item % m; l = item / m; }
-      const float2* src = s + l * sl;
-      int k = POW2 ? (j & (ns - 1)) : j % ns;
-#pragma unroll
-      for (int q = 0; q < R; q++) v[it][q] = src[(j + q * m) * si];
-      if (ns > 1) {
-#pragma unroll
-        for (int q = 1; q < R; q++) {
-          float2 w = __ldg(&tw[(q * k * tstep) * tws]);
-          if (inv) w.y = -w.y;
-          v[it][q] = cmul(v[it][q], w);
-        }
-      }
-      Radix<R>::dft(v[it], inv);
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int it = 0; it < IT; it++) {
-    int item = it * nt + tid;
-    if (item < total) {
-      int l, j;
-      if (lfast) { j = (int)fdiv(fl, (unsigned)item); l = item - j * nlines; }
-      else if (POW2) { j = item & (m - 1); l = item >> lgm; }
-      else { j = item % m; l = item / m; }
-      float2* dst = s + l * sl;
-      int base;
-      if (POW2) base = ((j >> lgns) << (lgns + LGR)) + (j & (ns - 1));
-      else base = (j / ns) * ns * R + j % ns;
-#pragma unroll
-      for (int q = 0; q < R; q++) dst[(base + q * ns) * si] = v[it][q];
-    }
-  }
-  __syncthreads();
-}
-
-// Full transform of every line of the tile (unnormalised).
-template <int EPT, bool POW2>
-__device__ void tile_fft(float2* s, const LineFFT& f, int nlines, int si, int sl, bool lfast, bool inv) {
-  int ns = 1, lgns = 0;
-  int lgL = POW2 ? 31 - __clz(f.L) : 0;
-  const FDiv fl = make_fdiv((unsigned)nlines);
-  const unsigned long long code = f.code;
-  for (int st = 0; st < f.nst; st++) {
-    int c = (int)((code >> (3 * st)) & 7ull);
-    int R = FFT_RADIX_OF(c);
-    if (POW2) {
-      switch (R) {
-        case 8: fft_stage<8, EPT, true>(s, f.L, lgL, ns, lgns, nlines, fl, si, sl, lfast, f.tw, f.tws, inv); break;
-        case 4: fft_stage<4, EPT, true>(s, f.L, lgL, ns, lgns, nlines, fl, si, sl, lfast, f.tw, f.tws, inv); break;
-        default: fft_stage<2, EPT, true>(s, f.L, lgL, ns, lgns, nlines, fl, si, sl, lfast, f.tw, f.tws, inv); break;
-      }
-      lgns += R == 8 ? 3 : R == 4 ? 2 : 1;
-    } else {
-      switch (R) {
-        case 8: fft_stage<8, EPT, false>(s, f.L, 0, ns, 0, nlines, fl, si, sl, lfast, f.tw, f.tws, inv); break;
-        case 4: fft_stage<4, EPT, false>(s, f.L, 0, ns, 0, nlines, fl, si, sl, lfast, f.tw, f.tws, inv); break;
-        case 2: fft_stage<2, EPT, false>(s, f.L, 0, ns, 0, nlines, fl, si, sl, lfast, f.tw, f.tws, inv); break;
-        case 3: fft_stage<3, EPT, false>(s, f.L, 0, ns, 0, nlines, fl, si, sl, lfast, f.tw, f.tws, inv); break;
-        case 5: fft_stage<5, EPT, false>(s, f.L, 0, ns, 0, nlines, fl, si, sl, lfast, f.tw, f.tws, inv); break;
-        case 7: fft_stage<7, EPT, false>(s, f.L, 0, ns, 0, nlines, fl, si, sl, lfast, f.tw, f.tws, inv); break;
-        default: break;
-      }
-    }
-    ns *= R;
-  }
-}
-
-// Launch shapes: THREADS x EPT elements per tile; (256 x 8), (256 x 16)
-// or (512 x 16).  The register budget is 128 per thread in all three.
-#define FFT_BOUNDS(THREADS) __launch_bounds__(THREADS, (THREADS) == 256 ? 2 : 1)
-
-static inline bool is_pow2(int x) { return x > 0 && (x & (x - 1)) == 0; }
-
 // ---------------------------------------------------------------------
 // Host-side plan construction helpers (fft_engine.cu).
 // ---------------------------------------------------------------------
-// Factor L into the supported radices (8 first, then 4, 2, 3, 5, 7).
-// Returns false if L has another prime factor or too many stages.
+// Splits L into as few stages as the radices of fft_mixed.cuh allow.
+// Returns false if L has a prime factor above 7.
 bool fft_factor(int L, LineFFT* f);
 // Device twiddle table exp(-2 pi i t / Lt), t < Lt, cached per length for
 // the lifetime of the process.

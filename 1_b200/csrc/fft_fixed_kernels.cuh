@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(T) k_zc2r_fx(const float2* __restrict__ src, f
 // Inverse Z of the three components of RT spatial rows + the solver epilogue.
 struct ZinvArgs {
   float2* S;
-  const float2* twz;
+  LineFFT fz;
   const float2* twP;
   int P1, HZ;
   int64_t CS;
@@ -507,7 +507,7 @@ __device__ __forceinline__ void zinv_body(const ZinvArgs& za, int bx) {
   const int64_t CS = za.CS;
   const EpiArgs& ea = za.ea;
   constexpr bool QK = rows_qk<M>();
-  load_twiddles_rows<M, T>(tw, za.twz, 2);
+  load_twiddles_rows<M, T>(tw, za.fz.tw, 2);
   const int r0 = bx * RT;
   const int nr = min(RT, nrows - r0);
   const int N1 = ea.N1, N2 = ea.N2;

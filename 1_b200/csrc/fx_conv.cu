@@ -1,6 +1,7 @@
 // The fused convolution passes, compiled for one axis each: FX_D2 = 0 the X
 // axis of a 3D grid, FX_D2 = 1 the Y axis of a film (single grid and batch).
 #include "fx_dispatch.cuh"
+#include "fft_mixed.cuh"
 
 template <int L, int TK, int T, bool D2, bool HALF>
 // at least 768 resident threads per SM (6 blocks of 128 for L = 64):
@@ -67,4 +68,13 @@ cudaError_t CAT_(bx_conv_, FX_D2)(const BatchLaunch& l, cudaStream_t st) {
 #undef C_
   }
   return cudaErrorInvalidValue;
+}
+cudaError_t CAT_(mx_conv_, FX_D2)(const mix::Conv& a, cudaStream_t st) {
+  if (3 * a.f.L > 8192) return cudaErrorInvalidValue;
+  size_t bytes;
+  const int lg = mix::pick_columns(a.f.L, 3, a.f.conv_nst > 1 ? 2 : 0, a.ncols, &bytes);
+  cudaError_t e = mix::allow(mix::k_conv_mix<FX_D2 != 0>, bytes);
+  if (e != cudaSuccess) return e;
+  mix::k_conv_mix<FX_D2 != 0><<<div_up(a.ncols, 1 << lg), mix::T_COL, bytes, st>>>(a, lg);
+  return cudaGetLastError();
 }

@@ -7,7 +7,11 @@
 // fused convolution pass: X axis of a 3D grid (fx_conv_0), Y axis of a film (fx_conv_1)
 cudaError_t fx_conv_0(int L, const ConvArgs& a, cudaStream_t st);
 cudaError_t fx_conv_1(int L, const ConvArgs& a, cudaStream_t st);
-// the same over a batch's instances (half: every instance's data fill half the line)
+// the same for other line lengths
+namespace mix { struct Conv; }
+cudaError_t mx_conv_0(const mix::Conv& a, cudaStream_t st);
+cudaError_t mx_conv_1(const mix::Conv& a, cudaStream_t st);
+// the compiled passes over a batch's instances (half: every instance's data fill half the line)
 struct BatchLaunch {
   int L, nseg, blocks, half, variant, flag;
   const void* args;
@@ -17,7 +21,8 @@ cudaError_t bx_conv_0(const BatchLaunch& l, cudaStream_t st);
 cudaError_t bx_conv_1(const BatchLaunch& l, cudaStream_t st);
 cudaError_t bx_col(const BatchLaunch& l, cudaStream_t st);    // flag: inverse
 cudaError_t bx_zr2c(const BatchLaunch& l, cudaStream_t st);   // flag: with the stage combination
-// inverse Z with an epilogue (EPI_*); fuse: followed by the next evaluation's forward Z
+// inverse Z with an epilogue (EPI_*), any line length for a single grid;
+// fuse: followed by the next evaluation's forward Z
 #define FX_ZINV_DECL(MODE)                                                                \
   cudaError_t fx_zinv_##MODE(int M, const ZinvArgs& za, bool fuse, cudaStream_t st);      \
   cudaError_t bx_zinv_##MODE(const BatchLaunch& l, bool fuse, cudaStream_t st);

@@ -1,6 +1,7 @@
 // The inverse Z passes with one epilogue each (FX_MODE, an EPI_* value):
 // plain and followed by the next evaluation's forward Z, single grid and batch.
 #include "fx_dispatch.cuh"
+#include "fft_mixed.cuh"
 
 template <int M, int RT, int T, int MODE>
 __global__ void __launch_bounds__(T) k_zinv_fx(ZinvArgs za) {
@@ -49,9 +50,30 @@ static cudaError_t launch_batch(const BatchLaunch& l, bool fuse, cudaStream_t st
   return cudaErrorInvalidValue;
 }
 
+// line lengths without compiled kernels
+template <int MODE>
+static cudaError_t launch_mix(const ZinvArgs& za, bool fuse, cudaStream_t st) {
+  const int M = za.fz.L;
+  if (3 * (M + 1) > 8192) return cudaErrorInvalidValue;
+  size_t bytes;
+  const int rt = mix::pick_rows(M, 3, za.nrows, &bytes);
+  auto go = [&](auto kern) {
+    cudaError_t e = mix::allow(kern, bytes);
+    if (e != cudaSuccess) return e;
+    kern<<<div_up(za.nrows, rt), mix::T_ROW, bytes, st>>>(za.S, za.fz, za.twP, za.P1, za.HZ, za.CS, za.nrows, za.ea,
+                                                          rt);
+    return cudaGetLastError();
+  };
+  if constexpr (IN_STEP) {
+    if (fuse) return go(mix::k_zinv_mix<MODE, true>);
+  }
+  return fuse ? cudaErrorInvalidValue : go(mix::k_zinv_mix<MODE, false>);
+}
+
 #define CAT2_(a, b) a##b
 #define CAT_(a, b) CAT2_(a, b)
 cudaError_t CAT_(fx_zinv_, FX_MODE)(int M, const ZinvArgs& za, bool fuse, cudaStream_t st) {
+  if (!fx_ok(M)) return launch_mix<FX_MODE>(za, fuse, st);
   switch (M) {
 #define C_(LL) \
   case LL: return launch<LL>(za, fuse, st);

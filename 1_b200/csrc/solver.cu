@@ -30,6 +30,7 @@
 #include "llg_ops.cuh"
 #include "epilogue.cuh"
 #include "kernmul.cuh"
+#include "fft_mixed.cuh"
 #include "fx_dispatch.cuh"
 #include "solver_state.cuh"
 #include "../../include/mmx.h"
@@ -61,172 +62,6 @@ __global__ void k_extract_octant(const float2* __restrict__ spec, float* __restr
     int kx = (int)(e / ((int64_t)HZ * O1));
     kh[e] = __fmul_rn(spec[((int64_t)kx * P1 + ky) * HZ + kz].x, norm);
   }
-}
-
-// ---------------------------------------------------------------------
-// Xconv (3D): columns (ky, kz) flattened, tile of tk columns x 3 comps.
-// Tile layout: element x of line (c, t) at sm[x * 3tk + c * tk + t].
-// ---------------------------------------------------------------------
-template <int THREADS, int EPT, bool POW2>
-__global__ void FFT_BOUNDS(THREADS) k_xconv(float2* __restrict__ S, LineFFT fx, KernOct K, int N0, int P1, int HZ,
-                                               int64_t CS, int tk) {
-  extern __shared__ float2 sm[];
-  const int P0 = fx.L;
-  const int ncol = P1 * HZ;
-  const int col0 = blockIdx.x * tk;
-  const int nc = min(tk, ncol - col0);
-  const int nl = 3 * tk;
-  const int64_t plane = (int64_t)P1 * HZ;
-  for (int e = threadIdx.x; e < P0 * nl; e += THREADS) {
-    int i = e / nl, l = e - i * nl;
-    int c = l / tk, t = l - c * tk;
-    float2 v = make_float2(0.f, 0.f);
-    if (i < N0 && t < nc) v = S[c * CS + i * plane + col0 + t];
-    sm[e] = v;
-  }
-  __syncthreads();
-  tile_fft<EPT, POW2>(sm, fx, nl, nl, 1, true, false);
-  for (int e = threadIdx.x; e < P0 * tk; e += THREADS) {
-    int kx = e / tk, t = e - kx * tk;
-    if (t >= nc) continue;
-    int col = col0 + t;
-    int ky = col / HZ, kz = col - ky * HZ;
-    float Kxx, Kyy, Kzz, Kyz, Kxz, Kxy;
-    kern_at(K, kx, ky, kz, Kxx, Kyy, Kzz, Kyz, Kxz, Kxy);
-    float2* b = sm + kx * nl + t;
-    float2 mx = b[0], my = b[tk], mz = b[2 * tk];
-    kmul6(mx, my, mz, Kxx, Kyy, Kzz, Kyz, Kxz, Kxy);
-    b[0] = mx;
-    b[tk] = my;
-    b[2 * tk] = mz;
-  }
-  __syncthreads();
-  tile_fft<EPT, POW2>(sm, fx, nl, nl, 1, true, true);
-  for (int e = threadIdx.x; e < N0 * nl; e += THREADS) {
-    int i = e / nl, l = e - i * nl;
-    int c = l / tk, t = l - c * tk;
-    if (t < nc) S[c * CS + i * plane + col0 + t] = sm[e];
-  }
-}
-
-// Yconv (2D, N0 = P0 = 1): columns kz, tile of tk columns x 3 comps.
-template <int THREADS, int EPT, bool POW2>
-__global__ void FFT_BOUNDS(THREADS) k_yconv2d(float2* __restrict__ S, LineFFT fy, KernOct K, int N1, int HZ,
-                                                 int64_t CS, int tk) {
-  extern __shared__ float2 sm[];
-  const int P1 = fy.L;
-  const int kz0 = blockIdx.x * tk;
-  const int nc = min(tk, HZ - kz0);
-  const int nl = 3 * tk;
-  for (int e = threadIdx.x; e < P1 * nl; e += THREADS) {
-    int i = e / nl, l = e - i * nl;
-    int c = l / tk, t = l - c * tk;
-    float2 v = make_float2(0.f, 0.f);
-    if (i < N1 && t < nc) v = S[c * CS + (int64_t)i * HZ + kz0 + t];
-    sm[e] = v;
-  }
-  __syncthreads();
-  tile_fft<EPT, POW2>(sm, fy, nl, nl, 1, true, false);
-  for (int e = threadIdx.x; e < P1 * tk; e += THREADS) {
-    int ky = e / tk, t = e - ky * tk;
-    if (t >= nc) continue;
-    float Kxx, Kyy, Kzz, Kyz, Kxz, Kxy;
-    kern_at(K, 0, ky, kz0 + t, Kxx, Kyy, Kzz, Kyz, Kxz, Kxy);
-    float2* b = sm + ky * nl + t;
-    float2 mx = b[0], my = b[tk], mz = b[2 * tk];
-    kmul4(mx, my, mz, Kxx, Kyy, Kzz, Kyz);
-    b[0] = mx;
-    b[tk] = my;
-    b[2 * tk] = mz;
-  }
-  __syncthreads();
-  tile_fft<EPT, POW2>(sm, fy, nl, nl, 1, true, true);
-  for (int e = threadIdx.x; e < N1 * nl; e += THREADS) {
-    int i = e / nl, l = e - i * nl;
-    int c = l / tk, t = l - c * tk;
-    if (t < nc) S[c * CS + (int64_t)i * HZ + kz0 + t] = sm[e];
-  }
-}
-
-// ---------------------------------------------------------------------
-// Zi + epilogue: inverse Z (C2R) of the three components of R rows in
-// shared memory, then the per-cell solver update.
-// ---------------------------------------------------------------------
-template <int THREADS, int EPT, bool POW2, int MODE>
-__global__ void FFT_BOUNDS(THREADS) k_zinv_epi(const float2* __restrict__ S, LineFFT fz,
-                                                  const float2* __restrict__ twP, int N0, int P1, int HZ, int64_t CS,
-                                                  int rows, int nrows_total, EpiArgs ea) {
-  extern __shared__ float2 sm[];
-  const int M = fz.L;
-  const int ld = M + 1;
-  const int nl = 3 * rows;
-  const int nt = THREADS;
-  const int r0 = blockIdx.x * rows;
-  const int nr = min(rows, nrows_total - r0);
-  const int N1 = ea.N1, N2 = ea.N2;
-  for (int e = threadIdx.x; e < nl * ld; e += nt) {
-    int l = e / ld, k = e - l * ld;
-    int r = l / 3, c = l - 3 * r;
-    float2 v = make_float2(0.f, 0.f);
-    if (r < nr) {
-      int gr = r0 + r;
-      int x = gr / N1, y = gr - x * N1;
-      v = S[c * CS + ((int64_t)x * P1 + y) * HZ + k];
-      if (k == 0 || k == M) v.y = 0.f;
-    }
-    sm[e] = v;
-  }
-  __syncthreads();
-  {
-    float2 v[EPT];
-#pragma unroll
-    for (int it = 0; it < EPT; it++) {
-      int e = it * nt + threadIdx.x;
-      if (e < nl * M) {
-        int l = e / M, k = e - l * M;
-        float2 Xk = sm[l * ld + k], Xm = sm[l * ld + (M - k)];
-        float2 A = make_float2(Xk.x + Xm.x, Xk.y - Xm.y);
-        float2 B = make_float2(Xk.x - Xm.x, Xk.y + Xm.y);
-        float2 w = __ldg(&twP[k]);
-        w.y = -w.y;
-        float2 C = cmul(B, w);
-        v[it] = make_float2(A.x - C.y, A.y + C.x);
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int it = 0; it < EPT; it++) {
-      int e = it * nt + threadIdx.x;
-      if (e < nl * M) {
-        int l = e / M, k = e - l * M;
-        sm[l * ld + k] = v[it];
-      }
-    }
-    __syncthreads();
-  }
-  tile_fft<EPT, POW2>(sm, fz, nl, 1, ld, false, true);
-
-  float lmax = 0.f;
-  double eacc = 0.0;
-  constexpr int C = 4;
-  for (int e0 = threadIdx.x; e0 < nr * N2; e0 += C * nt) {
-    EpiIn<MODE, false> in[C];
-    int64_t g[C];
-    float h[C][3];
-#pragma unroll
-    for (int i = 0; i < C; i++) {
-      const int e = e0 + i * nt;
-      g[i] = e < nr * N2 ? (int64_t)r0 * N2 + e : -1;
-      if (g[i] < 0) continue;
-      epi_load<MODE, false>(ea, g[i], in[i]);
-      const int r = e / N2, z = e - r * N2;
-      const float* base = reinterpret_cast<const float*>(sm + (r * 3) * ld + (z >> 1)) + (z & 1);
-#pragma unroll
-      for (int c = 0; c < 3; c++) h[i][c] = base[2 * c * ld];
-    }
-    epi_cells<MODE, false, C>(ea, g, h, in, lmax, eacc);
-  }
-  epi_flush_max<MODE>(ea, lmax, eacc);
 }
 
 // ---------------------------------------------------------------------
@@ -383,32 +218,38 @@ static void flush_timers(mmx_solver* s) {
   }
 }
 
-static cudaError_t launch_xconv(mmx_solver* s, cudaStream_t st) {
-  int P0 = s->P[0];
-  if (fx_ok(P0)) {
+// the fused convolution along X (3D) or Y (a film) with the given line
+static cudaError_t launch_conv(mmx_solver* s, bool d2, const LineFFT& f, int n_data, int ncols, int64_t stride,
+                               cudaStream_t st) {
+  if (fx_ok(f.L)) {
     ConvArgs a;
     a.S = s->S;
     a.K = s->K;
-    a.n_data = s->N[0];
-    a.ncols = s->P[1] * s->HZ;
+    a.n_data = n_data;
+    a.ncols = ncols;
     a.HZ = s->HZ;
-    a.stride = (int64_t)s->P[1] * s->HZ;
+    a.stride = stride;
     a.CS = s->CS;
-    a.tw = s->bp.fx.tw;
-    a.tws = s->bp.fx.tws;
-    ScopedPass sp(s, "xconv", st);
-    return fx_conv_0(P0, a, st);
+    a.tw = f.tw;
+    a.tws = f.tws;
+    return d2 ? fx_conv_1(f.L, a, st) : fx_conv_0(f.L, a, st);
   }
-  int tk = 1;
-  while (tk < 32 && P0 * 3 * tk * 2 <= (is_pow2(P0) ? 4096 : 2048)) tk *= 2;
-  size_t smem = sizeof(float2) * (size_t)P0 * 3 * tk;
-  int ncol = s->P[1] * s->HZ;
+  mix::Conv a;
+  a.S = s->S;
+  a.K = s->K;
+  a.f = f;
+  a.n_data = n_data;
+  a.ncols = ncols;
+  a.HZ = s->HZ;
+  a.stride = stride;
+  a.CS = s->CS;
+  return d2 ? mx_conv_1(a, st) : mx_conv_0(a, st);
+}
+
+static cudaError_t launch_xconv(mmx_solver* s, cudaStream_t st) {
+  const int64_t plane = (int64_t)s->P[1] * s->HZ;
   ScopedPass sp(s, "xconv", st);
-  SHAPE_DISPATCH(P0 * 3 * tk, is_pow2(P0), {
-    allow_smem(k_xconv<T, E, P2>, smem);
-    k_xconv<T, E, P2><<<div_up(ncol, tk), T, smem, st>>>(s->S, s->bp.fx, s->K, s->N[0], s->P[1], s->HZ, s->CS, tk);
-  });
-  return cudaGetLastError();
+  return launch_conv(s, false, s->bp.fx, s->N[0], (int)plane, plane, st);
 }
 
 int mmx_yconv2d_tc_launch(float2* S, int64_t CS, int HZ, int N1, const float* kt, int* err, cudaStream_t st);
@@ -416,42 +257,20 @@ int mmx_yconv2d_tc_prepare();
 int mmx_yconv2d_tc_kernel(const float* kh, int64_t kcs, int HZ, float** kt);
 
 static cudaError_t launch_yconv2d(mmx_solver* s, cudaStream_t st) {
-  int P1 = s->P[1];
   if (s->p.precision) {
     ScopedPass sp(s, "yconv2d_tc", st);
     int rc = mmx_yconv2d_tc_launch(s->S, s->CS, s->HZ, s->N[1], s->kt_tc, reinterpret_cast<int*>(s->scratch + 15),
                                    st);
     return rc == MMX_OK ? cudaSuccess : cudaErrorLaunchFailure;
   }
-  if (fx_ok(P1)) {
-    ConvArgs a;
-    a.S = s->S;
-    a.K = s->K;
-    a.n_data = s->N[1];
-    a.ncols = s->HZ;
-    a.HZ = s->HZ;
-    a.stride = s->HZ;
-    a.CS = s->CS;
-    a.tw = s->bp.fy.tw;
-    a.tws = s->bp.fy.tws;
-    ScopedPass sp(s, "yconv2d", st);
-    return fx_conv_1(P1, a, st);
-  }
-  int tk = 1;
-  while (tk < 32 && P1 * 3 * tk * 2 <= (is_pow2(P1) ? 4096 : 2048) && tk * 2 <= s->HZ) tk *= 2;
-  size_t smem = sizeof(float2) * (size_t)P1 * 3 * tk;
   ScopedPass sp(s, "yconv2d", st);
-  SHAPE_DISPATCH(P1 * 3 * tk, is_pow2(P1), {
-    allow_smem(k_yconv2d<T, E, P2>, smem);
-    k_yconv2d<T, E, P2><<<div_up(s->HZ, tk), T, smem, st>>>(s->S, s->bp.fy, s->K, s->N[1], s->HZ, s->CS, tk);
-  });
-  return cudaGetLastError();
+  return launch_conv(s, true, s->bp.fy, s->N[1], s->HZ, s->HZ, st);
 }
 
 static ZinvArgs zinv_args(mmx_solver* s, const EpiArgs& ea) {
   ZinvArgs za;
   za.S = s->S;
-  za.twz = s->bp.twz;
+  za.fz = s->bp.fz;
   za.twP = s->bp.twz;
   za.P1 = s->P[1];
   za.HZ = s->HZ;
@@ -463,19 +282,8 @@ static ZinvArgs zinv_args(mmx_solver* s, const EpiArgs& ea) {
 
 template <int MODE>
 static cudaError_t launch_zinv(mmx_solver* s, const EpiArgs& ea, cudaStream_t st) {
-  int M = s->P[2] / 2;
-  int nrows = s->N[0] * s->N[1];
   ScopedPass sp(s, "zinv_epi", st);
-  if (fx_ok(M)) return fx_zinv(MODE, M, zinv_args(s, ea), false, st);
-  int rows = 1;
-  while (3 * (rows * 2) * (M + 1) <= (is_pow2(M) ? 4096 : 2048) && rows * 2 <= nrows) rows *= 2;
-  size_t smem = sizeof(float2) * (size_t)3 * rows * (M + 1);
-  SHAPE_DISPATCH(3 * rows * (M + 1), is_pow2(M), {
-    allow_smem(k_zinv_epi<T, E, P2, MODE>, smem);
-    k_zinv_epi<T, E, P2, MODE><<<div_up(nrows, rows), T, smem, st>>>(s->S, s->bp.fz, s->bp.twz, s->N[0], s->P[1],
-                                                                        s->HZ, s->CS, rows, nrows, ea);
-  });
-  return cudaGetLastError();
+  return fx_zinv(MODE, s->P[2] / 2, zinv_args(s, ea), false, st);
 }
 
 // inverse Z + epilogue + the next evaluation's forward Z in one pass
@@ -485,13 +293,11 @@ static cudaError_t launch_zinv_fwd(mmx_solver* s, const EpiArgs& ea, cudaStream_
   return fx_zinv(MODE, s->P[2] / 2, zinv_args(s, ea), true, st);
 }
 
-// With an open Z boundary and a compiled Z length the inverse-Z pass can go
-// on to the forward Z of the magnetisation it has just produced (the next
+// With an open Z boundary the inverse-Z pass can go on to the forward Z of the magnetisation it has just produced (the next
 // evaluation's input is in its tile): the forward Z pass, its reads of m and
 // of the stage torques, and one launch per evaluation go away.
 bool solver_z_chain(const mmx_solver* s) {
-  int M = s->P[2] / 2;
-  return s->N[2] == M && s->p.periodic[2] == 0 && fx_ok(M);
+  return s->N[2] == s->P[2] / 2 && s->p.periodic[2] == 0;
 }
 // Fixed-step Heun: the spectrum buffer holds zfwd(m) between steps (spec_ready).
 static bool heun_fused(const mmx_solver* s) {
