@@ -234,7 +234,8 @@ __host__ __device__ constexpr int odd_up(int n) { return n | 1; }
 // ---------------------------------------------------------------------
 constexpr int T_COL = 128;
 
-static __global__ void __launch_bounds__(T_COL, 4) k_col_mix(const float2* src, float2* dst, ColPass cp, int lg) {
+template <int = 0>  // instantiated where it is launched
+__global__ void __launch_bounds__(T_COL, 4) k_col_mix(const float2* src, float2* dst, ColPass cp, int lg) {
   extern __shared__ float2 sm[];
   const int TK = 1 << lg, TKP = odd_up(TK), L = cp.f.L, nst = cp.f.nst;
   const int l = threadIdx.x & (TK - 1), j0 = threadIdx.x >> lg, dj = T_COL >> lg;
@@ -421,7 +422,8 @@ __device__ __forceinline__ int at(int i) { return i + (i >> 4); }
 // the stages of 'lines' rows from tile x, with tile y to alternate; elements
 // from 'limit' on are zero in the first stage.  Returns the tile that holds
 // the result.  Called with x complete, returns after a barrier.
-static __device__ __noinline__ float2* row_stages(float2* x, float2* y, const LineFFT& f, int lines, int pitch, int limit) {
+template <int = 0>
+__device__ __noinline__ float2* row_stages(float2* x, float2* y, const LineFFT& f, int lines, int pitch, int limit) {
   const int L = f.L, nst = f.nst;
   int ns = 1;
   for (int st = 0; st < nst; st++) {
@@ -580,7 +582,8 @@ __device__ __forceinline__ void load_merged(float2* x, int lines, int M, int pit
   }
 }
 
-static __global__ void __launch_bounds__(T_ROW) k_zc2r_mix(const float2* __restrict__ src, float* __restrict__ dst, ZPass z,
+template <int = 0>
+__global__ void __launch_bounds__(T_ROW) k_zc2r_mix(const float2* __restrict__ src, float* __restrict__ dst, ZPass z,
                                                     int RT) {
   extern __shared__ float2 sm[];
   __shared__ int64_t roff_s[MAX_ROWS], soff_s[MAX_ROWS];
@@ -704,12 +707,13 @@ static inline int pick_rows(int M, int lines_per_row, int nrows, size_t* bytes) 
   return rt;
 }
 
-static inline cudaError_t launch_col_mix(const float2* src, float2* dst, const ColPass& cp, cudaStream_t st) {
+template <int = 0>
+cudaError_t launch_col_mix(const float2* src, float2* dst, const ColPass& cp, cudaStream_t st) {
   size_t bytes;
   const int lg = pick_columns(cp.f.L, 1, cp.f.nst > 2 ? 2 : 1, (int64_t)cp.ncols * cp.nplanes, &bytes);
-  cudaError_t e = allow(k_col_mix, bytes);
+  cudaError_t e = allow(k_col_mix<>, bytes);
   if (e != cudaSuccess) return e;
-  k_col_mix<<<div_up((int64_t)cp.ncols * cp.nplanes, 1 << lg), T_COL, bytes, st>>>(src, dst, cp, lg);
+  k_col_mix<><<<div_up((int64_t)cp.ncols * cp.nplanes, 1 << lg), T_COL, bytes, st>>>(src, dst, cp, lg);
   return cudaGetLastError();
 }
 template <bool COMB>
@@ -723,12 +727,13 @@ static cudaError_t launch_zr2c_mix(const float* src, float2* dst, const ZPass& z
   k_zr2c_mix<COMB><<<div_up(z.nrows, rt), T_ROW, bytes, st>>>(src, dst, z, cb, vec2, rt);
   return cudaGetLastError();
 }
-static inline cudaError_t launch_zc2r_mix(const float2* src, float* dst, const ZPass& z, cudaStream_t st) {
+template <int = 0>
+cudaError_t launch_zc2r_mix(const float2* src, float* dst, const ZPass& z, cudaStream_t st) {
   size_t bytes;
   const int rt = pick_rows(z.f.L, 1, z.nrows, &bytes);
-  cudaError_t e = allow(k_zc2r_mix, bytes);
+  cudaError_t e = allow(k_zc2r_mix<>, bytes);
   if (e != cudaSuccess) return e;
-  k_zc2r_mix<<<div_up(z.nrows, rt), T_ROW, bytes, st>>>(src, dst, z, rt);
+  k_zc2r_mix<><<<div_up(z.nrows, rt), T_ROW, bytes, st>>>(src, dst, z, rt);
   return cudaGetLastError();
 }
 

@@ -23,16 +23,6 @@
 #include "solver_state.cuh"
 #include "../../include/mmx.h"
 
-struct RunDev {
-  double stop;              // internal time to stop at
-  long long iters, max_iters;
-  float unit_time, period, since, t;
-  int save, nrows, max_rows, pad;
-  double sum[3];
-  unsigned int kmin, kmax;  // ordered keys of min / max of component 0
-  float* rows;
-};
-
 // float <-> unsigned key with the order of the floats (both signs)
 __device__ __forceinline__ unsigned int order_key(float f) {
   unsigned int u = __float_as_uint(f);
@@ -42,23 +32,27 @@ __device__ __forceinline__ float order_key_inv(unsigned int k) {
   return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
-// Periodic.NeedSave at a step boundary (after an accepted trial) of the
-// device-controlled solver (simrun.go:27-35, simoutput.go:83-85)
-__global__ void k_run_check(RunDev* __restrict__ rd, const RkDev* __restrict__ dev) {
-  float t = __fmul_rn(__double2float_rn(dev->time), rd->unit_time);
-  rd->t = t;
-  rd->save = dev->accept && (t == 0.f || __fsub_rn(t, rd->since) >= rd->period);
-}
-
 // the host decided to save at time t (host-driven loop)
 __global__ void k_run_force(RunDev* __restrict__ rd, float t) {
   rd->t = t;
   rd->save = 1;
 }
 
-// per-component sums (float64) and min / max of component 0
-__global__ void k_run_rowsum(RunDev* __restrict__ rd, const float* __restrict__ m, int64_t n) {
-  if (!rd->save) return;
+// One table row if one is due (Table.Save, simoutput.go:226-272): per-component
+// sums (float64) and min / max of component 0, written by the last block to
+// finish.  Device-controlled runs (dev): every block decides for itself, from
+// Periodic.NeedSave at a step boundary after an accepted trial
+// (simrun.go:27-35, simoutput.go:83-85); host-driven ones: k_run_force did.
+__global__ void k_run_row(RunDev* __restrict__ rd, const RkDev* __restrict__ dev, const float* __restrict__ m,
+                          int64_t n, const float* __restrict__ torque) {
+  float now;
+  if (dev) {
+    now = __fmul_rn(__double2float_rn(dev->time), rd->unit_time);
+    if (!(dev->accept && (now == 0.f || __fsub_rn(now, rd->since) >= rd->period))) return;
+  } else {
+    if (!rd->save) return;
+    now = rd->t;
+  }
   double v[3] = {0.0, 0.0, 0.0};
   float lo = INFINITY, hi = -INFINITY;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -79,34 +73,36 @@ __global__ void k_run_rowsum(RunDev* __restrict__ rd, const float* __restrict__ 
     atomicMin(&rd->kmin, order_key(lo));
     atomicMax(&rd->kmax, order_key(hi));
   }
-}
-
-// writes the row (Table.Save, simoutput.go:226-272) and resets the sums
-__global__ void k_run_rowfin(RunDev* __restrict__ rd, const float* __restrict__ torque, int64_t n) {
-  if (!rd->save) return;
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  __threadfence();
+  if (atomicAdd(&rd->done, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  rd->done = 0u;
+  double sum[3];
+  for (int c = 0; c < 3; c++)
+    sum[c] = __longlong_as_double((long long)atomicExch(reinterpret_cast<unsigned long long*>(&rd->sum[c]), 0ull));
+  const unsigned int kmin = atomicExch(&rd->kmin, 0xffffffffu), kmax = atomicExch(&rd->kmax, 0u);
   if (rd->nrows < rd->max_rows) {
     float* r = rd->rows + 7 * (int64_t)rd->nrows;
     const double dn = (double)n;
-    r[0] = rd->t;
-    r[1] = (float)(rd->sum[2] / dn);  // user x = internal Z
-    r[2] = (float)(rd->sum[1] / dn);
-    r[3] = (float)(rd->sum[0] / dn);  // user z = internal X
+    r[0] = now;
+    r[1] = (float)(sum[2] / dn);  // user x = internal Z
+    r[2] = (float)(sum[1] / dn);
+    r[3] = (float)(sum[0] / dn);  // user z = internal X
     r[4] = torque ? *torque : 0.f;
-    r[5] = order_key_inv(rd->kmin);
-    r[6] = order_key_inv(rd->kmax);
+    r[5] = order_key_inv(kmin);
+    r[6] = order_key_inv(kmax);
     rd->nrows++;
   }
-  rd->since = rd->t;
-  rd->sum[0] = rd->sum[1] = rd->sum[2] = 0.0;
-  rd->kmin = 0xffffffffu;
-  rd->kmax = 0u;
+  rd->since = now;
   rd->save = 0;
 }
 
-// loop condition of the run graph: time < stop, no NaN, under the cap
-__global__ void k_run_cond(RunDev* __restrict__ rd, const RkDev* __restrict__ dev, cudaGraphConditionalHandle h,
-                           int count) {
-  if (count) rd->iters++;
+// condition before the first iteration of the run graph: time < stop, no NaN,
+// under the cap (each trial's end sets the next one, k_rk_finish)
+__global__ void k_run_cond(const RunDev* __restrict__ rd, const RkDev* __restrict__ dev,
+                           cudaGraphConditionalHandle h) {
   const int go = dev->time < rd->stop && !dev->bad && rd->iters < rd->max_iters;
   cudaGraphSetConditional(h, go ? 1u : 0u);
 }
@@ -183,16 +179,15 @@ static int run_buffers(mmx_solver* s, int max_rows) {
   return MMX_OK;
 }
 
-// the row reduction launches (after k_run_check or k_run_force)
-static cudaError_t row_launches(mmx_solver* s, RunDev* rd, cudaStream_t st) {
-  const float* torque = s->p.solver == MMX_SOLVER_HEUN ? nullptr : s->scratch + 1;
-  k_run_rowsum<<<solver_grid_1d(s->n), 256, 0, st>>>(rd, s->m, s->n);
-  k_run_rowfin<<<1, 1, 0, st>>>(rd, torque, s->n);
+// the row reduction; dev: the device controller whose time decides, else k_run_force came before
+static cudaError_t row_launch(mmx_solver* s, RunDev* rd, const RkDev* dev, cudaStream_t st) {
+  const float* torque = dev ? &dev->torque : s->p.solver == MMX_SOLVER_HEUN ? nullptr : s->scratch + 1;
+  k_run_row<<<solver_grid_1d(s->n), 256, 0, st>>>(rd, dev, s->m, s->n, torque);
   return cudaGetLastError();
 }
 
 // outer graph: the loop condition, then a WHILE node whose body is
-// {row check, row reduction, one FSAL trial, loop condition}
+// {row reduction where one is due, one FSAL trial, which sets the loop condition}
 static int build_run_graph(mmx_solver* s, cudaStream_t st) {
   if (s->rungraph && s->rungraph_stream == st) return MMX_OK;
   if (s->rungraph) { cudaGraphExecDestroy(s->rungraph); s->rungraph = nullptr; }
@@ -205,8 +200,7 @@ static int build_run_graph(mmx_solver* s, cudaStream_t st) {
   do {
     cudaGraphConditionalHandle h;
     if (cudaGraphConditionalHandleCreate(&h, g, 0, 0) != cudaSuccess) { rc = MMX_ERR_CUDA; break; }
-    int zero = 0;
-    void* args[4] = {&rd, &dev, &h, &zero};
+    void* args[3] = {&rd, &dev, &h};
     cudaKernelNodeParams kp;
     memset(&kp, 0, sizeof(kp));
     kp.func = (void*)k_run_cond;
@@ -228,13 +222,9 @@ static int build_run_graph(mmx_solver* s, cudaStream_t st) {
     if (cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking) != cudaSuccess) { rc = MMX_ERR_CUDA; break; }
     if (cudaStreamBeginCaptureToGraph(cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal) !=
         cudaSuccess) { rc = MMX_ERR_CUDA; break; }
-    k_run_check<<<1, 1, 0, cap>>>(rd, dev);
-    cudaError_t e = row_launches(s, rd, cap);
-    if (e == cudaSuccess) e = solver_device_trial(s, cap, false);
-    if (e == cudaSuccess) {
-      k_run_cond<<<1, 1, 0, cap>>>(rd, dev, h, 1);
-      e = cudaGetLastError();
-    }
+    const RunLoop loop = {rd, h};
+    cudaError_t e = row_launch(s, rd, dev, cap);
+    if (e == cudaSuccess) e = solver_device_trial(s, cap, false, &loop);
     cudaGraph_t out = nullptr;
     cudaError_t e2 = cudaStreamEndCapture(cap, &out);
     if (e != cudaSuccess || e2 != cudaSuccess) { rc = MMX_ERR_CUDA; break; }
@@ -284,7 +274,7 @@ extern "C" int mmx_solver_run(mmx_solver* s, double seconds, float period, float
       volatile float d = t - s->since;
       if (t == 0.f || d >= period) {
         k_run_force<<<1, 1, 0, st>>>(rd, t);
-        MMX_TRY(row_launches(s, rd, st));
+        MMX_TRY(row_launch(s, rd, nullptr, st));
         s->since = t;
       }
       MMX_CHECK_RC(mmx_solver_step(s, 1, st));
@@ -293,8 +283,7 @@ extern "C" int mmx_solver_run(mmx_solver* s, double seconds, float period, float
   } else if (s->time < stop) {
     if (s->fsal && !s->fsal_init) {
       // the first trial evaluates stage 0 itself: run it outside the loop
-      k_run_check<<<1, 1, 0, st>>>(rd, reinterpret_cast<const RkDev*>(s->rkdev));
-      MMX_TRY(row_launches(s, rd, st));
+      MMX_TRY(row_launch(s, rd, reinterpret_cast<const RkDev*>(s->rkdev), st));
       MMX_CHECK_RC(mmx_solver_step(s, 1, st));
     }
     MMX_CHECK_RC(build_run_graph(s, st));

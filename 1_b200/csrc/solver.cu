@@ -505,7 +505,8 @@ static cudaError_t rk_stage(mmx_solver* s, int i, cudaStream_t st, float* dt_dev
     return chain ? launch_zinv_fwd<EPI_RK>(s, ea, st) : launch_zinv<EPI_RK>(s, ea, st);
   }
   ea.out0 = s->kb[i];
-  if (i == 0) ea.err = s->scratch + 1;  // max |k0|: the reference's 'torque'
+  // max |k0|: the reference's 'torque'
+  if (i == 0) ea.err = s->devctl ? &reinterpret_cast<RkDev*>(s->rkdev)->tmax : s->scratch + 1;
   if (!chain) return launch_zinv<EPI_TORQUE>(s, ea, st);
   ea.rk = solver_rk_next(s, i);
   ea.aux0 = i == 0 ? nullptr : s->m;
@@ -513,13 +514,11 @@ static cudaError_t rk_stage(mmx_solver* s, int i, cudaStream_t st, float* dt_dev
   return launch_zinv_fwd<EPI_TORQUE>(s, ea, st);
 }
 
-// renorm_reject: normalise m also when the step was rejected (the host
-// controller's end of a step whose every trial failed); the device
-// controller leaves m untouched on a rejected trial and retries.
+// The end of a host-controlled step: normalize(m_high), or normalize(m) when
+// every trial was rejected.
 __global__ void k_finalize_accept(float* __restrict__ m, const float* __restrict__ mnew, int64_t n,
-                                  const int* __restrict__ accept, int renorm_reject = 1) {
-  bool acc = *accept != 0;
-  if (!acc && !renorm_reject) return;
+                                  const int* __restrict__ accept) {
+  const bool acc = *accept != 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     float x, y, z;
     if (acc) { x = mnew[i]; y = mnew[n + i]; z = mnew[2 * n + i]; }
@@ -952,22 +951,26 @@ static int step_once(mmx_solver* s, cudaStream_t st) {
 // ---------------------------------------------------------------------
 // Device-side controller of the adaptive RK solvers (mmx_solver_device_control).
 // One trial of RK.step (rk.go:279-445) is a fixed launch sequence captured
-// once as a CUDA graph: FSAL copy k0 <- k_last (a copy instead of the host
-// path's pointer swap), the stages (their dt read from device memory),
-// then a one-thread controller that applies rk.go's float32 rules --
-// factor = (maxErr/err)^(1/order) clamped to [0.01, 2], reject when
-// err > 2 maxErr, the min/max dt clamps -- accumulates the time in float64
-// and flags acceptance for the finalisation.  A rejected trial leaves m
-// untouched; the next replay retries with the reduced dt.  No host
-// synchronisation per step.
+// once as a CUDA graph: the stages (their dt read from device memory), then
+// one kernel (k_rk_finish) that applies rk.go's float32 rules -- factor =
+// (maxErr/err)^(1/order) clamped to [0.01, 2], reject when err > 2 maxErr,
+// the min/max dt clamps --, accumulates the time in float64, writes the
+// accepted m, and for FSAL tableaux prepares the next trial: k0 <- k_last (a
+// copy instead of the host path's pointer swap), its maximum, and the dt
+// bounds that follow from it.  A rejected trial leaves m untouched; the next
+// replay retries with the reduced dt.  No host synchronisation per step.
+//
+// On a small film a trial is bound by the number of its launches: with the
+// copy, the bounds, the controller, the finalisation and two clears as nodes
+// of their own a 128 x 32 film's RK23 trial was 13 nodes (17 in the run
+// loop) and 60 us.
 // ---------------------------------------------------------------------
 __global__ void k_fsal_copy(float* __restrict__ k0, const float* __restrict__ klast, int64_t n3,
-                            const RkDev* __restrict__ dev, int faithful, float* __restrict__ torque) {
-  const bool copy = dev->accept || faithful;  // rk.go:311-315 (retry: faithful reuses the rejected k_last)
+                            float* __restrict__ torque) {
   float lmax = 0.f;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n3; i += (int64_t)gridDim.x * blockDim.x) {
-    float v = copy ? klast[i] : k0[i];
-    if (copy) k0[i] = v;
+    const float v = klast[i];
+    k0[i] = v;
     lmax = fmaxf(lmax, fabsf(v));
   }
   for (int o = 16; o > 0; o >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
@@ -980,32 +983,71 @@ struct RkCtl {
   int bounds;
 };
 
-// dt bounds from the maximum torque of stage 0 (rk.go:348-373)
-__global__ void k_rk_bounds(float* __restrict__ scratch, RkDev* __restrict__ dev, RkCtl c) {
-  float mt = scratch[1];
-  float dt = scratch[2];
-  float dm = __fmul_rn(dt, mt);
+// dt within the bounds that the maximum torque of stage 0 gives (rk.go:348-373)
+__device__ __forceinline__ float rk_bounded(float dt, float mt, const RkCtl& c) {
+  const float dm = __fmul_rn(dt, mt);
   if (dm < c.min_dm) dt = __fdiv_rn(c.min_dm, mt);
   if (__fmul_rn(dt, c.unit_time) < c.min_dt) dt = __fdiv_rn(c.min_dt, c.unit_time);
   if (c.max_dm != 0.f && dm > c.max_dm) dt = __fdiv_rn(c.max_dm, mt);
   if (c.max_dt != 0.f && __fmul_rn(dt, c.unit_time) > c.max_dt) dt = __fdiv_rn(c.max_dt, c.unit_time);
+  return dt;
+}
+// the same for a trial that evaluates stage 0 itself
+__global__ void k_rk_bounds(float* __restrict__ scratch, RkDev* __restrict__ dev, RkCtl c) {
+  const float dt = rk_bounded(dev->dt, dev->tmax, c);
   if (dt != dt) dev->bad = 1;
   scratch[2] = dt;
-  dev->dt = dt;
 }
 
-// the error rule of rk.go:401-439 in float32; time in float64
-__global__ void k_rk_control(float* __restrict__ scratch, RkDev* __restrict__ dev, RkCtl c) {
+// The end of a trial.  Every block takes the accept decision from the error
+// and moves its cells; the last block to finish updates the controller.
+__global__ void k_rk_finish(float* __restrict__ m, const float* __restrict__ mnew, float* __restrict__ k0,
+                            const float* __restrict__ klast, int64_t n, float* __restrict__ scratch,
+                            RkDev* __restrict__ dev, RkCtl c, int fsal, int faithful, RunDev* __restrict__ rd,
+                            cudaGraphConditionalHandle h) {
   const float err = scratch[0];
+  const bool acc = !(err > __fmul_rn(2.f, c.max_error));
+  const bool copy = fsal && (acc || faithful);  // rk.go:311-315 (retry: faithful reuses the rejected k_last)
+  float lmax = 0.f;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    if (acc) {
+      float x = mnew[i], y = mnew[n + i], z = mnew[2 * n + i];
+      llg_normalize(x, y, z);
+      m[i] = x;
+      m[n + i] = y;
+      m[2 * n + i] = z;
+    }
+    if (copy) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        const float v = klast[d * n + i];
+        k0[d * n + i] = v;
+        lmax = fmaxf(lmax, fabsf(v));
+      }
+    }
+  }
+  if (copy) {
+    for (int o = 16; o > 0; o >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
+    if ((threadIdx.x & 31) == 0) atomic_max_nonneg(&dev->tacc, lmax);
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  __threadfence();
+  if (atomicAdd(&dev->done, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  dev->done = 0u;
+  // the error rule of rk.go:401-439 in float32; time in float64
   const float dt = scratch[2];
   float factor = (float)pow((double)__fdiv_rn(c.max_error, err), c.inv_order);
   if (factor > 2.f) factor = 2.f;
   if (factor < 0.01f) factor = 0.01f;
   float nd = __fmul_rn(dt, factor);
-  if (nd != nd || err != err) dev->bad = 1;
-  int acc = !(err > __fmul_rn(2.f, c.max_error));
+  int bad = dev->bad;
+  if (nd != nd || err != err) bad = 1;
+  double time = dev->time;
   if (acc) {
-    dev->time += (double)dt;
+    time += (double)dt;
+    dev->time = time;
     dev->accepted++;
     if (__fmul_rn(nd, c.unit_time) < c.min_dt) nd = __fdiv_rn(c.min_dt, c.unit_time);
     if (c.max_dt != 0.f && __fmul_rn(nd, c.unit_time) > c.max_dt) nd = __fdiv_rn(c.max_dt, c.unit_time);
@@ -1013,10 +1055,28 @@ __global__ void k_rk_control(float* __restrict__ scratch, RkDev* __restrict__ de
   dev->trials++;
   dev->accept = acc;
   dev->err = err;
-  dev->torque = scratch[1];
   dev->dt = nd;
+  scratch[0] = 0.f;
+  float t = dev->tmax;
+  scratch[1] = dev->torque = t;
+  scratch[3] = __int_as_float(acc ? 1 : 0);
+  // the next trial's stage 0
+  if (copy) {
+    t = __uint_as_float(atomicExch(reinterpret_cast<unsigned int*>(&dev->tacc), 0u));
+    dev->tmax = t;
+  } else if (!fsal) {
+    dev->tmax = 0.f;
+  }
+  if (fsal && c.bounds) {
+    nd = rk_bounded(nd, t, c);
+    if (nd != nd) bad = 1;
+  }
   scratch[2] = nd;
-  reinterpret_cast<int*>(scratch)[3] = acc;
+  dev->bad = bad;
+  if (rd) {
+    const long long iters = ++rd->iters;
+    cudaGraphSetConditional(h, time < rd->stop && !bad && iters < rd->max_iters ? 1u : 0u);
+  }
 }
 
 static RkCtl rk_ctl(const mmx_solver* s) {
@@ -1033,9 +1093,8 @@ static RkCtl rk_ctl(const mmx_solver* s) {
 }
 
 // one trial; first: stage 0 evaluated (no FSAL value yet)
-static cudaError_t rk_device_trial(mmx_solver* s, cudaStream_t st, bool first) {
+static cudaError_t rk_device_trial(mmx_solver* s, cudaStream_t st, bool first, const RunLoop* loop) {
   float* dt_dev = s->scratch + 2;
-  const int* acc_dev = reinterpret_cast<const int*>(s->scratch + 3);
   RkDev* dev = reinterpret_cast<RkDev*>(s->rkdev);
   const RkCtl c = rk_ctl(s);
   const int last = s->stages - 1;
@@ -1044,28 +1103,22 @@ static cudaError_t rk_device_trial(mmx_solver* s, cudaStream_t st, bool first) {
   cudaError_t e;
   for (int i = 0; i < s->stages; i++) {
     if (i == 0) {
-      if ((e = cudaMemsetAsync(s->scratch + 1, 0, sizeof(float), st)) != cudaSuccess) return e;
-      if (s->fsal && !first) {
-        k_fsal_copy<<<solver_grid_1d(3 * s->n), 256, 0, st>>>(s->kb[0], s->kb[last], 3 * s->n, dev, s->p.faithful,
-                                                              s->scratch + 1);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-      } else {
-        have_z = zc && !c.bounds;
-        if ((e = rk_stage(s, 0, st, dt_dev, false, have_z)) != cudaSuccess) return e;
-      }
+      if (s->fsal && !first) continue;  // k_rk_finish left k0, its maximum and the bounded dt
+      if (s->fsal && (e = cudaMemsetAsync(&dev->tmax, 0, sizeof(float), st)) != cudaSuccess) return e;
+      have_z = zc && !c.bounds;
+      if ((e = rk_stage(s, 0, st, dt_dev, false, have_z)) != cudaSuccess) return e;
       if (c.bounds) {
         k_rk_bounds<<<1, 1, 0, st>>>(s->scratch, dev, c);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
       }
       continue;
     }
-    if (i == last && (e = cudaMemsetAsync(s->scratch, 0, sizeof(float), st)) != cudaSuccess) return e;
     if ((e = rk_stage(s, i, st, dt_dev, have_z, zc && i < last)) != cudaSuccess) return e;
     have_z = zc;
   }
-  k_rk_control<<<1, 1, 0, st>>>(s->scratch, dev, c);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  k_finalize_accept<<<solver_grid_1d(s->n), 256, 0, st>>>(s->m, s->mnew, s->n, acc_dev, 0);
+  k_rk_finish<<<solver_grid_1d(s->n), 256, 0, st>>>(s->m, s->mnew, s->kb[0], s->kb[last], s->n, s->scratch, dev, c,
+                                                    s->fsal, s->p.faithful, loop ? loop->rd : nullptr,
+                                                    loop ? loop->h : 0);
   return cudaGetLastError();
 }
 
@@ -1084,7 +1137,9 @@ static int rk_device_download(mmx_solver* s) {
   return MMX_OK;
 }
 
-cudaError_t solver_device_trial(mmx_solver* s, cudaStream_t st, bool first) { return rk_device_trial(s, st, first); }
+cudaError_t solver_device_trial(mmx_solver* s, cudaStream_t st, bool first, const RunLoop* loop) {
+  return rk_device_trial(s, st, first, loop);
+}
 int solver_device_download(mmx_solver* s) { return rk_device_download(s); }
 
 extern "C" int mmx_solver_device_control(mmx_solver* s, int on) {
@@ -1107,8 +1162,20 @@ extern "C" int mmx_solver_device_control(mmx_solver* s, int on) {
     h.time = s->time;
     h.dt = s->dt;
     h.accept = 1;
+    // host steps may still run on any stream
+    MMX_TRY(cudaDeviceSynchronize());
     MMX_TRY(cudaMemcpy(s->rkdev, &h, sizeof(h), cudaMemcpyHostToDevice));
-    MMX_TRY(cudaMemcpy(s->scratch + 2, &s->dt, sizeof(float), cudaMemcpyHostToDevice));
+    const float sc[3] = {0.f, s->torque, s->dt};
+    MMX_TRY(cudaMemcpy(s->scratch, sc, sizeof(sc), cudaMemcpyHostToDevice));
+    if (s->fsal && s->fsal_init) {
+      // the trial that follows the host's last step: k0 <- k_last, and its bounds
+      RkDev* dev = reinterpret_cast<RkDev*>(s->rkdev);
+      const RkCtl c = rk_ctl(s);
+      k_fsal_copy<<<solver_grid_1d(3 * s->n), 256>>>(s->kb[0], s->kb[s->stages - 1], 3 * s->n, &dev->tmax);
+      if (c.bounds) k_rk_bounds<<<1, 1>>>(s->scratch, dev, c);
+      MMX_TRY(cudaGetLastError());
+      MMX_TRY(cudaDeviceSynchronize());
+    }
     s->steps_base = s->steps;
     s->devctl = 1;
   } else if (!on && s->devctl) {
@@ -1130,7 +1197,7 @@ static int rk_device_steps(mmx_solver* s, int n, cudaStream_t st) {
       if (cap == 0) { MMX_TRY(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking)); own = true; }
       cudaGraph_t gr;
       MMX_TRY(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-      cudaError_t e = rk_device_trial(s, cap, g == 0);
+      cudaError_t e = rk_device_trial(s, cap, g == 0, nullptr);
       cudaError_t e2 = cudaStreamEndCapture(cap, &gr);
       if (own) cudaStreamDestroy(cap);
       if (e != cudaSuccess || e2 != cudaSuccess) { mmx_set_error("graph capture failed"); return MMX_ERR_CUDA; }

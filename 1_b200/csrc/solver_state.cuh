@@ -24,6 +24,21 @@ struct RkDev {
   long long accepted, trials;
   float torque, err;
   int bad;
+  float tmax;         // max |k0| of the trial that runs or comes next
+  float tacc;         // the same being collected for the next trial (FSAL copy)
+  unsigned int done;  // blocks of the running reduction that have finished
+};
+
+// Device side of Sim.Run (run.cu): the loop's bounds and the table rows.
+struct RunDev {
+  double stop;              // internal time to stop at
+  long long iters, max_iters;
+  float unit_time, period, since, t;
+  int save, nrows, max_rows;
+  unsigned int done;        // blocks of the row reduction that have finished
+  double sum[3];
+  unsigned int kmin, kmax;  // ordered keys of min / max of component 0
+  float* rows;
 };
 
 struct mmx_solver {
@@ -116,7 +131,12 @@ bool solver_z_chain(const mmx_solver* s);
 int solver_field_conv(mmx_solver* s, const float* m, float* h, cudaStream_t st);
 // One trial of the device-controlled adaptive RK step (first: no FSAL
 // value yet), as plain launches on st (capturable).
-cudaError_t solver_device_trial(mmx_solver* s, cudaStream_t st, bool first);
+// With 'loop' the trial ends by setting the run loop's condition.
+struct RunLoop {
+  RunDev* rd;
+  cudaGraphConditionalHandle h;
+};
+cudaError_t solver_device_trial(mmx_solver* s, cudaStream_t st, bool first, const RunLoop* loop = nullptr);
 // Reads the device controller's time, dt and step counts back (syncs).
 int solver_device_download(mmx_solver* s);
 // Frees the run loop's buffers and graph (run.cu).
