@@ -191,15 +191,15 @@ static int col_tiles(int L, int ncols, int nplanes, int variant) {
   }
   return div_up(ncols * nplanes, tk);
 }
-static int conv_tiles(int L, int ncols) {
-  int tk = 1;
+static int conv_blocks(int L, int ncols, bool d2) {
+  int tk = 1, per = 1;
   switch (L) {
 #define C_(LL) \
-  case LL: tk = conv_tkp_narrow(LL); break;
+  case LL: tk = conv_tkp_narrow(LL); per = d2 && conv_split(LL, conv_tkp_narrow(LL)) ? 2 : 1; break;
     FX_SIZES(C_)
 #undef C_
   }
-  return div_up(ncols, tk);
+  return div_up(ncols, tk) * per;
 }
 static int zrows_per_tile(int M, int lines_per_row) {
   switch (M) {
@@ -421,7 +421,7 @@ static int build_eval(mmx_batch* b, std::vector<Launch>& out, int mode, bool fir
           c.tws = s->bp.fx.tws;
         }
         a.push_back(c);
-        t.push_back(conv_tiles(g.first, c.ncols));
+        t.push_back(conv_blocks(g.first, c.ncols, d2 != 0));
       }
       if ((rc = add_launch(b, out, L_CONV, g.first, d2, a, t)) != MMX_OK) return rc;
       out.back().inst = g.second;

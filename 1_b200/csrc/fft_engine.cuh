@@ -103,9 +103,7 @@ __device__ __forceinline__ void Radix<16>::dft(float2* v, bool inv) {
 // Radix-R DFTs whose upper half of inputs is zero (a zero-padded line's
 // first stage): the zero terms are never added.
 template <int R>
-__device__ __forceinline__ void dft_half(float2* v, bool inv) {
-  Radix<R>::dft(v, inv);
-}
+__device__ __forceinline__ void dft_half(float2* v, bool inv);
 template <>
 __device__ __forceinline__ void dft_half<8>(float2* v, bool inv) {
   // DFT4 of [a, b, 0, 0] = (a + b, a + W4 b, a - b, a - W4 b)
@@ -146,49 +144,6 @@ __device__ __forceinline__ void dft_half<16>(float2* v, bool inv) {
     v[k] = cadd(e[k], t);
     v[k + 8] = csub(e[k], t);
   }
-}
-
-// Odd radices: direct DFT with constant twiddles cos/sin(2 pi k / R).
-template <int R>
-__device__ __forceinline__ void odd_dft(float2* v, bool inv, const float* c, const float* s) {
-  float2 out[R];
-#pragma unroll
-  for (int o = 0; o < R; o++) {
-    float2 acc = v[0];
-#pragma unroll
-    for (int q = 1; q < R; q++) {
-      int t = (o * q) % R;
-      float2 w = make_float2(c[t], inv ? s[t] : -s[t]);
-      float2 p = cmul(v[q], w);
-      acc = cadd(acc, p);
-    }
-    out[o] = acc;
-  }
-#pragma unroll
-  for (int o = 0; o < R; o++) v[o] = out[o];
-}
-
-template <>
-__device__ __forceinline__ void Radix<3>::dft(float2* v, bool inv) {
-  const float c[3] = {1.f, -0.5f, -0.5f};
-  const float s[3] = {0.f, 0.86602540378443864676f, -0.86602540378443864676f};
-  odd_dft<3>(v, inv, c, s);
-}
-template <>
-__device__ __forceinline__ void Radix<5>::dft(float2* v, bool inv) {
-  const float c[5] = {1.f, 0.30901699437494742410f, -0.80901699437494742410f, -0.80901699437494742410f,
-                      0.30901699437494742410f};
-  const float s[5] = {0.f, 0.95105651629515357212f, 0.58778525229247312917f, -0.58778525229247312917f,
-                      -0.95105651629515357212f};
-  odd_dft<5>(v, inv, c, s);
-}
-template <>
-__device__ __forceinline__ void Radix<7>::dft(float2* v, bool inv) {
-  const float c[7] = {1.f, 0.62348980185873353053f, -0.22252093395631440429f, -0.90096886790241912624f,
-                      -0.90096886790241912624f, -0.22252093395631440429f, 0.62348980185873353053f};
-  const float s[7] = {0.f, 0.78183148246802980871f, 0.97492791218182360702f, 0.43388373911755812048f,
-                      -0.43388373911755812048f, -0.97492791218182360702f, -0.78183148246802980871f};
-  odd_dft<7>(v, inv, c, s);
 }
 
 // ---------------------------------------------------------------------

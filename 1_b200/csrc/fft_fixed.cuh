@@ -9,13 +9,13 @@
 // store straight to global memory (pruned outputs are not stored), so a
 // transform of R^s points makes s-1 round trips through shared memory.
 //
-// Radix plan: radix-16 or radix-8 stages first, then 4 or 2, then 3, 5, 7
-// (a line length is any product of these); the inverse applies the stages in
+// Radix plan: radix-16 or radix-8 stages first, then 4 or 2; lines of 3 * 2^k
+// end with a radix of 6 or 12; the inverse applies the stages in
 // reverse order, so that the last forward stage and the first inverse stage
 // group the same elements in the same thread (the kernel multiplication
 // between them stays in registers).
 #pragma once
-#include "fft_engine.cuh"
+#include "fft_dft.cuh"
 
 // FMA complex multiply (the transforms need not be bit-reproducible against
 // a CPU, only deterministic, which a fixed instruction sequence is)
@@ -27,17 +27,22 @@ __device__ __forceinline__ float2 cmulc_f(float2 a, float2 b) {  // a * conj(b)
 }
 
 __host__ __device__ constexpr int ilog2c(int x) { return x <= 1 ? 0 : 1 + ilog2c(x >> 1); }
-// Radix plan of a line length L = 2^a 3^b 5^c 7^d: radix 8 while 8 divides
-// the rest, then 4 or 2, then the odd radices.
-__host__ __device__ constexpr int first_radix8(int L) {
-  return L % 8 == 0 ? 8 : L % 4 == 0 ? 4 : L % 2 == 0 ? 2 : L % 3 == 0 ? 3 : L % 5 == 0 ? 5 : 7;
-}
+// Radix plan of a line length L = 2^k: radix 8 while 8 divides the rest, then
+// 4 or 2.
+__host__ __device__ constexpr int first_radix8(int L) { return L % 8 == 0 ? 8 : L % 4 == 0 ? 4 : 2; }
 __host__ __device__ constexpr int n_stages8(int L) { return L <= 1 ? 0 : 1 + n_stages8(L / first_radix8(L)); }
+// L = 3 2^k: the factor 3 goes into the last stage's radix, 6 or 12, which
+// saves a stage over a radix-3 stage of its own (192 = 16 * 12 instead of
+// 8 * 8 * 3, 384 = 8 * 8 * 6 instead of 8 * 8 * 2 * 3, 3072 = 16 * 16 * 12
+// instead of 16 * 8 * 8 * 3).
+__host__ __device__ constexpr int first_radix3(int L) {
+  return L <= 12 ? L : L == 24 ? 4 : L == 192 || L >= 1536 ? 16 : 8;
+}
 // Radix 16 first when it saves a stage (one shared-memory round trip),
 // e.g. 256 = 16*16 instead of 8*8*4.
 __host__ __device__ constexpr int n_stages(int L);
 __host__ __device__ constexpr int first_radix(int L) {
-  return (L % 16 == 0 && 1 + n_stages(L / 16) < n_stages8(L)) ? 16 : first_radix8(L);
+  return L % 3 == 0 ? first_radix3(L) : (L % 16 == 0 && 1 + n_stages(L / 16) < n_stages8(L)) ? 16 : first_radix8(L);
 }
 __host__ __device__ constexpr int n_stages(int L) { return L <= 1 ? 0 : 1 + n_stages(L / first_radix(L)); }
 // radix of forward stage st
@@ -102,7 +107,21 @@ struct St {
 
 template <int R>
 __device__ __forceinline__ void dft(float2* v, bool inv) {
-  Radix<R>::dft(v, inv);
+  if constexpr (R % 3 == 0) {
+    // the inverse is the forward transform with real and imaginary parts exchanged
+    float2 t[R];
+#pragma unroll
+    for (int q = 0; q < R; q++) t[q] = inv ? make_float2(v[q].y, v[q].x) : v[q];
+    mix::Dft<R>::run(t);
+#pragma unroll
+    for (int q = 0; q < R; q++) v[q] = inv ? make_float2(t[q].y, t[q].x) : t[q];
+  } else {
+    Radix<R>::dft(v, inv);
+  }
+}
+template <int R>
+__device__ __forceinline__ void dft_half(float2* v, bool inv) {
+  dft<R>(v, inv);
 }
 
 // Generic smem-to-smem stage over a tile: element (l, i) at s[i*SI + l*SL].
@@ -145,12 +164,6 @@ struct MidStages {
     }
   }
 };
-
-// Full transform of the tile in shared memory (all stages smem to smem).
-template <int L, int TK, int T, bool LFAST, int SI, int SL, bool INV>
-__device__ __forceinline__ void tile_fft_fixed(float2* s, const float2* tw) {
-  MidStages<L, 0, n_stages(L), TK, T, LFAST, SI, SL, INV>::run(s, tw);
-}
 
 // ---------------------------------------------------------------------
 // Row tiles: NLINES lines of L stored row-major with one float2 of padding

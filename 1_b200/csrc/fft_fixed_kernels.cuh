@@ -26,7 +26,9 @@ __device__ __forceinline__ void col_body(const float2* src, float2* dst, const C
   extern __shared__ float2 sm[];
   constexpr int NST = n_stages(L);
   constexpr int TKP = odd_pitch(TK);
+  pass_begin();
   load_twiddles<L, T>(tw, cp.f.tw, cp.f.tws);
+  pass_wait();
   // Tiles run over the flattened columns of all planes: column g is column
   // g % ncols of plane g / ncols, so a tile may straddle two planes and no
   // tile at the end of a plane is left mostly empty.
@@ -142,6 +144,11 @@ struct ConvArgs {
 template <int L, int R, int NS, int TK, int T>
 using St3 = St<L, R, NS, TK, T, true>;  // (t, j) butterflies, components looped inside
 
+// A film's kernel couples only the components y and z (Kxy = Kxz = 0), so
+// its blocks can come in two kinds, components 1 and 2 and component 0 (see
+// conv_split for where they do).
+__host__ __device__ constexpr int conv_comps(bool split) { return split ? 2 : 3; }
+
 // HALF: the line holds data in its lower half only (n_data = L/2, the
 // open-boundary case): the first stage skips the zero half and the last
 // inverse stage computes only the stored half.
@@ -151,19 +158,22 @@ using St3 = St<L, R, NS, TK, T, true>;  // (t, j) butterflies, components looped
 // only: there the X convolution gains more (75.3 -> 72.7 us on the 256 x 256
 // x 32 grid) than the inverse Y pass loses by reading its input from DRAM
 // (38.2 -> 39.2 us).
-template <int L, int TK, int T, bool D2, bool HALF, bool STREAM = false>
-__device__ __forceinline__ void conv_body(const ConvArgs& a, int bx) {
+// C0, NC: the components of the block.  tw: L twiddles in shared memory.
+template <int L, int TK, int T, bool D2, int C0, int NC, bool HALF, bool STREAM = false>
+__device__ __forceinline__ void conv_body(const ConvArgs& a, int bx, float2* tw) {
   auto sload = [](const float2* p) -> float2 { return STREAM ? __ldcs(p) : *p; };
   auto sstore = [](float2* p, float2 v) {
     if (STREAM) __stcs(p, v);
     else *p = v;
   };
-  __shared__ float2 tw[L];
   extern __shared__ float2 sm[];
   constexpr int NST = n_stages(L);
-  constexpr int NL = 3 * TK;
+  constexpr int NL = NC * TK;
   constexpr int NLP = odd_pitch(NL);
+  float2* const S = a.S + C0 * a.CS;
+  pass_begin();
   load_twiddles<L, T>(tw, a.tw, a.tws);
+  pass_wait();
   const int col0 = bx * TK;
   const int nc = min(TK, a.ncols - col0);
   const int nd = a.n_data;
@@ -174,7 +184,7 @@ __device__ __forceinline__ void conv_body(const ConvArgs& a, int bx) {
   constexpr int RL = fwd_radix(L, NST - 1);
   constexpr int NSL = fwd_span(L, NST - 1);
   using SL = St3<L, RL, NSL, TK, T>;
-  float2 v[SL::NB][3][RL];
+  float2 v[SL::NB][NC][RL];
   if constexpr (NST == 1) {
 #pragma unroll
     for (int i = 0; i < S0::NB; i++) {
@@ -182,11 +192,11 @@ __device__ __forceinline__ void conv_body(const ConvArgs& a, int bx) {
       int t, j;
       S0::lj(i, t, j);
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
+      for (int c = 0; c < NC; c++) {
 #pragma unroll
         for (int q = 0; q < R0; q++) {
           int idx = S0::in_idx(j, q);
-          v[i][c][q] = ((HALF ? q < R0 / 2 : idx < nd) && t < nc) ? sload(&a.S[c * a.CS + idx * a.stride + col0 + t])
+          v[i][c][q] = ((HALF ? q < R0 / 2 : idx < nd) && t < nc) ? sload(&S[c * a.CS + idx * a.stride + col0 + t])
                                                                   : make_float2(0.f, 0.f);
         }
         if (HALF) dft_half<R0>(v[i][c], false);
@@ -194,18 +204,18 @@ __device__ __forceinline__ void conv_body(const ConvArgs& a, int bx) {
       }
     }
   } else {
-    float2 u[S0::NB][3][R0];
+    float2 u[S0::NB][NC][R0];
 #pragma unroll
     for (int i = 0; i < S0::NB; i++) {
       if (!S0::valid(i)) continue;
       int t, j;
       S0::lj(i, t, j);
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
+      for (int c = 0; c < NC; c++) {
 #pragma unroll
         for (int q = 0; q < R0; q++) {
           int idx = S0::in_idx(j, q);
-          u[i][c][q] = ((HALF ? q < R0 / 2 : idx < nd) && t < nc) ? sload(&a.S[c * a.CS + idx * a.stride + col0 + t])
+          u[i][c][q] = ((HALF ? q < R0 / 2 : idx < nd) && t < nc) ? sload(&S[c * a.CS + idx * a.stride + col0 + t])
                                                                   : make_float2(0.f, 0.f);
         }
         if (HALF) dft_half<R0>(u[i][c], false);
@@ -222,7 +232,7 @@ __device__ __forceinline__ void conv_body(const ConvArgs& a, int bx) {
       int t, j;
       SL::lj(i, t, j);
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
+      for (int c = 0; c < NC; c++) {
 #pragma unroll
         for (int q = 0; q < RL; q++) v[i][c][q] = sm[SL::in_idx(j, q) * NLP + c * TK + t];
         SL::twiddle(v[i][c], j, tw, false);
@@ -245,7 +255,13 @@ __device__ __forceinline__ void conv_body(const ConvArgs& a, int bx) {
     for (int q = 0; q < RL; q++) {
       int k = SL::out_idx(j, q);
       float Kxx, Kyy, Kzz, Kyz, Kxz, Kxy;
-      if (D2) {
+      if constexpr (NC == 1) {
+        kern_at(a.K, 0, k, kzc, Kxx, Kyy, Kzz, Kyz, Kxz, Kxy);
+        v[i][0][q] = make_float2(v[i][0][q].x * Kxx, v[i][0][q].y * Kxx);
+      } else if constexpr (NC == 2) {
+        kern_at(a.K, 0, k, kzc, Kxx, Kyy, Kzz, Kyz, Kxz, Kxy);
+        kmul2_fma(v[i][0][q], v[i][1][q], Kyy, Kzz, Kyz);
+      } else if constexpr (D2) {
         kern_at(a.K, 0, k, kzc, Kxx, Kyy, Kzz, Kyz, Kxz, Kxy);
         kmul4_fma(v[i][0][q], v[i][1][q], v[i][2][q], Kxx, Kyy, Kzz, Kyz);
       } else {
@@ -262,12 +278,12 @@ __device__ __forceinline__ void conv_body(const ConvArgs& a, int bx) {
       int t, j;
       SL::lj(i, t, j);
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
+      for (int c = 0; c < NC; c++) {
         dft<RL>(v[i][c], true);
 #pragma unroll
         for (int q = 0; q < RL; q++) {
           int idx = SL::out_idx(j, q);
-          if ((HALF ? q < RL / 2 : idx < nd) && t < nc) sstore(&a.S[c * a.CS + idx * a.stride + col0 + t], v[i][c][q]);
+          if ((HALF ? q < RL / 2 : idx < nd) && t < nc) sstore(&S[c * a.CS + idx * a.stride + col0 + t], v[i][c][q]);
         }
       }
     }
@@ -281,7 +297,7 @@ __device__ __forceinline__ void conv_body(const ConvArgs& a, int bx) {
       int t, j;
       SL::lj(i, t, j);
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
+      for (int c = 0; c < NC; c++) {
         dft<RL>(v[i][c], true);
 #pragma unroll
         for (int q = 0; q < RL; q++) sm[I0::out_idx(j, q) * NLP + c * TK + t] = v[i][c][q];
@@ -298,7 +314,7 @@ __device__ __forceinline__ void conv_body(const ConvArgs& a, int bx) {
       int t, j;
       SI::lj(i, t, j);
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
+      for (int c = 0; c < NC; c++) {
         float2 w[RI];
 #pragma unroll
         for (int q = 0; q < RI; q++) w[q] = sm[SI::in_idx(j, q) * NLP + c * TK + t];
@@ -307,7 +323,7 @@ __device__ __forceinline__ void conv_body(const ConvArgs& a, int bx) {
 #pragma unroll
         for (int q = 0; q < RI; q++) {
           int idx = SI::out_idx(j, q);
-          if ((HALF ? q < RI / 2 : idx < nd) && t < nc) sstore(&a.S[c * a.CS + idx * a.stride + col0 + t], w[q]);
+          if ((HALF ? q < RI / 2 : idx < nd) && t < nc) sstore(&S[c * a.CS + idx * a.stride + col0 + t], w[q]);
         }
       }
     }
@@ -329,6 +345,7 @@ __device__ __forceinline__ void zr2c_body(const float* __restrict__ src, float2*
   constexpr int PITCH = row_pitch(M);
   constexpr int NST = n_stages(M);
   constexpr bool QK = rows_qk<M>();
+  pass_begin();
   load_twiddles_rows<M, T>(tw, z.f.tw, z.f.tws);
   const int r0 = bx * RT;
   const int nl = min(RT, z.nrows - r0);
@@ -338,6 +355,7 @@ __device__ __forceinline__ void zr2c_body(const float* __restrict__ src, float2*
     roff_s[threadIdx.x] = ro;
     soff_s[threadIdx.x] = so;
   }
+  pass_wait();
   __syncthreads();
   const float dt = COMB ? *cb.dt : 0.f;
   const int nreal = z.n_real;
@@ -445,35 +463,58 @@ __device__ __forceinline__ float2 c2r_pre(float2 Xk, float2 Xm, int k, int M, co
   return make_float2(A.x - C.y, A.y + C.x);
 }
 
+// C2R rows of one component (the drop-in plan): the row tile of the forward
+// pass, first stage from global memory with the split undone on the way in.
+// An index-major tile of whole merged lines, with both spectrum values of
+// every point read twice and all stages in shared memory, took 15.4 us where
+// this takes as long as the forward pass (128 x 128 x 16 grid: 5.3 us).
 template <int M, int RT, int T>
-__global__ void __launch_bounds__(T) k_zc2r_fx(const float2* __restrict__ src, float* __restrict__ dst, ZPass z) {
+__global__ void __launch_bounds__(T) k_zc2r_fx(const float2* __restrict__ src, float* __restrict__ dst, ZPass z,
+                                               int vec2) {
   __shared__ float2 tw[M];
+  __shared__ int64_t roff_s[RT], soff_s[RT];
   extern __shared__ float2 sm[];
-  constexpr int SIP = odd_pitch(RT);
-  load_twiddles<M, T>(tw, z.f.tw, z.f.tws);
+  constexpr int PITCH = row_pitch(M);
+  constexpr bool QK = rows_qk<M>();
+  pass_begin();
+  load_twiddles_rows<M, T>(tw, z.f.tw, z.f.tws);
   const int r0 = blockIdx.x * RT;
   const int nl = min(RT, z.nrows - r0);
-  for (int e = threadIdx.x; e < RT * M; e += T) {
-    int l = e / M, k = e - l * M;
-    float2 v = make_float2(0.f, 0.f);
-    if (l < nl) {
-      int64_t roff, soff;
-      zrow_offsets(z, r0 + l, &roff, &soff);
-      v = c2r_pre(src[soff + k], src[soff + M - k], k, M, z.twP);
+  if ((int)threadIdx.x < nl) zrow_offsets(z, r0 + threadIdx.x, &roff_s[threadIdx.x], &soff_s[threadIdx.x]);
+  pass_wait();
+  __syncthreads();
+  constexpr int R0 = inv_radix(M, 0);
+  using S0 = St<M, R0, 1, RT, T, false>;
+#pragma unroll
+  for (int i = 0; i < S0::NB; i++) {
+    if (!S0::valid(i)) continue;
+    int l, j;
+    S0::lj(i, l, j);
+    if (l >= nl) continue;
+    const float2* row = src + soff_s[l];
+    float2 v[R0];
+#pragma unroll
+    for (int q = 0; q < R0; q++) {
+      const int k = S0::in_idx(j, q);
+      v[q] = c2r_pre(row[k], row[M - k], k, M, z.twP);
     }
-    sm[k * SIP + l] = v;
+    dft<R0>(v, true);
+#pragma unroll
+    for (int q = 0; q < R0; q++) sm[l * PITCH + padi(S0::out_idx(j, q))] = v[q];
   }
   __syncthreads();
-  tile_fft_fixed<M, RT, T, true, SIP, 1, true>(sm, tw);
-  for (int e = threadIdx.x; e < nl * M; e += T) {
-    int l = e / M, n = e - l * M;
-    int i0 = 2 * n;
-    if (i0 >= z.n_real) continue;
-    int64_t roff, soff;
-    zrow_offsets(z, r0 + l, &roff, &soff);
-    float2 v = sm[n * SIP + l];
-    dst[roff + i0] = v.x;
-    if (i0 + 1 < z.n_real) dst[roff + i0 + 1] = v.y;
+  MidRows<M, 1, n_stages(M), RT, T, PITCH, true, QK>::run(sm, tw);
+  const int np = (z.n_real + 1) / 2;
+  for (int e = threadIdx.x; e < nl * np; e += T) {
+    const int l = e / np, n = e - l * np;
+    const float2 v = sm[l * PITCH + padi(n)];
+    float* o = dst + roff_s[l] + 2 * n;
+    if (vec2 && 2 * n + 1 < z.n_real) {
+      *reinterpret_cast<float2*>(o) = v;
+    } else {
+      o[0] = v.x;
+      if (2 * n + 1 < z.n_real) o[1] = v.y;
+    }
   }
 }
 
@@ -507,6 +548,7 @@ __device__ __forceinline__ void zinv_body(const ZinvArgs& za, int bx) {
   const int64_t CS = za.CS;
   const EpiArgs& ea = za.ea;
   constexpr bool QK = rows_qk<M>();
+  pass_begin();
   load_twiddles_rows<M, T>(tw, za.fz.tw, 2);
   const int r0 = bx * RT;
   const int nr = min(RT, nrows - r0);
@@ -516,6 +558,7 @@ __device__ __forceinline__ void zinv_body(const ZinvArgs& za, int bx) {
     int x = gr / N1, y = gr - x * N1;
     rbase_s[threadIdx.x] = ((int64_t)x * P1 + y) * HZ;
   }
+  pass_wait();
   __syncthreads();
   // first inverse stage straight from global memory: line l = 3 r + c,
   // butterfly j combines bins k = j + q M/R0 (each after the C2R split)
@@ -712,10 +755,22 @@ __host__ __device__ constexpr int conv_tkp(int L) {
 }
 // shared-memory tile of a convolution block of TK columns (none for
 // one-stage lines, whose butterflies stay in registers from load to store)
-__host__ __device__ constexpr size_t conv_smem_tk(int L, int TK) {
-  return n_stages(L) == 1 ? 0 : sizeof(float2) * (size_t)odd_pitch(3 * TK) * L;
+__host__ __device__ constexpr size_t conv_smem(int L, int TK, bool split) {
+  return n_stages(L) == 1 ? 0 : sizeof(float2) * (size_t)odd_pitch(conv_comps(split) * TK) * L;
 }
-__host__ __device__ constexpr size_t conv_smem(int L) { return conv_smem_tk(L, conv_tkp(L)); }
+// Films: a split block holds two thirds (one third) of the tile and of the
+// registers, and there are twice as many.  That is faster for blocks of up to
+// 256 threads (more of them resident: a field of a 1024 x 256 film with a
+// periodic 256-point line 44.9 -> 37.2 us) and for lines whose three
+// components leave no room for 4 columns (2048 x 1536 film, 3072-point lines:
+// a Heun step 1078 -> 861 us).  In between (1024 and 1536 points) a block has
+// 512 threads, two of them fit an SM only with spilled registers, and three
+// components in one block are faster (512 x 512 film, RK23 trial: 104 us
+// against 119 us split).
+__host__ __device__ constexpr bool conv_split(int L, int TK) { return TK < 4 || TK * conv_bf(L) <= 256; }
+__host__ __device__ constexpr int conv_threads(int L, int TK) {
+  return TK * conv_bf(L) < 64 ? 64 : TK * conv_bf(L) > 512 ? 512 : (TK * conv_bf(L) + 31) / 32 * 32;
+}
 __host__ __device__ constexpr int fx_threads(int elems) {
   return elems / 16 < 64 ? 64 : (elems / 16 > 512 ? 512 : ((elems / 16 + 31) / 32) * 32);
 }
@@ -729,12 +784,11 @@ cudaError_t fx_launch_col(const float2* src, float2* dst, const ColPass& cp, cud
   const bool half = 2 * (INV ? cp.n_out : cp.n_in) == L;
   if (half) {
     if (smem > 48 * 1024) cudaFuncSetAttribute(k_col_fx<L, TK, T, INV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_col_fx<L, TK, T, INV, true><<<grid, T, smem, st>>>(src, dst, cp);
+    return launch_pass(k_col_fx<L, TK, T, INV, true>, grid, T, smem, st, src, dst, cp);
   } else {
     if (smem > 48 * 1024) cudaFuncSetAttribute(k_col_fx<L, TK, T, INV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_col_fx<L, TK, T, INV, false><<<grid, T, smem, st>>>(src, dst, cp);
+    return launch_pass(k_col_fx<L, TK, T, INV, false>, grid, T, smem, st, src, dst, cp);
   }
-  return cudaGetLastError();
 }
 
 // rows per Z tile: 2048 elements for the forward pass (smaller blocks, more
@@ -752,16 +806,16 @@ cudaError_t fx_launch_zr2c(const float* src, float2* dst, const ZPass& z, const 
   if (smem > 48 * 1024) cudaFuncSetAttribute(k_zr2c_fx<M, RT, T, COMB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   // 8-byte loads when every row starts at an even float offset
   int vec2 = (z.ld_real % 2 == 0) && (z.comp_stride_real % 2 == 0) && (((uintptr_t)src & 7) == 0);
-  k_zr2c_fx<M, RT, T, COMB><<<div_up(z.nrows, RT), T, smem, st>>>(src, dst, z, cb, vec2);
-  return cudaGetLastError();
+  return launch_pass(k_zr2c_fx<M, RT, T, COMB>, div_up(z.nrows, RT), T, smem, st, src, dst, z, cb, vec2);
 }
 
 template <int M>
 cudaError_t fx_launch_zc2r(const float2* src, float* dst, const ZPass& z, cudaStream_t st) {
   constexpr int RT = fx_rows(M, 1);
   constexpr int T = fx_threads(RT * M);
-  size_t smem = sizeof(float2) * (size_t)odd_pitch(RT) * M;
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k_zc2r_fx<M, RT, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_zc2r_fx<M, RT, T><<<div_up(z.nrows, RT), T, smem, st>>>(src, dst, z);
-  return cudaGetLastError();
+  size_t smem = sizeof(float2) * (size_t)RT * row_pitch(M);
+  if (smem > 16 * 1024) cudaFuncSetAttribute(k_zc2r_fx<M, RT, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // 8-byte stores when every row starts at an even float offset
+  const int vec2 = z.ld_real % 2 == 0 && z.comp_stride_real % 2 == 0 && ((uintptr_t)dst & 7) == 0;
+  return launch_pass(k_zc2r_fx<M, RT, T>, div_up(z.nrows, RT), T, smem, st, src, dst, z, vec2);
 }

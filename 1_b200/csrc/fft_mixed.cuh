@@ -19,154 +19,11 @@
 // registers, so four such blocks fit an SM), 256 for rows.
 #pragma once
 #include "epilogue.cuh"
+#include "fft_dft.cuh"
 #include "fft_passes.cuh"
 #include "kernmul.cuh"
 
 namespace mix {
-
-// cos and sin of 2 pi k / n in float64 at compile time (Taylor series of an
-// argument reduced to the first octant)
-constexpr double pi = 3.14159265358979323846264338327950288;
-constexpr double cos_small(double x) {
-  double t = 1, s = 1;
-  for (int i = 1; i < 14; i++) {
-    t *= -x * x / ((2 * i - 1) * (2 * i));
-    s += t;
-  }
-  return s;
-}
-constexpr double sin_small(double x) {
-  double t = x, s = x;
-  for (int i = 1; i < 14; i++) {
-    t *= -x * x / ((2 * i) * (2 * i + 1));
-    s += t;
-  }
-  return s;
-}
-constexpr double cos_of(int k, int n);
-constexpr double sin_of(int k, int n) {
-  k %= n;
-  if (2 * k > n) return -sin_of(n - k, n);
-  if (4 * k > n) {  // sin(pi - x)
-    return 4 * k == n ? 1.0 : (8 * k < 3 * n ? cos_small(2 * pi * (4 * k - n) / (4.0 * n))
-                                             : sin_small(2 * pi * (n - 2 * k) / (2.0 * n)));
-  }
-  return 8 * k <= n ? sin_small(2 * pi * k / n) : cos_small(2 * pi * (n - 4 * k) / (4.0 * n));
-}
-constexpr double cos_of(int k, int n) { return sin_of((4 * (k % n) + n) % (4 * n), 4 * n); }
-
-// exp(-2 pi i k / n)
-template <int K, int N>
-struct W {
-  static constexpr float c = (float)cos_of(K, N);
-  static constexpr float s = (float)-sin_of(K, N);
-};
-template <int K, int N>
-__device__ __forceinline__ float2 times_w(float2 a) {
-  constexpr int k = K % N;
-  if constexpr (k == 0) return a;
-  else if constexpr (4 * k == N) return make_float2(a.y, -a.x);
-  else if constexpr (2 * k == N) return make_float2(-a.x, -a.y);
-  else if constexpr (4 * k == 3 * N) return make_float2(-a.y, a.x);
-  else {
-    constexpr float c = W<k, N>::c, s = W<k, N>::s;
-    return make_float2(fmaf(a.x, c, -a.y * s), fmaf(a.x, s, a.y * c));
-  }
-}
-
-__host__ __device__ constexpr int split_of(int r) { return r == 4 ? 2 : r == 8 ? 4 : r == 16 ? 4 : r == 6 ? 2 : r == 9 ? 3 : r == 10 ? 2 : r == 12 ? 4 : r == 14 ? 2 : r == 15 ? 3 : r == 20 ? 4 : r == 25 ? 5 : 1; }
-
-// forward DFT of R points in registers
-template <int R>
-struct Dft;
-
-template <int A, int B, int I>
-__device__ __forceinline__ void twiddle_row(float2 (&t)[A]) {
-  // t[k1] *= W_(AB)^(I k1)
-  if constexpr (A > 1) t[1] = times_w<I * 1, A * B>(t[1]);
-  if constexpr (A > 2) t[2] = times_w<I * 2, A * B>(t[2]);
-  if constexpr (A > 3) t[3] = times_w<I * 3, A * B>(t[3]);
-  if constexpr (A > 4) t[4] = times_w<I * 4, A * B>(t[4]);
-}
-template <int A, int B, int I>
-__device__ __forceinline__ void first_rows(float2 (&u)[B][A], const float2 (&v)[A * B]) {
-  if constexpr (I < B) {
-#pragma unroll
-    for (int n1 = 0; n1 < A; n1++) u[I][n1] = v[n1 * B + I];
-    Dft<A>::run(u[I]);
-    twiddle_row<A, B, I>(u[I]);
-    first_rows<A, B, I + 1>(u, v);
-  }
-}
-// composite R = A B: n = n1 B + n2, k = k1 + A k2
-template <int R>
-struct Dft {
-  __device__ __forceinline__ static void run(float2 (&v)[R]) {
-    constexpr int A = split_of(R), B = R / A;
-    float2 u[B][A];
-    first_rows<A, B, 0>(u, v);
-#pragma unroll
-    for (int k1 = 0; k1 < A; k1++) {
-      float2 w[B];
-#pragma unroll
-      for (int n2 = 0; n2 < B; n2++) w[n2] = u[n2][k1];
-      Dft<B>::run(w);
-#pragma unroll
-      for (int k2 = 0; k2 < B; k2++) v[k1 + A * k2] = w[k2];
-    }
-  }
-};
-template <>
-struct Dft<2> {
-  __device__ __forceinline__ static void run(float2 (&v)[2]) {
-    float2 a = v[0], b = v[1];
-    v[0] = cadd(a, b);
-    v[1] = csub(a, b);
-  }
-};
-template <>
-struct Dft<4> {
-  __device__ __forceinline__ static void run(float2 (&v)[4]) { Radix<4>::dft(v, false); }
-};
-// odd primes: pairs (j, R - j) share their products,
-// X_k = v0 + sum_j cos(2 pi jk/R) (v_j + v_-j) - i sum_j sin(2 pi jk/R) (v_j - v_-j)
-template <int R>
-struct DftOdd {
-  template <int J, int K>
-  __device__ __forceinline__ static void term(const float2 (&s)[R / 2 + 1], const float2 (&d)[R / 2 + 1], float2& a,
-                                              float2& b) {
-    if constexpr (J <= R / 2) {
-      constexpr float c = W<(J * K) % R, R>::c, n = -W<(J * K) % R, R>::s;
-      a = make_float2(fmaf(c, s[J].x, a.x), fmaf(c, s[J].y, a.y));
-      b = make_float2(fmaf(n, d[J].x, b.x), fmaf(n, d[J].y, b.y));
-      term<J + 1, K>(s, d, a, b);
-    }
-  }
-  template <int K>
-  __device__ __forceinline__ static void out(float2 (&v)[R], float2 v0, const float2 (&s)[R / 2 + 1],
-                                             const float2 (&d)[R / 2 + 1]) {
-    if constexpr (K <= R / 2) {
-      float2 a = v0, b = make_float2(0.f, 0.f);
-      term<1, K>(s, d, a, b);
-      v[K] = make_float2(a.x + b.y, a.y - b.x);
-      v[R - K] = make_float2(a.x - b.y, a.y + b.x);
-      out<K + 1>(v, v0, s, d);
-    }
-  }
-  __device__ __forceinline__ static void run(float2 (&v)[R]) {
-    float2 s[R / 2 + 1], d[R / 2 + 1], v0 = v[0];
-#pragma unroll
-    for (int j = 1; j <= R / 2; j++) {
-      s[j] = cadd(v[j], v[R - j]);
-      d[j] = csub(v[j], v[R - j]);
-      v[0] = cadd(v[0], s[j]);
-    }
-    out<1>(v, v0, s, d);
-  }
-};
-template <> struct Dft<3> : DftOdd<3> {};
-template <> struct Dft<5> : DftOdd<5> {};
-template <> struct Dft<7> : DftOdd<7> {};
 
 // the radices a plan may hold; the last one of a convolution plan (whose three components share a
 // thread's registers) is at most 10
@@ -237,6 +94,7 @@ constexpr int T_COL = 128;
 template <int = 0>  // instantiated where it is launched
 __global__ void __launch_bounds__(T_COL, 4) k_col_mix(const float2* src, float2* dst, ColPass cp, int lg) {
   extern __shared__ float2 sm[];
+  pass_begin();
   const int TK = 1 << lg, TKP = odd_up(TK), L = cp.f.L, nst = cp.f.nst;
   const int l = threadIdx.x & (TK - 1), j0 = threadIdx.x >> lg, dj = T_COL >> lg;
   const int g = blockIdx.x * TK + l, pl = g / cp.ncols;
@@ -248,6 +106,7 @@ __global__ void __launch_bounds__(T_COL, 4) k_col_mix(const float2* src, float2*
     if (ok && i < n_out) dst[base + i * sti] = swapped(v, inv);
   };
   float2 *x = sm + l, *y = sm + L * TKP + l;
+  pass_wait();
   int ns = 1;
   for (int st = 0; st < nst; st++) {
     const int r = radix_at(cp.f.code, st);
@@ -290,6 +149,7 @@ struct Conv {
 template <bool D2>
 __global__ void __launch_bounds__(T_COL, 3) k_conv_mix(Conv a, int lg) {
   extern __shared__ float2 sm[];
+  pass_begin();
   const int TK = 1 << lg, NLP = odd_up(3 * TK), L = a.f.L, nst = a.f.conv_nst;
   const int t = threadIdx.x & (TK - 1), j0 = threadIdx.x >> lg, dj = T_COL >> lg;
   const int col = blockIdx.x * TK + t;
@@ -305,6 +165,7 @@ __global__ void __launch_bounds__(T_COL, 3) k_conv_mix(Conv a, int lg) {
   const float2* tw = a.f.tw;
   const int tws = a.f.tws;
   int ns = 1;
+  pass_wait();
   // forward stages but the last; a thread's butterflies of all components
   for (int st = 0; st < nst - 1; st++) {
     const int r = radix_at(a.f.conv_code, st);
@@ -481,6 +342,8 @@ __global__ void __launch_bounds__(T_ROW) k_zr2c_mix(const float* __restrict__ sr
   const int M = z.f.L, pitch = row_tile_pitch(M), nreal = z.n_real;
   const int r0 = blockIdx.x * RT, nl = min(RT, z.nrows - r0);
   if ((int)threadIdx.x < nl) zrow_offsets(z, r0 + threadIdx.x, &roff_s[threadIdx.x], &soff_s[threadIdx.x]);
+  pass_begin();
+  pass_wait();
   __syncthreads();
   // the rows' (x_2n, x_2n+1) pairs, four in flight a thread
   const int np = (nreal + 1) / 2;
@@ -590,6 +453,8 @@ __global__ void __launch_bounds__(T_ROW) k_zc2r_mix(const float2* __restrict__ s
   const int M = z.f.L, pitch = row_tile_pitch(M);
   const int r0 = blockIdx.x * RT, nl = min(RT, z.nrows - r0);
   if ((int)threadIdx.x < nl) zrow_offsets(z, r0 + threadIdx.x, &roff_s[threadIdx.x], &soff_s[threadIdx.x]);
+  pass_begin();
+  pass_wait();
   __syncthreads();
   load_merged(sm, nl, M, pitch, z.twP, [&](int l) { return src + soff_s[l]; });
   __syncthreads();
@@ -614,6 +479,8 @@ __global__ void __launch_bounds__(T_ROW, 2) k_zinv_mix(float2* S, LineFFT fz, co
     const int gr = r0 + threadIdx.x, xp = gr / N1, yr = gr - xp * N1;
     rbase_s[threadIdx.x] = ((int64_t)xp * P1 + yr) * HZ;
   }
+  pass_begin();
+  pass_wait();
   __syncthreads();
   float2 *A = sm, *B = sm + 3 * RT * pitch;
   auto spec_row = [&](int l) {
@@ -685,22 +552,24 @@ static cudaError_t allow(K kern, size_t bytes) {
   return bytes > 40 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
                            : cudaSuccess;
 }
-// widest tile (2^lg columns, at most 16 and no more than there are) whose
-// shared memory stays below a third of an SM's, but 4 columns (a 32-byte
+// widest tile (2^lg columns, at most 16 and no more than there are, fewer
+// where an SM would have no tile) whose shared memory stays below a third of an SM's, but 4 columns (a 32-byte
 // sector of every row) where they fit at all
 static inline int pick_columns(int L, int comps, int tiles, int64_t ncols, size_t* bytes) {
   int lg = 4;
   auto need = [&](int g) { return sizeof(float2) * (size_t)tiles * L * odd_up(comps << g); };
   while (lg > 0 && (1ll << (lg - 1)) >= ncols) lg--;
+  while (lg > 2 && (ncols >> lg) < mmx_sm_count()) lg--;
   while (lg > 2 && need(lg) > 72 * 1024) lg--;
   while (lg > 0 && need(lg) > 200 * 1024) lg--;
   *bytes = need(lg);
   return lg;
 }
-// rows of a Z tile: about 1024 elements a component, and shared memory below half an SM's
+// rows of a Z tile: about 1024 elements a component, fewer where an SM would
+// have no tile, and shared memory below half an SM's
 static inline int pick_rows(int M, int lines_per_row, int nrows, size_t* bytes) {
   int rt = 1024 / M < 1 ? 1 : 1024 / M > MAX_ROWS ? MAX_ROWS : 1024 / M;
-  if (rt > nrows) rt = nrows;
+  if (rt > div_up(nrows, mmx_sm_count())) rt = div_up(nrows, mmx_sm_count());
   auto need = [&](int r) { return sizeof(float2) * 2 * (size_t)r * lines_per_row * row_tile_pitch(M); };
   while (rt > 1 && need(rt) > 100 * 1024) rt--;
   *bytes = need(rt);
@@ -713,8 +582,7 @@ cudaError_t launch_col_mix(const float2* src, float2* dst, const ColPass& cp, cu
   const int lg = pick_columns(cp.f.L, 1, cp.f.nst > 2 ? 2 : 1, (int64_t)cp.ncols * cp.nplanes, &bytes);
   cudaError_t e = allow(k_col_mix<>, bytes);
   if (e != cudaSuccess) return e;
-  k_col_mix<><<<div_up((int64_t)cp.ncols * cp.nplanes, 1 << lg), T_COL, bytes, st>>>(src, dst, cp, lg);
-  return cudaGetLastError();
+  return launch_pass(k_col_mix<>, div_up((int64_t)cp.ncols * cp.nplanes, 1 << lg), T_COL, bytes, st, src, dst, cp, lg);
 }
 template <bool COMB>
 static cudaError_t launch_zr2c_mix(const float* src, float2* dst, const ZPass& z, const ZComb& cb, cudaStream_t st) {
@@ -724,8 +592,7 @@ static cudaError_t launch_zr2c_mix(const float* src, float2* dst, const ZPass& z
   if (e != cudaSuccess) return e;
   // 8-byte accesses when every row starts at an even float offset
   const int vec2 = z.ld_real % 2 == 0 && z.comp_stride_real % 2 == 0 && ((uintptr_t)src & 7) == 0;
-  k_zr2c_mix<COMB><<<div_up(z.nrows, rt), T_ROW, bytes, st>>>(src, dst, z, cb, vec2, rt);
-  return cudaGetLastError();
+  return launch_pass(k_zr2c_mix<COMB>, div_up(z.nrows, rt), T_ROW, bytes, st, src, dst, z, cb, vec2, rt);
 }
 template <int = 0>
 cudaError_t launch_zc2r_mix(const float2* src, float* dst, const ZPass& z, cudaStream_t st) {
@@ -733,8 +600,7 @@ cudaError_t launch_zc2r_mix(const float2* src, float* dst, const ZPass& z, cudaS
   const int rt = pick_rows(z.f.L, 1, z.nrows, &bytes);
   cudaError_t e = allow(k_zc2r_mix<>, bytes);
   if (e != cudaSuccess) return e;
-  k_zc2r_mix<><<<div_up(z.nrows, rt), T_ROW, bytes, st>>>(src, dst, z, rt);
-  return cudaGetLastError();
+  return launch_pass(k_zc2r_mix<>, div_up(z.nrows, rt), T_ROW, bytes, st, src, dst, z, rt);
 }
 
 }  // namespace mix

@@ -3,49 +3,59 @@
 #include "fx_dispatch.cuh"
 #include "fft_mixed.cuh"
 
-template <int L, int TK, int T, bool D2, bool HALF>
-// at least 768 resident threads per SM (6 blocks of 128 for L = 64):
-// measured faster than the unconstrained 96-register build (5 blocks) and
-// than 7 or 8 blocks (register spills)
-__global__ void __launch_bounds__(T, (768 / T) > 0 ? (768 / T) : 1) k_conv_fx(ConvArgs a) {
-  conv_body<L, TK, T, D2, HALF, !D2>(a, blockIdx.x);
+// the blocks of one tile: a film's split tile is two blocks, components 1 and 2 and component 0
+template <int L, int TK, int T, bool D2, bool HALF, bool STREAM>
+__device__ __forceinline__ void conv_block(const ConvArgs& a, int bx) {
+  __shared__ float2 tw[L];
+  if constexpr (D2 && conv_split(L, TK)) {
+    if (bx & 1) conv_body<L, TK, T, true, 0, 1, HALF, STREAM>(a, bx >> 1, tw);
+    else conv_body<L, TK, T, true, 1, 2, HALF, STREAM>(a, bx >> 1, tw);
+  } else {
+    conv_body<L, TK, T, D2, 0, 3, HALF, STREAM>(a, bx, tw);
+  }
 }
 
+// at least 768 resident threads per SM (6 blocks of 128 for L = 64):
+// measured faster than the unconstrained 96-register build (5 blocks) and
+// than 7 or 8 blocks (register spills).  Split blocks of a film: 1024, as far
+// as the shared memory of a block allows.
+__host__ __device__ constexpr int conv_min_blocks(int L, int TK, int T, bool split) {
+  const int want = (split ? 1024 : 768) / T;
+  const int fit = (int)(220 * 1024 / (conv_smem(L, TK, split) + sizeof(float2) * L + 1024));
+  return want < 1 || (split && fit < 1) ? 1 : !split || want < fit ? want : fit;
+}
+template <int L, int TK, int T, bool D2, bool HALF>
+__global__ void __launch_bounds__(T, conv_min_blocks(L, TK, T, D2 && conv_split(L, TK))) k_conv_fx(ConvArgs a) {
+  conv_block<L, TK, T, D2, HALF, !D2>(a, blockIdx.x);
+}
 template <int L, int TK, int T, bool D2, bool HALF>
 __global__ void __launch_bounds__(T) kb_conv(const ConvArgs* __restrict__ a, const int* __restrict__ starts,
                                              int nseg) {
   int s = find_seg(starts, nseg, blockIdx.x);
-  conv_body<L, TK, T, D2, HALF>(a[s], blockIdx.x - starts[s]);
+  conv_block<L, TK, T, D2, HALF, false>(a[s], blockIdx.x - starts[s]);
+}
+
+template <int L, bool D2, bool HALF>
+static cudaError_t launch_conv(const ConvArgs& a, cudaStream_t st) {
+  constexpr int TK = conv_tkp(L), T = conv_threads(L, TK);
+  constexpr bool split = D2 && conv_split(L, TK);
+  constexpr size_t smem = conv_smem(L, TK, split);
+  if (smem > 24 * 1024) cudaFuncSetAttribute(k_conv_fx<L, TK, T, D2, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return launch_pass(k_conv_fx<L, TK, T, D2, HALF>, div_up(a.ncols, TK) * (split ? 2 : 1), T, smem, st, a);
 }
 template <int L, bool D2>
-cudaError_t fx_launch_conv(const ConvArgs& a, cudaStream_t st) {
-  constexpr int TKP = conv_tkp(L);
-  // one thread per (column, radix-8 butterfly): it owns the three components
-  constexpr int NBF = TKP * (L / fwd_radix(L, n_stages(L) - 1));
-  constexpr int T = NBF < 64 ? 64 : (NBF > 512 ? 512 : ((NBF + 31) / 32) * 32);
-  size_t smem = conv_smem(L);
-  if (2 * a.n_data == L) {
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(k_conv_fx<L, TKP, T, D2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_conv_fx<L, TKP, T, D2, true><<<div_up(a.ncols, TKP), T, smem, st>>>(a);
-  } else {
-    if (smem > 48 * 1024)
-      cudaFuncSetAttribute(k_conv_fx<L, TKP, T, D2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_conv_fx<L, TKP, T, D2, false><<<div_up(a.ncols, TKP), T, smem, st>>>(a);
-  }
-  return cudaGetLastError();
+static cudaError_t fx_launch_conv(const ConvArgs& a, cudaStream_t st) {
+  return 2 * a.n_data == L ? launch_conv<L, D2, true>(a, st) : launch_conv<L, D2, false>(a, st);
 }
 
 // batch: narrow tiles (conv_tkp_narrow)
 template <int L, bool D2, bool HALF>
 static cudaError_t run_conv(const BatchLaunch& l, cudaStream_t st) {
-  constexpr int TKP = conv_tkp_narrow(L);
-  constexpr int NBF = TKP * (L / fwd_radix(L, n_stages(L) - 1));
-  constexpr int T = NBF < 64 ? 64 : (NBF > 512 ? 512 : ((NBF + 31) / 32) * 32);
-  size_t smem = conv_smem_tk(L, TKP);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(kb_conv<L, TKP, T, D2, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  kb_conv<L, TKP, T, D2, HALF><<<l.blocks, T, smem, st>>>((const ConvArgs*)l.args, l.starts, l.nseg);
+  constexpr int TK = conv_tkp_narrow(L), T = conv_threads(L, TK);
+  constexpr bool split = D2 && conv_split(L, TK);
+  constexpr size_t smem = conv_smem(L, TK, split);
+  if (smem > 24 * 1024) cudaFuncSetAttribute(kb_conv<L, TK, T, D2, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  kb_conv<L, TK, T, D2, HALF><<<l.blocks, T, smem, st>>>((const ConvArgs*)l.args, l.starts, l.nseg);
   return cudaGetLastError();
 }
 
@@ -75,6 +85,5 @@ cudaError_t CAT_(mx_conv_, FX_D2)(const mix::Conv& a, cudaStream_t st) {
   const int lg = mix::pick_columns(a.f.L, 3, a.f.conv_nst > 1 ? 2 : 0, a.ncols, &bytes);
   cudaError_t e = mix::allow(mix::k_conv_mix<FX_D2 != 0>, bytes);
   if (e != cudaSuccess) return e;
-  mix::k_conv_mix<FX_D2 != 0><<<div_up(a.ncols, 1 << lg), mix::T_COL, bytes, st>>>(a, lg);
-  return cudaGetLastError();
+  return launch_pass(mix::k_conv_mix<FX_D2 != 0>, div_up(a.ncols, 1 << lg), mix::T_COL, bytes, st, a, lg);
 }

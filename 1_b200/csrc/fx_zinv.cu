@@ -29,8 +29,7 @@ static cudaError_t launch(const ZinvArgs& za, bool fuse, cudaStream_t st) {
   size_t smem = sizeof(float2) * (size_t)3 * RT * row_pitch(M);
   auto go = [&](auto kern) {
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    kern<<<div_up(za.nrows, RT), T, smem, st>>>(za);
-    return cudaGetLastError();
+    return launch_pass(kern, div_up(za.nrows, RT), T, smem, st, za);
   };
   if (!fuse) return go(k_zinv_fx<M, RT, T, FX_MODE>);
   if constexpr (IN_STEP) return go(k_zinv_fwd_fx<M, RT, T, FX_MODE>);
@@ -60,9 +59,8 @@ static cudaError_t launch_mix(const ZinvArgs& za, bool fuse, cudaStream_t st) {
   auto go = [&](auto kern) {
     cudaError_t e = mix::allow(kern, bytes);
     if (e != cudaSuccess) return e;
-    kern<<<div_up(za.nrows, rt), mix::T_ROW, bytes, st>>>(za.S, za.fz, za.twP, za.P1, za.HZ, za.CS, za.nrows, za.ea,
-                                                          rt);
-    return cudaGetLastError();
+    return launch_pass(kern, div_up(za.nrows, rt), mix::T_ROW, bytes, st, za.S, za.fz, za.twP, za.P1, za.HZ, za.CS,
+                       za.nrows, za.ea, rt);
   };
   if constexpr (IN_STEP) {
     if (fuse) return go(mix::k_zinv_mix<MODE, true>);

@@ -70,16 +70,14 @@ __device__ __forceinline__ void kmul6_fma(float2& mx, float2& my, float2& mz, fl
   my = hy;
   mz = hz;
 }
-__device__ __forceinline__ void kmul4_fma(float2& mx, float2& my, float2& mz, float Kxx, float Kyy, float Kzz,
-                                          float Kyz) {
-  float2 hx, hy, hz;
-  hx.x = mx.x * Kxx;
-  hx.y = mx.y * Kxx;
-  hy.x = fmaf(mz.x, Kyz, my.x * Kyy);
-  hy.y = fmaf(mz.y, Kyz, my.y * Kyy);
-  hz.x = fmaf(mz.x, Kzz, my.x * Kyz);
-  hz.y = fmaf(mz.y, Kzz, my.y * Kyz);
-  mx = hx;
+__device__ __forceinline__ void kmul2_fma(float2& my, float2& mz, float Kyy, float Kzz, float Kyz) {
+  const float2 hy = make_float2(fmaf(mz.x, Kyz, my.x * Kyy), fmaf(mz.y, Kyz, my.y * Kyy));
+  const float2 hz = make_float2(fmaf(mz.x, Kzz, my.x * Kyz), fmaf(mz.y, Kzz, my.y * Kyz));
   my = hy;
   mz = hz;
+}
+__device__ __forceinline__ void kmul4_fma(float2& mx, float2& my, float2& mz, float Kxx, float Kyy, float Kzz,
+                                          float Kyz) {
+  mx = make_float2(mx.x * Kxx, mx.y * Kxx);
+  kmul2_fma(my, mz, Kyy, Kzz, Kyz);
 }
