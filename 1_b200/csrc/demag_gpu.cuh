@@ -12,51 +12,57 @@
 #pragma once
 #include "mmx_common.cuh"
 
-__device__ __forceinline__ float fk_norm(const float v[3]) {
-  float s = __fmul_rn(v[0], v[0]);
-  s = __fadd_rn(s, __fmul_rn(v[1], v[1]));
-  s = __fadd_rn(s, __fmul_rn(v[2], v[2]));
-  return __fsqrt_rn(s);
-}
-
-__device__ void fk_face_integral(float B[3], const float R[3], const float cs[3], int s, int n) {
-  int u = s, v = (s + 1) % 3, w = (s + 2) % 3;
-  float charge = __fmul_rn(cs[v], cs[w]);
-  float pu1 = __fdiv_rn(cs[u], 2.f);
-  float pu2 = -pu1;
+// Field at R of the two charged faces, n x n point charges each, of a cell
+// magnetised along S; only the components d >= S that the symmetric kernel
+// keeps.  Bound by the square roots and divisions of its 2 n^2 charges a
+// point.  With the axis a template parameter the displacements stay in
+// registers (a run-time axis indexed local memory), differences and squares
+// that a row of charges shares are formed once, 1/r is one rounded
+// reciprocal, and sc = +-(charge / den).  Every value is rounded as in the Go
+// code: differences, products, the sum of squares in the order x, y, z,
+// then the quotients, products and sums.
+template <int S>
+__device__ __forceinline__ void fk_face_integral(float (&B)[3], const float R[3], const float cs[3], int n) {
+  constexpr int U = S, V = (S + 1) % 3, W = (S + 2) % 3;
+  const float charge = __fmul_rn(cs[V], cs[W]);
+  const float pu1 = __fdiv_rn(cs[U], 2.f);
   const float four_pi = 12.566370614359172f;
-  float tv0 = __fadd_rn(-__fdiv_rn(cs[v], 2.f), __fdiv_rn(cs[v], (float)(2 * n)));
-  float tv1 = __fdiv_rn(cs[v], (float)n);
-  float tw0 = __fadd_rn(-__fdiv_rn(cs[w], 2.f), __fdiv_rn(cs[w], (float)(2 * n)));
-  float tw1 = __fdiv_rn(cs[w], (float)n);
+  const float tv0 = __fadd_rn(-__fdiv_rn(cs[V], 2.f), __fdiv_rn(cs[V], (float)(2 * n)));
+  const float tv1 = __fdiv_rn(cs[V], (float)n);
+  const float tw0 = __fadd_rn(-__fdiv_rn(cs[W], 2.f), __fdiv_rn(cs[W], (float)(2 * n)));
+  const float tw1 = __fdiv_rn(cs[W], (float)n);
+  const float du[2] = {__fsub_rn(R[U], pu1), __fsub_rn(R[U], -pu1)};
+  const float qu[2] = {__fmul_rn(du[0], du[0]), __fmul_rn(du[1], du[1])};
   B[0] = B[1] = B[2] = 0.f;
   for (int i = 0; i < n; i++) {
-    float pv = __fadd_rn(tv0, __fmul_rn((float)i, tv1));
+    const float dv = __fsub_rn(R[V], __fadd_rn(tv0, __fmul_rn((float)i, tv1)));
+    const float qv = __fmul_rn(dv, dv);
+#pragma unroll 4
     for (int j = 0; j < n; j++) {
-      float pw = __fadd_rn(tw0, __fmul_rn((float)j, tw1));
+      const float dw = __fsub_rn(R[W], __fadd_rn(tw0, __fmul_rn((float)j, tw1)));
+      const float qw = __fmul_rn(dw, dw);
 #pragma unroll
       for (int side = 0; side < 2; side++) {
-        float pole[3];
-        pole[u] = side == 0 ? pu1 : pu2;
-        pole[v] = pv;
-        pole[w] = pw;
-        float R2[3];
+        // squares in the order of the axes 0, 1, 2
+        float q[3], R2[3];
+        q[U] = qu[side];
+        q[V] = qv;
+        q[W] = qw;
+        R2[U] = du[side];
+        R2[V] = dv;
+        R2[W] = dw;
+        const float r = __fsqrt_rn(__fadd_rn(__fadd_rn(q[0], q[1]), q[2]));
+        const float inv = __frcp_rn(r);
+        const float quot = __fdiv_rn(charge, __fmul_rn(__fmul_rn(four_pi, r), r));
+        const float sc = side == 0 ? quot : -quot;
 #pragma unroll
-        for (int d = 0; d < 3; d++) R2[d] = __fsub_rn(R[d], pole[d]);
-        float r = fk_norm(R2);
-        float inv = __fdiv_rn(1.f, r);
-#pragma unroll
-        for (int d = 0; d < 3; d++) R2[d] = __fmul_rn(R2[d], inv);
-        float den = __fmul_rn(__fmul_rn(four_pi, r), r);
-        float sc = __fdiv_rn(side == 0 ? charge : -charge, den);
-#pragma unroll
-        for (int d = 0; d < 3; d++) B[d] = __fadd_rn(B[d], __fmul_rn(R2[d], sc));
+        for (int d = S; d < 3; d++) B[d] = __fadd_rn(B[d], __fmul_rn(__fmul_rn(R2[d], inv), sc));
       }
     }
   }
-  float fin = __fdiv_rn(1.f, (float)(n * n));
+  const float fin = __fdiv_rn(1.f, (float)(n * n));
 #pragma unroll
-  for (int d = 0; d < 3; d++) B[d] = __fmul_rn(B[d], fin);
+  for (int d = S; d < 3; d++) B[d] = __fmul_rn(B[d], fin);
 }
 
 struct FaceKernelArgs {
@@ -87,26 +93,35 @@ __global__ void k_face_kernel6(float* __restrict__ k6, FaceKernelArgs a) {
     int z0 = zw;
     while (z0 - a.P[2] >= a.lo[2]) z0 -= a.P[2];
     while (z0 < a.lo[2]) z0 += a.P[2];
-    for (int s = 0; s < 3; s++) {
+    // one component of magnetisation after the other, each over all images
+    auto images = [&](auto add) {
       for (int x = x0; x <= a.hi[0]; x += a.P[0])
         for (int y = y0; y <= a.hi[1]; y += a.P[1])
           for (int z = z0; z <= a.hi[2]; z += a.P[2]) {
-            float R[3] = {__fmul_rn((float)x, a.cs[0]), __fmul_rn((float)y, a.cs[1]), __fmul_rn((float)z, a.cs[2])};
-            float B[3];
-            fk_face_integral(B, R, a.cs, s, a.accuracy);
-            // KernIdx (kernel.go:95-98): order XX,YY,ZZ,YZ,XZ,XY
-            if (s == 0) {
-              acc[0] = __fadd_rn(acc[0], B[0]);
-              acc[5] = __fadd_rn(acc[5], B[1]);
-              acc[4] = __fadd_rn(acc[4], B[2]);
-            } else if (s == 1) {
-              acc[1] = __fadd_rn(acc[1], B[1]);
-              acc[3] = __fadd_rn(acc[3], B[2]);
-            } else {
-              acc[2] = __fadd_rn(acc[2], B[2]);
-            }
+            const float R[3] = {__fmul_rn((float)x, a.cs[0]), __fmul_rn((float)y, a.cs[1]),
+                                __fmul_rn((float)z, a.cs[2])};
+            add(R);
           }
-    }
+    };
+    // KernIdx (kernel.go:95-98): order XX,YY,ZZ,YZ,XZ,XY
+    images([&](const float* R) {
+      float B[3];
+      fk_face_integral<0>(B, R, a.cs, a.accuracy);
+      acc[0] = __fadd_rn(acc[0], B[0]);
+      acc[5] = __fadd_rn(acc[5], B[1]);
+      acc[4] = __fadd_rn(acc[4], B[2]);
+    });
+    images([&](const float* R) {
+      float B[3];
+      fk_face_integral<1>(B, R, a.cs, a.accuracy);
+      acc[1] = __fadd_rn(acc[1], B[1]);
+      acc[3] = __fadd_rn(acc[3], B[2]);
+    });
+    images([&](const float* R) {
+      float B[3];
+      fk_face_integral<2>(B, R, a.cs, a.accuracy);
+      acc[2] = __fadd_rn(acc[2], B[2]);
+    });
 #pragma unroll
     for (int c = 0; c < 6; c++) k6[c * n3 + idx] = acc[c];
   }
