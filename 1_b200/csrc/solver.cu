@@ -751,15 +751,8 @@ static void solver_free(mmx_solver* s) {
   for (int g = 0; g < 2; g++)
     if (s->dgraph[g]) cudaGraphExecDestroy(s->dgraph[g]);
   cudaFree(s->rkdev);
-  cudaFree(s->S);
-  cudaFree(s->kh);
+  cudaFree(s->block);
   cudaFree(s->kt_tc);
-  cudaFree(s->m);
-  cudaFree(s->t0);
-  cudaFree(s->m1);
-  cudaFree(s->mnew);
-  cudaFree(s->scratch);
-  for (int i = 0; i < RK_MAXS; i++) cudaFree(s->kb[i]);
   for (auto& t : s->timers)
     for (auto& pr : t.pending) { cudaEventDestroy(pr.first); cudaEventDestroy(pr.second); }
   delete s;
@@ -801,39 +794,51 @@ extern "C" int mmx_solver_create(const mmx_params* p, mmx_solver** out) {
   }
   s->dt = p->dt;
   size_t n3 = 3 * (size_t)s->n;
-#define ALLOC(ptr, bytes)                                                   \
-  if (cudaMalloc(&(ptr), (bytes)) != cudaSuccess) {                         \
-    solver_free(s);                                                         \
-    mmx_set_error("out of device memory");                                  \
-    return MMX_ERR_MEM;                                                     \
+  // the solver's arrays, in one allocation (an allocation and its release cost
+  // 10 us to 1 ms each, and a served solve pays for both)
+  const int O0 = s->P[0] / 2 + 1, O1 = s->P[1] / 2 + 1;
+  const int64_t ocs = (int64_t)O0 * O1 * s->HZ;
+  struct Part { void** p; size_t bytes; };
+  std::vector<Part> parts = {{(void**)&s->S, sizeof(float2) * 3 * (size_t)s->CS},
+                             {(void**)&s->m, sizeof(float) * n3},
+                             {(void**)&s->m1, sizeof(float) * n3},
+                             {(void**)&s->scratch, sizeof(float) * 16},
+                             {(void**)&s->kh, sizeof(float) * 6 * (size_t)ocs}};
+  if (p->solver == MMX_SOLVER_HEUN) {
+    parts.push_back({(void**)&s->t0, sizeof(float) * n3});
+  } else {
+    for (int i = 0; i < s->stages; i++) parts.push_back({(void**)&s->kb[i], sizeof(float) * n3});
+    if (s->adaptive) parts.push_back({(void**)&s->mnew, sizeof(float) * n3});
   }
-  ALLOC(s->S, sizeof(float2) * 3 * (size_t)s->CS);
-  ALLOC(s->m, sizeof(float) * n3);
-  ALLOC(s->m1, sizeof(float) * n3);
-  ALLOC(s->scratch, sizeof(float) * 16);
+  size_t total = 0;
+  for (const Part& q : parts) total += (q.bytes + 255) & ~(size_t)255;
+  if (cudaMalloc(&s->block, total) != cudaSuccess) {
+    cudaGetLastError();
+    solver_free(s);
+    mmx_set_error("out of device memory");
+    return MMX_ERR_MEM;
+  }
+  size_t off = 0;
+  for (const Part& q : parts) {
+    *q.p = s->block + off;
+    off += (q.bytes + 255) & ~(size_t)255;
+  }
   cudaMemset(s->m, 0, sizeof(float) * n3);
   cudaMemset(s->scratch, 0, sizeof(float) * 16);
-  if (p->solver == MMX_SOLVER_HEUN) {
-    ALLOC(s->t0, sizeof(float) * n3);
-  } else {
-    for (int i = 0; i < s->stages; i++) ALLOC(s->kb[i], sizeof(float) * n3);
-    ALLOC(s->mnew, sizeof(float) * n3);
-  }
   // kernel: real space on the GPU, transformed component by component
   {
     int64_t p3 = (int64_t)s->P[0] * s->P[1] * s->P[2];
-    float* k6 = nullptr;
-    float2* spec = nullptr;
-    int O0 = s->P[0] / 2 + 1, O1 = s->P[1] / 2 + 1;
-    int64_t ocs = (int64_t)O0 * O1 * s->HZ;
-    ALLOC(s->kh, sizeof(float) * 6 * ocs);
-    if (cudaMalloc(&k6, sizeof(float) * 6 * p3) != cudaSuccess ||
-        cudaMalloc(&spec, sizeof(float2) * (size_t)s->P[0] * s->P[1] * s->HZ) != cudaSuccess) {
-      cudaFree(k6);
+    // real-space kernel (6 components) and one component's spectrum
+    const size_t k6b = (sizeof(float) * 6 * p3 + 255) & ~(size_t)255;
+    char* tmp = nullptr;
+    if (cudaMalloc(&tmp, k6b + sizeof(float2) * (size_t)s->P[0] * s->P[1] * s->HZ) != cudaSuccess) {
+      cudaGetLastError();
       solver_free(s);
       mmx_set_error("out of device memory (kernel build)");
       return MMX_ERR_MEM;
     }
+    float* k6 = reinterpret_cast<float*>(tmp);
+    float2* spec = reinterpret_cast<float2*>(tmp + k6b);
     float cs[3] = {p->cellsize[0], p->cellsize[1], p->cellsize[2]};
     rc = mmx_face_kernel6(s->P, p->periodic, cs, s->p.accuracy, p->exch_type == 6, k6, 0);
     BoxPlan full;
@@ -849,8 +854,7 @@ extern "C" int mmx_solver_create(const mmx_params* p, mmx_solver** out) {
       k_extract_octant<<<solver_grid_1d(ocs), 256>>>(spec, s->kh + c * ocs, O0, O1, s->P[1], s->HZ, norm);
     }
     cudaError_t ce = cudaDeviceSynchronize();
-    cudaFree(k6);
-    cudaFree(spec);
+    cudaFree(tmp);
     if (rc != MMX_OK || ce != cudaSuccess) {
       solver_free(s);
       mmx_set_error(ce != cudaSuccess ? cudaGetErrorString(ce) : "kernel build failed");
@@ -864,7 +868,6 @@ extern "C" int mmx_solver_create(const mmx_params* p, mmx_solver** out) {
     s->K.P1 = s->P[1];
     s->K.cs = ocs;
   }
-#undef ALLOC
   if (s->p.precision) {
     rc = mmx_yconv2d_tc_prepare();
     if (rc == MMX_OK) rc = mmx_yconv2d_tc_kernel(s->K.kh, s->K.cs, s->HZ, &s->kt_tc);

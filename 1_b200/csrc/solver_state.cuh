@@ -47,6 +47,7 @@ struct mmx_solver {
   int64_t n;
   int is2d;
   BoxPlan bp;
+  char* block = nullptr;  // the allocation that S, kh, m, t0, m1, scratch, kb and mnew lie in
   float2* S = nullptr;
   int64_t CS = 0;
   float* kh = nullptr;
@@ -57,7 +58,7 @@ struct mmx_solver {
   float* m1 = nullptr;
   float* scratch = nullptr;  // device scalars: [0] err, [1] torque, [2] dt
   float* kb[RK_MAXS] = {nullptr};
-  float* mnew = nullptr;
+  float* mnew = nullptr;  // adaptive RK
   // solver scalars (host mirror)
   double time = 0;
   float dt = 0;
