@@ -79,12 +79,12 @@ __global__ void kb_clear(float** p, int n) {
 static cudaError_t run_launch(const Launch& l, cudaStream_t st) {
   BatchLaunch b;
   b.L = l.L;
-  b.nseg = l.nseg;
   b.blocks = l.blocks;
   b.half = l.half;
   b.variant = l.variant;
   b.flag = l.flag;
   b.args = l.args;
+  b.nseg = l.nseg;
   b.starts = l.starts;
   switch (l.kind) {
     case L_COL: return bx_col(b, st);
@@ -448,9 +448,10 @@ static int build_eval(mmx_batch* b, std::vector<Launch>& out, int mode, bool fir
       z.HZ = s->HZ;
       z.CS = s->CS;
       z.nrows = s->N[0] * s->N[1];
+      z.rt = zrows_per_tile(key.first, 3);
       z.ea = epi_for(i, fuse);
       a.push_back(z);
-      t.push_back(div_up(z.nrows, zrows_per_tile(key.first, 3)));
+      t.push_back(div_up(z.nrows, z.rt));
     }
     int r = add_launch(b, to, L_ZINV, key.first, mode, a, t);
     if (r != MMX_OK) return r;
@@ -587,7 +588,8 @@ static int batch_build(mmx_batch* b) {
   if (rc != MMX_OK) return rc;
   if ((rc = batch_upload(b)) != MMX_OK) return rc;
   for (auto& st : b->stage) b->launches_per_step += (int)st.size();
-  b->launches_per_step += (int)(b->z0.size() + b->last_z.size()) + (b->torque_ptrs ? 1 : 0);
+  // a step among others of one call (z0 runs once per call)
+  b->launches_per_step += (int)b->last_z_carry.size() + (b->torque_ptrs ? 1 : 0);
   return MMX_OK;
 }
 

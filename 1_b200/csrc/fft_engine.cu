@@ -51,15 +51,21 @@ bool fft_factor(int L, LineFFT* f) {
     while (m % p == 0) m /= p;
   if (m != 1) return false;
   f->L = L;
-  for (int conv = 0; conv < 2; conv++) {
+  auto search = [&](int most, int last, int* nst, unsigned long long* code) {
     int cur[8], best[8], n = -1;
-    plan_search(L, 25, conv ? 10 : 25, 0, cur, best, &n);
-    if (n < 0) return false;
-    unsigned long long code = 0;
-    for (int i = 0; i < n; i++) code |= (unsigned long long)best[i] << (8 * i);
-    (conv ? f->conv_nst : f->nst) = n;
-    (conv ? f->conv_code : f->code) = code;
-  }
+    plan_search(L, most, last, 0, cur, best, &n);
+    *code = 0;
+    for (int i = 0; i < n; i++) *code |= (unsigned long long)best[i] << (8 * i);
+    *nst = n;
+  };
+  int n_small;
+  unsigned long long small;
+  search(25, 25, &f->nst, &f->code);
+  search(25, 10, &f->conv_nst, &f->conv_code);
+  search(12, 5, &n_small, &small);
+  if (f->nst < 0 || f->conv_nst < 0) return false;
+  f->conv_small = n_small >= 0 && n_small <= f->conv_nst;
+  if (f->conv_small) f->conv_code = small;
   return true;
 }
 

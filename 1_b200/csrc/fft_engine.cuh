@@ -9,10 +9,11 @@
 
 // A line length is any product of 2, 3, 5 and 7.  The radix of stage s is
 // byte s of 'code'; the second plan, for the fused convolution, ends with a
-// radix of at most 10.
+// radix of at most 10 (5 where that takes no more stages).
 struct LineFFT {
   int L;                       // complex length of the line
   int nst, conv_nst;           // number of stages
+  int conv_small;              // the convolution plan's radices are at most 12, its last at most 5
   unsigned long long code, conv_code;
   const float2* tw;            // twiddle table, length L * tws
   int tws;                     // table stride (table built for a multiple of L)

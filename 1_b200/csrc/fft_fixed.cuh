@@ -198,8 +198,15 @@ __device__ __forceinline__ void load_twiddles_rows(float2* tw, const float2* __r
   }
 }
 
+// nl: the lines in use (NLINES where the tile is always full).  Butterflies of
+// the others are skipped where that costs a full tile nothing: a thread with
+// several butterflies loads them together, and a branch around each would keep
+// their loads apart (M = 512, two butterflies a thread: an RK23 trial 104 -> 110
+// us), so there only short lines, whose tiles hold many rows, skip.
+__host__ __device__ constexpr bool rows_skip(int L, int nb) { return nb == 1 || L <= 192; }
+
 template <int L, int R, int NS, int NLINES, int T, int PITCH, bool QK = false>
-__device__ __forceinline__ void stage_rows(float2* s, const float2* tw, bool inv) {
+__device__ __forceinline__ void stage_rows(float2* s, const float2* tw, bool inv, int nl) {
   using S = St<L, R, NS, NLINES, T, false>;
   float2 v[S::NB][R];
 #pragma unroll
@@ -207,6 +214,7 @@ __device__ __forceinline__ void stage_rows(float2* s, const float2* tw, bool inv
     if (!S::valid(i)) continue;
     int l, j;
     S::lj(i, l, j);
+    if (rows_skip(L, S::NB) && l >= nl) continue;
 #pragma unroll
     for (int q = 0; q < R; q++) v[i][q] = s[l * PITCH + padi(S::in_idx(j, q))];
     if constexpr (QK) S::twiddle_qk(v[i], j, tw, inv);
@@ -219,6 +227,7 @@ __device__ __forceinline__ void stage_rows(float2* s, const float2* tw, bool inv
     if (!S::valid(i)) continue;
     int l, j;
     S::lj(i, l, j);
+    if (rows_skip(L, S::NB) && l >= nl) continue;
 #pragma unroll
     for (int q = 0; q < R; q++) s[l * PITCH + padi(S::out_idx(j, q))] = v[i][q];
   }
@@ -228,7 +237,7 @@ __device__ __forceinline__ void stage_rows(float2* s, const float2* tw, bool inv
 // A row-tile stage whose outputs past L/2 are never read (the last inverse
 // stage of a zero-padded line): only the lower half is computed and stored.
 template <int L, int R, int NS, int NLINES, int T, int PITCH, bool QK = false>
-__device__ __forceinline__ void stage_rows_lower(float2* s, const float2* tw, bool inv) {
+__device__ __forceinline__ void stage_rows_lower(float2* s, const float2* tw, bool inv, int nl) {
   static_assert(NS * R == L, "the lower-half store is for the last stage");
   using S = St<L, R, NS, NLINES, T, false>;
   float2 v[S::NB][R];
@@ -237,6 +246,7 @@ __device__ __forceinline__ void stage_rows_lower(float2* s, const float2* tw, bo
     if (!S::valid(i)) continue;
     int l, j;
     S::lj(i, l, j);
+    if (rows_skip(L, S::NB) && l >= nl) continue;
 #pragma unroll
     for (int q = 0; q < R; q++) v[i][q] = s[l * PITCH + padi(S::in_idx(j, q))];
     if constexpr (QK) S::twiddle_qk(v[i], j, tw, inv);
@@ -249,6 +259,7 @@ __device__ __forceinline__ void stage_rows_lower(float2* s, const float2* tw, bo
     if (!S::valid(i)) continue;
     int l, j;
     S::lj(i, l, j);
+    if (rows_skip(L, S::NB) && l >= nl) continue;
 #pragma unroll
     for (int q = 0; q < R / 2; q++) s[l * PITCH + padi(S::out_idx(j, q))] = v[i][q];
   }
@@ -258,12 +269,12 @@ __device__ __forceinline__ void stage_rows_lower(float2* s, const float2* tw, bo
 // stages [ST, ST1) of a forward or inverse transform of a row tile
 template <int L, int ST, int ST1, int NLINES, int T, int PITCH, bool INV, bool QK = false>
 struct MidRows {
-  __device__ __forceinline__ static void run(float2* s, const float2* tw) {
+  __device__ __forceinline__ static void run(float2* s, const float2* tw, int nl) {
     if constexpr (ST < ST1) {
       constexpr int R = INV ? inv_radix(L, ST) : fwd_radix(L, ST);
       constexpr int NS = INV ? inv_span(L, ST) : fwd_span(L, ST);
-      stage_rows<L, R, NS, NLINES, T, PITCH, QK>(s, tw, INV);
-      MidRows<L, ST + 1, ST1, NLINES, T, PITCH, INV, QK>::run(s, tw);
+      stage_rows<L, R, NS, NLINES, T, PITCH, QK>(s, tw, INV, nl);
+      MidRows<L, ST + 1, ST1, NLINES, T, PITCH, INV, QK>::run(s, tw, nl);
     }
   }
 };

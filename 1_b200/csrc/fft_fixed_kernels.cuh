@@ -27,8 +27,8 @@ __device__ __forceinline__ void col_body(const float2* src, float2* dst, const C
   constexpr int NST = n_stages(L);
   constexpr int TKP = odd_pitch(TK);
   pass_begin();
-  load_twiddles<L, T>(tw, cp.f.tw, cp.f.tws);
   pass_wait();
+  load_twiddles<L, T>(tw, cp.f.tw, cp.f.tws);
   // Tiles run over the flattened columns of all planes: column g is column
   // g % ncols of plane g / ncols, so a tile may straddle two planes and no
   // tile at the end of a plane is left mostly empty.
@@ -149,6 +149,14 @@ using St3 = St<L, R, NS, TK, T, true>;  // (t, j) butterflies, components looped
 // conv_split for where they do).
 __host__ __device__ constexpr int conv_comps(bool split) { return split ? 2 : 3; }
 
+// A stage of m butterflies a line (the outer stages of a line whose first
+// radix is larger than its last, 1024 = 16 * 8 * 8) leaves part of the block
+// idle when a thread does all components of a butterfly; its components are
+// spread over the threads where that takes fewer rounds.
+__host__ __device__ constexpr bool conv_spread(int m, int comps, int TK, int T) {
+  return (comps * TK * m + T - 1) / T < comps * ((TK * m + T - 1) / T);
+}
+
 // HALF: the line holds data in its lower half only (n_data = L/2, the
 // open-boundary case): the first stage skips the zero half and the last
 // inverse stage computes only the stored half.
@@ -172,8 +180,8 @@ __device__ __forceinline__ void conv_body(const ConvArgs& a, int bx, float2* tw)
   constexpr int NLP = odd_pitch(NL);
   float2* const S = a.S + C0 * a.CS;
   pass_begin();
-  load_twiddles<L, T>(tw, a.tw, a.tws);
   pass_wait();
+  load_twiddles<L, T>(tw, a.tw, a.tws);
   const int col0 = bx * TK;
   const int nc = min(TK, a.ncols - col0);
   const int nd = a.n_data;
@@ -204,24 +212,46 @@ __device__ __forceinline__ void conv_body(const ConvArgs& a, int bx, float2* tw)
       }
     }
   } else {
-    float2 u[S0::NB][NC][R0];
+    if constexpr (conv_spread(L / R0, NC, TK, T)) {
+      using SP = St<L, R0, 1, NL, T, true>;
 #pragma unroll
-    for (int i = 0; i < S0::NB; i++) {
-      if (!S0::valid(i)) continue;
-      int t, j;
-      S0::lj(i, t, j);
-#pragma unroll
-      for (int c = 0; c < NC; c++) {
+      for (int i = 0; i < SP::NB; i++) {
+        if (!SP::valid(i)) continue;
+        int l, j;
+        SP::lj(i, l, j);
+        const int c = l / TK, t = l - c * TK;
+        float2 u[R0];
 #pragma unroll
         for (int q = 0; q < R0; q++) {
-          int idx = S0::in_idx(j, q);
-          u[i][c][q] = ((HALF ? q < R0 / 2 : idx < nd) && t < nc) ? sload(&S[c * a.CS + idx * a.stride + col0 + t])
-                                                                  : make_float2(0.f, 0.f);
+          const int idx = SP::in_idx(j, q);
+          u[q] = ((HALF ? q < R0 / 2 : idx < nd) && t < nc) ? sload(&S[c * a.CS + idx * a.stride + col0 + t])
+                                                            : make_float2(0.f, 0.f);
         }
-        if (HALF) dft_half<R0>(u[i][c], false);
-        else dft<R0>(u[i][c], false);
+        if (HALF) dft_half<R0>(u, false);
+        else dft<R0>(u, false);
 #pragma unroll
-        for (int q = 0; q < R0; q++) sm[S0::out_idx(j, q) * NLP + c * TK + t] = u[i][c][q];
+        for (int q = 0; q < R0; q++) sm[SP::out_idx(j, q) * NLP + l] = u[q];
+      }
+    } else {
+      float2 u[S0::NB][NC][R0];
+#pragma unroll
+      for (int i = 0; i < S0::NB; i++) {
+        if (!S0::valid(i)) continue;
+        int t, j;
+        S0::lj(i, t, j);
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+#pragma unroll
+          for (int q = 0; q < R0; q++) {
+            int idx = S0::in_idx(j, q);
+            u[i][c][q] = ((HALF ? q < R0 / 2 : idx < nd) && t < nc) ? sload(&S[c * a.CS + idx * a.stride + col0 + t])
+                                                                    : make_float2(0.f, 0.f);
+          }
+          if (HALF) dft_half<R0>(u[i][c], false);
+          else dft<R0>(u[i][c], false);
+#pragma unroll
+          for (int q = 0; q < R0; q++) sm[S0::out_idx(j, q) * NLP + c * TK + t] = u[i][c][q];
+        }
       }
     }
     __syncthreads();
@@ -307,25 +337,147 @@ __device__ __forceinline__ void conv_body(const ConvArgs& a, int bx, float2* tw)
     MidStages<L, 1, NST - 1, NL, T, true, NLP, 1, true>::run(sm, tw);
     constexpr int RI = inv_radix(L, NST - 1);
     constexpr int NSI = inv_span(L, NST - 1);
-    using SI = St3<L, RI, NSI, TK, T>;
+    if constexpr (conv_spread(L / RI, NC, TK, T)) {
+      using SP = St<L, RI, NSI, NL, T, true>;
 #pragma unroll
-    for (int i = 0; i < SI::NB; i++) {
-      if (!SI::valid(i)) continue;
-      int t, j;
-      SI::lj(i, t, j);
-#pragma unroll
-      for (int c = 0; c < NC; c++) {
+      for (int i = 0; i < SP::NB; i++) {
+        if (!SP::valid(i)) continue;
+        int l, j;
+        SP::lj(i, l, j);
+        const int c = l / TK, t = l - c * TK;
         float2 w[RI];
 #pragma unroll
-        for (int q = 0; q < RI; q++) w[q] = sm[SI::in_idx(j, q) * NLP + c * TK + t];
-        SI::twiddle(w, j, tw, true);
+        for (int q = 0; q < RI; q++) w[q] = sm[SP::in_idx(j, q) * NLP + l];
+        SP::twiddle(w, j, tw, true);
         dft<RI>(w, true);
 #pragma unroll
         for (int q = 0; q < RI; q++) {
-          int idx = SI::out_idx(j, q);
+          const int idx = SP::out_idx(j, q);
           if ((HALF ? q < RI / 2 : idx < nd) && t < nc) sstore(&S[c * a.CS + idx * a.stride + col0 + t], w[q]);
         }
       }
+    } else {
+      using SI = St3<L, RI, NSI, TK, T>;
+#pragma unroll
+      for (int i = 0; i < SI::NB; i++) {
+        if (!SI::valid(i)) continue;
+        int t, j;
+        SI::lj(i, t, j);
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+          float2 w[RI];
+#pragma unroll
+          for (int q = 0; q < RI; q++) w[q] = sm[SI::in_idx(j, q) * NLP + c * TK + t];
+          SI::twiddle(w, j, tw, true);
+          dft<RI>(w, true);
+#pragma unroll
+          for (int q = 0; q < RI; q++) {
+            int idx = SI::out_idx(j, q);
+            if ((HALF ? q < RI / 2 : idx < nd) && t < nc) sstore(&S[c * a.CS + idx * a.stride + col0 + t], w[q]);
+          }
+        }
+      }
+    }
+  }
+}
+
+// The same for grids that leave SMs free: one thread per component of a
+// (column, butterfly) instead of one for all three.  Such a pass lasts as long as one
+// thread's instructions, here a third of conv_body's; the kernel product
+// reads the other components' bins from the tile, one more pass through
+// shared memory.  The operations on a value are conv_body's, in its order.
+template <int L, int TK, int T, bool D2, bool HALF>
+__device__ __forceinline__ void conv_wide_body(const ConvArgs& a, int bx, float2* tw) {
+  extern __shared__ float2 sm[];
+  constexpr int NST = n_stages(L);
+  constexpr int NL = 3 * TK;
+  constexpr int NLP = odd_pitch(NL);
+  static_assert(NST > 1, "one-stage lines stay in registers");
+  pass_begin();
+  pass_wait();
+  load_twiddles<L, T>(tw, a.tw, a.tws);
+  const int col0 = bx * TK;
+  const int nd = a.n_data;
+  // line l = c TK + t; T is a multiple of NL, so a thread's butterflies are of one line
+  const int l = threadIdx.x % NL, c = l / TK, col = col0 + (l - c * TK);
+  const bool ok = col < a.ncols;
+  float2* const S = a.S + c * a.CS + col;
+  constexpr int R0 = fwd_radix(L, 0);
+  using S0 = St<L, R0, 1, NL, T, true>;
+#pragma unroll
+  for (int i = 0; i < S0::NB; i++) {
+    if (!S0::valid(i)) continue;
+    int ll, j;
+    S0::lj(i, ll, j);
+    float2 v[R0];
+#pragma unroll
+    for (int q = 0; q < R0; q++) {
+      const int idx = S0::in_idx(j, q);
+      v[q] = (HALF ? q < R0 / 2 : idx < nd) && col < a.ncols ? S[idx * a.stride] : make_float2(0.f, 0.f);
+    }
+    if (HALF) dft_half<R0>(v, false);
+    else dft<R0>(v, false);
+#pragma unroll
+    for (int q = 0; q < R0; q++) sm[S0::out_idx(j, q) * NLP + ll] = v[q];
+  }
+  __syncthreads();
+  MidStages<L, 1, NST, NL, T, true, NLP, 1, false>::run(sm, tw);
+  // kernel product and first inverse stage
+  constexpr int RL = fwd_radix(L, NST - 1);
+  using SL = St<L, RL, 1, NL, T, true>;
+  static_assert(SL::NB == 1, "one butterfly per thread");
+  const int j = threadIdx.x / NL;
+  float2 v[RL];
+  if (ok) {
+    int kyc = 0, kzc = col;
+    if (!D2) {
+      kyc = col / a.HZ;
+      kzc = col - kyc * a.HZ;
+    }
+#pragma unroll
+    for (int q = 0; q < RL; q++) {
+      const int k = SL::in_idx(j, q);
+      const float2* b = sm + k * NLP + (l - c * TK);
+      float Kxx, Kyy, Kzz, Kyz, Kxz, Kxy;
+      kern_at(a.K, D2 ? 0 : k, D2 ? k : kyc, kzc, Kxx, Kyy, Kzz, Kyz, Kxz, Kxy);
+      if (D2) {
+        const float2 x = b[0], y = b[TK], z = b[2 * TK];
+        float2 my = y, mz = z;
+        kmul2_fma(my, mz, Kyy, Kzz, Kyz);
+        v[q] = c == 0 ? make_float2(x.x * Kxx, x.y * Kxx) : c == 1 ? my : mz;
+      } else {
+        const float2 x = b[0], y = b[TK], z = b[2 * TK];
+        const float k0 = c == 0 ? Kxx : c == 1 ? Kxy : Kxz, k1 = c == 0 ? Kxy : c == 1 ? Kyy : Kyz,
+                    k2 = c == 0 ? Kxz : c == 1 ? Kyz : Kzz;
+        v[q] = make_float2(fmaf(z.x, k2, fmaf(y.x, k1, x.x * k0)), fmaf(z.y, k2, fmaf(y.y, k1, x.y * k0)));
+      }
+    }
+    dft<RL>(v, true);
+  }
+  __syncthreads();
+  if (ok) {
+#pragma unroll
+    for (int q = 0; q < RL; q++) sm[SL::out_idx(j, q) * NLP + l] = v[q];
+  }
+  __syncthreads();
+  MidStages<L, 1, NST - 1, NL, T, true, NLP, 1, true>::run(sm, tw);
+  constexpr int RI = inv_radix(L, NST - 1);
+  constexpr int NSI = inv_span(L, NST - 1);
+  using SI = St<L, RI, NSI, NL, T, true>;
+#pragma unroll
+  for (int i = 0; i < SI::NB; i++) {
+    if (!SI::valid(i)) continue;
+    int ll, jj;
+    SI::lj(i, ll, jj);
+    float2 w[RI];
+#pragma unroll
+    for (int q = 0; q < RI; q++) w[q] = sm[SI::in_idx(jj, q) * NLP + ll];
+    SI::twiddle(w, jj, tw, true);
+    dft<RI>(w, true);
+#pragma unroll
+    for (int q = 0; q < RI; q++) {
+      const int idx = SI::out_idx(jj, q);
+      if ((HALF ? q < RI / 2 : idx < nd) && col < a.ncols) S[idx * a.stride] = w[q];
     }
   }
 }
@@ -336,9 +488,10 @@ __device__ __forceinline__ void conv_body(const ConvArgs& a, int bx, float2* tw)
 // the lines (conflict-free).
 // ---------------------------------------------------------------------
 
-template <int M, int RT, int T, bool COMB>
+// FULL: blocks take RT rows (the batch), else rt of them.
+template <int M, int RT, int T, bool COMB, bool FULL>
 __device__ __forceinline__ void zr2c_body(const float* __restrict__ src, float2* __restrict__ dst, const ZPass& z,
-                                          const ZComb& cb, int vec2, int bx) {
+                                          const ZComb& cb, int vec2, int rt, int bx) {
   __shared__ float2 tw[M];
   __shared__ int64_t roff_s[RT], soff_s[RT];
   extern __shared__ float2 sm[];
@@ -346,16 +499,17 @@ __device__ __forceinline__ void zr2c_body(const float* __restrict__ src, float2*
   constexpr int NST = n_stages(M);
   constexpr bool QK = rows_qk<M>();
   pass_begin();
+  pass_wait();
   load_twiddles_rows<M, T>(tw, z.f.tw, z.f.tws);
-  const int r0 = bx * RT;
-  const int nl = min(RT, z.nrows - r0);
+  if (FULL) rt = RT;
+  const int r0 = bx * rt;
+  const int nl = min(rt, z.nrows - r0);
   if (threadIdx.x < RT) {
     int64_t ro = 0, so = 0;
     if ((int)threadIdx.x < nl) zrow_offsets(z, r0 + threadIdx.x, &ro, &so);
     roff_s[threadIdx.x] = ro;
     soff_s[threadIdx.x] = so;
   }
-  pass_wait();
   __syncthreads();
   const float dt = COMB ? *cb.dt : 0.f;
   const int nreal = z.n_real;
@@ -368,6 +522,7 @@ __device__ __forceinline__ void zr2c_body(const float* __restrict__ src, float2*
     if (!S0::valid(i)) continue;
     int l, j;
     S0::lj(i, l, j);
+    if (!FULL && rows_skip(M, S0::NB) && l >= nl) continue;
     float2 v[R0];
     const int64_t roff = l < nl ? roff_s[l] : 0;
     if (COMB && vec2 && l < nl) {
@@ -430,7 +585,7 @@ __device__ __forceinline__ void zr2c_body(const float* __restrict__ src, float2*
     for (int q = 0; q < R0; q++) sm[l * PITCH + padi(S0::out_idx(j, q))] = v[q];
   }
   __syncthreads();
-  MidRows<M, 1, NST, RT, T, PITCH, false, QK>::run(sm, tw);
+  MidRows<M, 1, NST, RT, T, PITCH, false, QK>::run(sm, tw, FULL ? RT : nl);
   // R2C split, one thread per pair (k, M - k), k <= M/2:
   // X_k = E_k + w^k O_k and X_{M-k} = conj(E_k - w^k O_k)
   constexpr int HP = M / 2 + 1;
@@ -449,8 +604,8 @@ __device__ __forceinline__ void zr2c_body(const float* __restrict__ src, float2*
 
 template <int M, int RT, int T, bool COMB>
 __global__ void __launch_bounds__(T) k_zr2c_fx(const float* __restrict__ src, float2* __restrict__ dst, ZPass z,
-                                               ZComb cb, int vec2) {
-  zr2c_body<M, RT, T, COMB>(src, dst, z, cb, vec2, blockIdx.x);
+                                               ZComb cb, int vec2, int rt) {
+  zr2c_body<M, RT, T, COMB, false>(src, dst, z, cb, vec2, rt, blockIdx.x);
 }
 
 // Z'_k = (X_k + conj X_{M-k}) + i (X_k - conj X_{M-k}) w^{-k}; X_0, X_M real
@@ -470,18 +625,18 @@ __device__ __forceinline__ float2 c2r_pre(float2 Xk, float2 Xm, int k, int M, co
 // this takes as long as the forward pass (128 x 128 x 16 grid: 5.3 us).
 template <int M, int RT, int T>
 __global__ void __launch_bounds__(T) k_zc2r_fx(const float2* __restrict__ src, float* __restrict__ dst, ZPass z,
-                                               int vec2) {
+                                               int vec2, int rt) {
   __shared__ float2 tw[M];
   __shared__ int64_t roff_s[RT], soff_s[RT];
   extern __shared__ float2 sm[];
   constexpr int PITCH = row_pitch(M);
   constexpr bool QK = rows_qk<M>();
   pass_begin();
-  load_twiddles_rows<M, T>(tw, z.f.tw, z.f.tws);
-  const int r0 = blockIdx.x * RT;
-  const int nl = min(RT, z.nrows - r0);
-  if ((int)threadIdx.x < nl) zrow_offsets(z, r0 + threadIdx.x, &roff_s[threadIdx.x], &soff_s[threadIdx.x]);
   pass_wait();
+  load_twiddles_rows<M, T>(tw, z.f.tw, z.f.tws);
+  const int r0 = blockIdx.x * rt;
+  const int nl = min(rt, z.nrows - r0);
+  if ((int)threadIdx.x < nl) zrow_offsets(z, r0 + threadIdx.x, &roff_s[threadIdx.x], &soff_s[threadIdx.x]);
   __syncthreads();
   constexpr int R0 = inv_radix(M, 0);
   using S0 = St<M, R0, 1, RT, T, false>;
@@ -503,7 +658,7 @@ __global__ void __launch_bounds__(T) k_zc2r_fx(const float2* __restrict__ src, f
     for (int q = 0; q < R0; q++) sm[l * PITCH + padi(S0::out_idx(j, q))] = v[q];
   }
   __syncthreads();
-  MidRows<M, 1, n_stages(M), RT, T, PITCH, true, QK>::run(sm, tw);
+  MidRows<M, 1, n_stages(M), RT, T, PITCH, true, QK>::run(sm, tw, nl);
   const int np = (z.n_real + 1) / 2;
   for (int e = threadIdx.x; e < nl * np; e += T) {
     const int l = e / np, n = e - l * np;
@@ -526,6 +681,7 @@ struct ZinvArgs {
   int P1, HZ;
   int64_t CS;
   int nrows;
+  int rt;  // rows per block, at most the tile's RT
   EpiArgs ea;
 };
 
@@ -534,7 +690,8 @@ struct ZinvArgs {
 // tile, so the block also runs the next forward Z transform on them and
 // writes the same spectrum rows it read -- the next evaluation needs no
 // separate forward Z pass and never re-reads m.
-template <int M, int RT, int T, int MODE, bool FUSE = false>
+// FULL: blocks take RT rows (the batch), else za.rt of them.
+template <int M, int RT, int T, int MODE, bool FUSE, bool FULL>
 __device__ __forceinline__ void zinv_body(const ZinvArgs& za, int bx) {
   __shared__ float2 tw[M];
   __shared__ int64_t rbase_s[RT];
@@ -549,16 +706,17 @@ __device__ __forceinline__ void zinv_body(const ZinvArgs& za, int bx) {
   const EpiArgs& ea = za.ea;
   constexpr bool QK = rows_qk<M>();
   pass_begin();
+  pass_wait();
   load_twiddles_rows<M, T>(tw, za.fz.tw, 2);
-  const int r0 = bx * RT;
-  const int nr = min(RT, nrows - r0);
+  const int rt = FULL ? RT : za.rt;
+  const int r0 = bx * rt;
+  const int nr = min(rt, nrows - r0), nl = FULL ? NL : 3 * nr;
   const int N1 = ea.N1, N2 = ea.N2;
   if (threadIdx.x < RT) {
     int gr = r0 + threadIdx.x;
     int x = gr / N1, y = gr - x * N1;
     rbase_s[threadIdx.x] = ((int64_t)x * P1 + y) * HZ;
   }
-  pass_wait();
   __syncthreads();
   // first inverse stage straight from global memory: line l = 3 r + c,
   // butterfly j combines bins k = j + q M/R0 (each after the C2R split)
@@ -569,6 +727,7 @@ __device__ __forceinline__ void zinv_body(const ZinvArgs& za, int bx) {
     if (!S0::valid(i)) continue;
     int l, j;
     S0::lj(i, l, j);
+    if (rows_skip(M, S0::NB) && l >= nl) continue;
     const int r = l / 3, c = l - 3 * r;
     float2 v[R0];
     const float2* row = S + c * CS + rbase_s[r < nr ? r : 0];
@@ -585,13 +744,13 @@ __device__ __forceinline__ void zinv_body(const ZinvArgs& za, int bx) {
   if constexpr (NST >= 2) {
     if (N2 == M) {
       // open boundary: the cells use the lower half of each line only
-      MidRows<M, 1, NST - 1, NL, T, PITCH, true, QK>::run(sm, tw);
-      stage_rows_lower<M, inv_radix(M, NST - 1), inv_span(M, NST - 1), NL, T, PITCH, QK>(sm, tw, true);
+      MidRows<M, 1, NST - 1, NL, T, PITCH, true, QK>::run(sm, tw, nl);
+      stage_rows_lower<M, inv_radix(M, NST - 1), inv_span(M, NST - 1), NL, T, PITCH, QK>(sm, tw, true, nl);
     } else {
-      MidRows<M, 1, NST, NL, T, PITCH, true, QK>::run(sm, tw);
+      MidRows<M, 1, NST, NL, T, PITCH, true, QK>::run(sm, tw, nl);
     }
   } else {
-    MidRows<M, 1, NST, NL, T, PITCH, true, QK>::run(sm, tw);
+    MidRows<M, 1, NST, NL, T, PITCH, true, QK>::run(sm, tw, nl);
   }
   float lmax = 0.f;
   double eacc = 0.0;
@@ -645,6 +804,7 @@ __device__ __forceinline__ void zinv_body(const ZinvArgs& za, int bx) {
         if (!SF::valid(i)) continue;
         int l, j;
         SF::lj(i, l, j);
+        if (rows_skip(M, SF::NB) && l >= nl) continue;
 #pragma unroll
         for (int q = 0; q < F0; q++)
           f[i][q] = (q < F0 / 2) ? sm[l * PITCH + padi(SF::in_idx(j, q))] : make_float2(0.f, 0.f);
@@ -655,12 +815,13 @@ __device__ __forceinline__ void zinv_body(const ZinvArgs& za, int bx) {
         if (!SF::valid(i)) continue;
         int l, j;
         SF::lj(i, l, j);
+        if (rows_skip(M, SF::NB) && l >= nl) continue;
         dft_half<F0>(f[i], false);
 #pragma unroll
         for (int q = 0; q < F0; q++) sm[l * PITCH + padi(SF::out_idx(j, q))] = f[i][q];
       }
       __syncthreads();
-      MidRows<M, 1, NST, NL, T, PITCH, false, QK>::run(sm, tw);
+      MidRows<M, 1, NST, NL, T, PITCH, false, QK>::run(sm, tw, nl);
       // R2C split, one thread per pair (k, M - k), k <= M/2:
       // X_k = E_k + w^k O_k and X_{M-k} = conj(E_k - w^k O_k)
       constexpr int HP = M / 2 + 1;
@@ -710,7 +871,7 @@ __device__ __forceinline__ void zinv_body(const ZinvArgs& za, int bx) {
   X(2) X(4) X(8) X(16) X(32) X(64) X(128) X(256) X(512) X(1024) X(2048) X(4096) X(6) X(12) X(24) X(48) \
       X(96) X(192) X(384) X(768) X(1536) X(3072)
 static inline bool fx_ok(int L) {
-  if (L < 2) return false;
+  if (L < 2 || L == 3) return false;
   int m = L % 3 == 0 ? L / 3 : L;
   return (m & (m - 1)) == 0 && L <= 4096;
 }
@@ -798,6 +959,16 @@ __host__ __device__ constexpr int fx_rows(int M, int lines_per_row) {
                             : ((4096 / (M * lines_per_row)) < 1 ? 1 : (4096 / (M * lines_per_row) > 32 ? 32 : 4096 / (M * lines_per_row)));
 }
 
+// Rows of a tile that a pass uses, at most the tile's rt: as many as give
+// every SM the same number of blocks, of the same size.  A grid of full tiles
+// that leaves SMs without a block, or some with one block more than others,
+// lasts as long as its fullest SM (64^3 grid: 196 blocks of 21 rows, two on
+// some SMs; 14 rows are two on all).
+static inline int rows_in_use(int rt, int nrows) {
+  const int sms = mmx_sm_count();
+  return div_up(nrows, (int64_t)sms * div_up(nrows, (int64_t)rt * sms));
+}
+
 template <int M, bool COMB>
 cudaError_t fx_launch_zr2c(const float* src, float2* dst, const ZPass& z, const ZComb& cb, cudaStream_t st) {
   constexpr int RT = fx_rows(M, 1);
@@ -806,7 +977,8 @@ cudaError_t fx_launch_zr2c(const float* src, float2* dst, const ZPass& z, const 
   if (smem > 48 * 1024) cudaFuncSetAttribute(k_zr2c_fx<M, RT, T, COMB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   // 8-byte loads when every row starts at an even float offset
   int vec2 = (z.ld_real % 2 == 0) && (z.comp_stride_real % 2 == 0) && (((uintptr_t)src & 7) == 0);
-  return launch_pass(k_zr2c_fx<M, RT, T, COMB>, div_up(z.nrows, RT), T, smem, st, src, dst, z, cb, vec2);
+  const int rt = rows_in_use(RT, z.nrows);
+  return launch_pass(k_zr2c_fx<M, RT, T, COMB>, div_up(z.nrows, rt), T, smem, st, src, dst, z, cb, vec2, rt);
 }
 
 template <int M>
@@ -817,5 +989,6 @@ cudaError_t fx_launch_zc2r(const float2* src, float* dst, const ZPass& z, cudaSt
   if (smem > 16 * 1024) cudaFuncSetAttribute(k_zc2r_fx<M, RT, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   // 8-byte stores when every row starts at an even float offset
   const int vec2 = z.ld_real % 2 == 0 && z.comp_stride_real % 2 == 0 && ((uintptr_t)dst & 7) == 0;
-  return launch_pass(k_zc2r_fx<M, RT, T>, div_up(z.nrows, RT), T, smem, st, src, dst, z, vec2);
+  const int rt = rows_in_use(RT, z.nrows);
+  return launch_pass(k_zc2r_fx<M, RT, T>, div_up(z.nrows, rt), T, smem, st, src, dst, z, vec2, rt);
 }

@@ -15,8 +15,7 @@
 // These kernels replace ones whose stages were limited to radix 8 (four
 // stages for 250 points), divided by run-time values several times per
 // element and passed through shared memory in place with two barriers a
-// stage.  Shapes: 128 threads for columns (25-point butterflies hold 50
-// registers, so four such blocks fit an SM), 256 for rows.
+// stage.  Blocks have 256 threads for rows, and for columns what pick_threads says.
 #pragma once
 #include "epilogue.cuh"
 #include "fft_dft.cuh"
@@ -38,6 +37,18 @@ namespace mix {
     MIX_CASE_(2, __VA_ARGS__) MIX_CASE_(3, __VA_ARGS__) MIX_CASE_(4, __VA_ARGS__) MIX_CASE_(5, __VA_ARGS__) \
     MIX_CASE_(6, __VA_ARGS__) MIX_CASE_(7, __VA_ARGS__) MIX_CASE_(8, __VA_ARGS__) MIX_CASE_(9, __VA_ARGS__) \
     MIX_CASE_(10, __VA_ARGS__)                                                                             \
+    default: break;                                                                                        \
+  }
+#define MIX_LE5(r, ...)                                                                                    \
+  switch (r) {                                                                                             \
+    MIX_CASE_(2, __VA_ARGS__) MIX_CASE_(3, __VA_ARGS__) MIX_CASE_(4, __VA_ARGS__) MIX_CASE_(5, __VA_ARGS__) \
+    default: break;                                                                                        \
+  }
+#define MIX_LE12(r, ...)                                                                                   \
+  switch (r) {                                                                                             \
+    MIX_CASE_(2, __VA_ARGS__) MIX_CASE_(3, __VA_ARGS__) MIX_CASE_(4, __VA_ARGS__) MIX_CASE_(5, __VA_ARGS__) \
+    MIX_CASE_(6, __VA_ARGS__) MIX_CASE_(7, __VA_ARGS__) MIX_CASE_(8, __VA_ARGS__) MIX_CASE_(9, __VA_ARGS__) \
+    MIX_CASE_(10, __VA_ARGS__) MIX_CASE_(12, __VA_ARGS__)                                                  \
     default: break;                                                                                        \
   }
 #define MIX_RADIX(r, ...)                                                                                  \
@@ -89,14 +100,14 @@ __host__ __device__ constexpr int odd_up(int n) { return n | 1; }
 // ---------------------------------------------------------------------
 // Columns: 2^lg adjacent columns, element i of column l at s[i * TKP + l].
 // ---------------------------------------------------------------------
-constexpr int T_COL = 128;
+constexpr int T_COL = 256;  // at most
 
 template <int = 0>  // instantiated where it is launched
-__global__ void __launch_bounds__(T_COL, 4) k_col_mix(const float2* src, float2* dst, ColPass cp, int lg) {
+__global__ void __launch_bounds__(T_COL, 2) k_col_mix(const float2* src, float2* dst, ColPass cp, int lg) {
   extern __shared__ float2 sm[];
   pass_begin();
   const int TK = 1 << lg, TKP = odd_up(TK), L = cp.f.L, nst = cp.f.nst;
-  const int l = threadIdx.x & (TK - 1), j0 = threadIdx.x >> lg, dj = T_COL >> lg;
+  const int l = threadIdx.x & (TK - 1), j0 = threadIdx.x >> lg, dj = blockDim.x >> lg;
   const int g = blockIdx.x * TK + l, pl = g / cp.ncols;
   const bool ok = g < cp.nplanes * cp.ncols, inv = cp.inv != 0;
   const int64_t base = (int64_t)pl * cp.plane_stride + (g - pl * cp.ncols), sti = cp.stride_i;
@@ -146,12 +157,26 @@ struct Conv {
   int64_t stride, CS;
 };
 
-template <bool D2>
-__global__ void __launch_bounds__(T_COL, 3) k_conv_mix(Conv a, int lg) {
+// SMALL: radices up to 12, the last up to 5 (f.conv_small), which takes 85 instead of
+// 168 registers (X lines of 20 points: 47 us with the large ones, 250 x 100 x 10 grid)
+#define MIX_ANY(r, ...)                    \
+  if constexpr (SMALL) {                   \
+    MIX_LE12(r, __VA_ARGS__)               \
+  } else {                                 \
+    MIX_RADIX(r, __VA_ARGS__)              \
+  }
+#define MIX_LAST(r, ...)                   \
+  if constexpr (SMALL) {                   \
+    MIX_LE5(r, __VA_ARGS__)                \
+  } else {                                 \
+    MIX_SMALL(r, __VA_ARGS__)              \
+  }
+template <bool D2, bool SMALL>
+__global__ void __launch_bounds__(SMALL ? 256 : 128, 3) k_conv_mix(Conv a, int lg) {
   extern __shared__ float2 sm[];
   pass_begin();
   const int TK = 1 << lg, NLP = odd_up(3 * TK), L = a.f.L, nst = a.f.conv_nst;
-  const int t = threadIdx.x & (TK - 1), j0 = threadIdx.x >> lg, dj = T_COL >> lg;
+  const int t = threadIdx.x & (TK - 1), j0 = threadIdx.x >> lg, dj = blockDim.x >> lg;
   const int col = blockIdx.x * TK + t;
   const bool ok = col < a.ncols;
   const int nd = a.n_data;
@@ -170,7 +195,7 @@ __global__ void __launch_bounds__(T_COL, 3) k_conv_mix(Conv a, int lg) {
   for (int st = 0; st < nst - 1; st++) {
     const int r = radix_at(a.f.conv_code, st);
     const Div dns(ns);
-    MIX_RADIX(r, {
+    MIX_ANY(r, {
       const int M = L / R;
       const Div dm(M);
       for (int b = j0; b < 3 * M; b += dj) {
@@ -197,7 +222,7 @@ __global__ void __launch_bounds__(T_COL, 3) k_conv_mix(Conv a, int lg) {
   // last forward stage, kernel product, first inverse stage
   const int rl = radix_at(a.f.conv_code, nst - 1);
   const Div dnl(ns);
-  MIX_SMALL(rl, {
+  MIX_LAST(rl, {
     const int M = L / R;
     for (int j = j0; j < M; j += dj) {
       float2 v[3][R];
@@ -251,7 +276,7 @@ MIX_UNROLL
     y = s;
     const int r = radix_at(a.f.conv_code, st);
     const Div dns(ns);
-    MIX_RADIX(r, {
+    MIX_ANY(r, {
       const int M = L / R;
       const Div dm(M);
       for (int b = j0; b < 3 * M; b += dj) {
@@ -565,6 +590,25 @@ static inline int pick_columns(int L, int comps, int tiles, int64_t ncols, size_
   *bytes = need(lg);
   return lg;
 }
+// threads of a block whose stage s has items[s] butterflies of radix[s]: the
+// multiple of 32 from 128 on that leaves the fewest idle slots over all
+// stages (smaller blocks waste fewer still, but the tiles then limit an SM to
+// few threads: 210 x 140 x 8 grid, 280-point columns, 242 us a Heun step pair
+// with 128 threads, 270 us with 64)
+static inline int pick_threads(int nst, const int* items, const int* radix, int most) {
+  int best = 128;
+  long best_cost = -1;
+  for (int t = 128; t <= most; t += 32) {
+    long cost = 0;
+    for (int s = 0; s < nst; s++) cost += (long)div_up(items[s], t) * t * radix[s];
+    // more threads at the same cost: fewer rounds
+    if (best_cost < 0 || cost <= best_cost) {
+      best_cost = cost;
+      best = t;
+    }
+  }
+  return best;
+}
 // rows of a Z tile: about 1024 elements a component, fewer where an SM would
 // have no tile, and shared memory below half an SM's
 static inline int pick_rows(int M, int lines_per_row, int nrows, size_t* bytes) {
@@ -582,7 +626,13 @@ cudaError_t launch_col_mix(const float2* src, float2* dst, const ColPass& cp, cu
   const int lg = pick_columns(cp.f.L, 1, cp.f.nst > 2 ? 2 : 1, (int64_t)cp.ncols * cp.nplanes, &bytes);
   cudaError_t e = allow(k_col_mix<>, bytes);
   if (e != cudaSuccess) return e;
-  return launch_pass(k_col_mix<>, div_up((int64_t)cp.ncols * cp.nplanes, 1 << lg), T_COL, bytes, st, src, dst, cp, lg);
+  int items[8], radix[8];
+  for (int s = 0; s < cp.f.nst; s++) {
+    radix[s] = (int)((cp.f.code >> (8 * s)) & 255);
+    items[s] = (cp.f.L / radix[s]) << lg;
+  }
+  const int t = pick_threads(cp.f.nst, items, radix, T_COL);
+  return launch_pass(k_col_mix<>, div_up((int64_t)cp.ncols * cp.nplanes, 1 << lg), t, bytes, st, src, dst, cp, lg);
 }
 template <bool COMB>
 static cudaError_t launch_zr2c_mix(const float* src, float2* dst, const ZPass& z, const ZComb& cb, cudaStream_t st) {

@@ -7,17 +7,20 @@ static void set_smem(K kern, size_t bytes) {
 }
 
 template <int L, int TK, int T, bool INV, bool HALF>
-__global__ void __launch_bounds__(T) kb_col(const BCol* __restrict__ a, const int* __restrict__ starts, int nseg) {
+__global__ void __launch_bounds__(T) kb_col(const BCol* __restrict__ a, const int* __restrict__ starts,
+                                             int nseg) {
   int s = find_seg(starts, nseg, blockIdx.x);
   int t = blockIdx.x - starts[s];
   const BCol& c = a[s];
   col_body<L, TK, T, INV, HALF>(c.src, c.dst, c.cp, t);
 }
 template <int M, int RT, int T, bool COMB>
-__global__ void __launch_bounds__(T) kb_zr2c(const BZr2c* __restrict__ a, const int* __restrict__ starts, int nseg) {
+__global__ void __launch_bounds__(T) kb_zr2c(const BZr2c* __restrict__ a, const int* __restrict__ starts,
+                                             int nseg) {
   int s = find_seg(starts, nseg, blockIdx.x);
+  int t = blockIdx.x - starts[s];
   const BZr2c& c = a[s];
-  zr2c_body<M, RT, T, COMB>(c.src, c.dst, c.z, c.cb, c.vec2, blockIdx.x - starts[s]);
+  zr2c_body<M, RT, T, COMB, true>(c.src, c.dst, c.z, c.cb, c.vec2, RT, t);
 }
 template <int L, int TK>
 static cudaError_t run_col_tk(const BatchLaunch& l, cudaStream_t st) {

@@ -32,11 +32,37 @@ template <int L, int TK, int T, bool D2, bool HALF>
 __global__ void __launch_bounds__(T) kb_conv(const ConvArgs* __restrict__ a, const int* __restrict__ starts,
                                              int nseg) {
   int s = find_seg(starts, nseg, blockIdx.x);
-  conv_block<L, TK, T, D2, HALF, false>(a[s], blockIdx.x - starts[s]);
+  int t = blockIdx.x - starts[s];
+  conv_block<L, TK, T, D2, HALF, false>(a[s], t);
+}
+
+// Wide blocks (a thread per component) take 4 columns, a 32-byte
+// sector of every row, and serve grids of at most one such block per SM, for the
+// lines whose block then has 48 to 768 threads.
+#define WIDE_TK 4
+__host__ __device__ constexpr bool wide_ok(int L) {
+  return n_stages(L) > 1 && 3 * WIDE_TK * conv_bf(L) >= 48 && 3 * WIDE_TK * conv_bf(L) <= 768;
+}
+// (A batch keeps its tiles: its launches run side by side and are bound by the
+// work of all of them.  Wide blocks and Z tiles of fewer rows for its launches
+// of few blocks made a step of 24 instances 393 -> 454 us.)
+template <int L, int TK, int T, bool D2, bool HALF>
+__global__ void __launch_bounds__(T) k_conv_wide(ConvArgs a) {
+  __shared__ float2 tw[L];
+  conv_wide_body<L, TK, T, D2, HALF>(a, blockIdx.x, tw);
 }
 
 template <int L, bool D2, bool HALF>
 static cudaError_t launch_conv(const ConvArgs& a, cudaStream_t st) {
+  if constexpr (wide_ok(L)) {
+    constexpr int TK = WIDE_TK, T = 3 * TK * conv_bf(L);
+    const int blocks = div_up(a.ncols, TK);
+    if (blocks <= mmx_sm_count()) {
+      constexpr size_t smem = conv_smem(L, TK, false);
+      if (smem > 24 * 1024) cudaFuncSetAttribute(k_conv_wide<L, TK, T, D2, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      return launch_pass(k_conv_wide<L, TK, T, D2, HALF>, blocks, T, smem, st, a);
+    }
+  }
   constexpr int TK = conv_tkp(L), T = conv_threads(L, TK);
   constexpr bool split = D2 && conv_split(L, TK);
   constexpr size_t smem = conv_smem(L, TK, split);
@@ -83,7 +109,22 @@ cudaError_t CAT_(mx_conv_, FX_D2)(const mix::Conv& a, cudaStream_t st) {
   if (3 * a.f.L > 8192) return cudaErrorInvalidValue;
   size_t bytes;
   const int lg = mix::pick_columns(a.f.L, 3, a.f.conv_nst > 1 ? 2 : 0, a.ncols, &bytes);
-  cudaError_t e = mix::allow(mix::k_conv_mix<FX_D2 != 0>, bytes);
+  // a stage's items are the butterflies of three components; the product's are of all three
+  int items[8], radix[8];
+  for (int s = 0; s < a.f.conv_nst; s++) {
+    const int r = (int)((a.f.conv_code >> (8 * s)) & 255), last = s == a.f.conv_nst - 1;
+    items[s] = ((last ? 1 : 3) * (a.f.L / r)) << lg;
+    radix[s] = (last ? 3 : 1) * r;
+  }
+  const int blocks = div_up(a.ncols, 1 << lg);
+  if (a.f.conv_small) {
+    cudaError_t e = mix::allow(mix::k_conv_mix<FX_D2 != 0, true>, bytes);
+    if (e != cudaSuccess) return e;
+    const int t = mix::pick_threads(a.f.conv_nst, items, radix, 256);
+    return launch_pass(mix::k_conv_mix<FX_D2 != 0, true>, blocks, t, bytes, st, a, lg);
+  }
+  cudaError_t e = mix::allow(mix::k_conv_mix<FX_D2 != 0, false>, bytes);
   if (e != cudaSuccess) return e;
-  return launch_pass(mix::k_conv_mix<FX_D2 != 0>, div_up(a.ncols, 1 << lg), mix::T_COL, bytes, st, a, lg);
+  const int t = mix::pick_threads(a.f.conv_nst, items, radix, 128);
+  return launch_pass(mix::k_conv_mix<FX_D2 != 0, false>, blocks, t, bytes, st, a, lg);
 }

@@ -5,31 +5,33 @@
 
 template <int M, int RT, int T, int MODE>
 __global__ void __launch_bounds__(T) k_zinv_fx(ZinvArgs za) {
-  zinv_body<M, RT, T, MODE>(za, blockIdx.x);
+  zinv_body<M, RT, T, MODE, false, false>(za, blockIdx.x);
 }
 template <int M, int RT, int T, int MODE>
 __global__ void __launch_bounds__(T) k_zinv_fwd_fx(ZinvArgs za) {
-  zinv_body<M, RT, T, MODE, true>(za, blockIdx.x);
+  zinv_body<M, RT, T, MODE, true, false>(za, blockIdx.x);
 }
 
 template <int M, int RT, int T, int MODE, bool FUSE>
 __global__ void __launch_bounds__(T) kb_zinv(const ZinvArgs* __restrict__ a, const int* __restrict__ starts,
                                              int nseg) {
   int s = find_seg(starts, nseg, blockIdx.x);
-  zinv_body<M, RT, T, MODE, FUSE>(a[s], blockIdx.x - starts[s]);
+  int t = blockIdx.x - starts[s];
+  zinv_body<M, RT, T, MODE, FUSE, true>(a[s], t);
 }
 
 // epilogues that a step can follow with the next forward Z, and that a batch runs
 static constexpr bool IN_STEP = FX_MODE >= EPI_HEUN1 && FX_MODE <= EPI_RK;
 
 template <int M>
-static cudaError_t launch(const ZinvArgs& za, bool fuse, cudaStream_t st) {
+static cudaError_t launch(ZinvArgs za, bool fuse, cudaStream_t st) {
   constexpr int RT = fx_rows(M, 3);
+  za.rt = rows_in_use(RT, za.nrows);
   constexpr int T = fx_threads(3 * RT * M);
   size_t smem = sizeof(float2) * (size_t)3 * RT * row_pitch(M);
   auto go = [&](auto kern) {
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return launch_pass(kern, div_up(za.nrows, RT), T, smem, st, za);
+    return launch_pass(kern, div_up(za.nrows, za.rt), T, smem, st, za);
   };
   if (!fuse) return go(k_zinv_fx<M, RT, T, FX_MODE>);
   if constexpr (IN_STEP) return go(k_zinv_fwd_fx<M, RT, T, FX_MODE>);
