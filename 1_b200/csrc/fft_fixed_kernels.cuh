@@ -1,7 +1,6 @@
-// Fixed-size pass kernels of the zero-aware padded FFT.
-// Drop-in replacements for k_col / k_z_r2c / k_z_c2r (fft_passes.cuh) and
-// for the fused k_xconv / k_yconv2d / k_zinv_epi (solver.cu) when the line
-// length has compiled kernels (FX_SIZES).
+// Pass kernels of the zero-aware padded FFT for the compiled line lengths
+// (FX_SIZES): column passes, the fused convolution, and the Z rows with the
+// solver epilogues.  Other lengths run the same passes from fft_mixed.cuh.
 #pragma once
 #include "epilogue.cuh"
 #include "kernmul.cuh"

@@ -25,38 +25,9 @@ __device__ __forceinline__ void kern_at(const KernOct& K, int kx, int ky, int kz
   if (nx != ny) Kxy = -Kxy;
 }
 
-// H = K M per bin in the order of gpu_kernelmul6 (gpu_kernmul.cu:51-58)
-__device__ __forceinline__ void kmul6(float2& mx, float2& my, float2& mz, float Kxx, float Kyy, float Kzz, float Kyz,
-                                      float Kxz, float Kxy) {
-  float2 hx, hy, hz;
-  hx.x = FA(FA(FM(mx.x, Kxx), FM(my.x, Kxy)), FM(mz.x, Kxz));
-  hx.y = FA(FA(FM(mx.y, Kxx), FM(my.y, Kxy)), FM(mz.y, Kxz));
-  hy.x = FA(FA(FM(mx.x, Kxy), FM(my.x, Kyy)), FM(mz.x, Kyz));
-  hy.y = FA(FA(FM(mx.y, Kxy), FM(my.y, Kyy)), FM(mz.y, Kyz));
-  hz.x = FA(FA(FM(mx.x, Kxz), FM(my.x, Kyz)), FM(mz.x, Kzz));
-  hz.y = FA(FA(FM(mx.y, Kxz), FM(my.y, Kyz)), FM(mz.y, Kzz));
-  mx = hx;
-  my = hy;
-  mz = hz;
-}
-// 2D: Kxy = Kxz = 0 (gpu_kernmul.cu:114-119)
-__device__ __forceinline__ void kmul4(float2& mx, float2& my, float2& mz, float Kxx, float Kyy, float Kzz,
-                                      float Kyz) {
-  float2 hx, hy, hz;
-  hx.x = FM(mx.x, Kxx);
-  hx.y = FM(mx.y, Kxx);
-  hy.x = FA(FM(my.x, Kyy), FM(mz.x, Kyz));
-  hy.y = FA(FM(my.y, Kyy), FM(mz.y, Kyz));
-  hz.x = FA(FM(my.x, Kyz), FM(mz.x, Kzz));
-  hz.y = FA(FM(my.y, Kyz), FM(mz.y, Kzz));
-  mx = hx;
-  my = hy;
-  mz = hz;
-}
-
-// The same products with fused multiply-adds, for the fused convolution
+// H = K M per bin with fused multiply-adds, for the fused convolution
 // passes (their results are compared with the FP64 oracle within a
-// tolerance; the drop-in gpu_kernelmul6/4 keep the rounding above).
+// tolerance; the drop-in gpu_kernelmul6/4 keep the rounding of gpu_kernmul.cu).
 __device__ __forceinline__ void kmul6_fma(float2& mx, float2& my, float2& mz, float Kxx, float Kyy, float Kzz,
                                           float Kyz, float Kxz, float Kxy) {
   float2 hx, hy, hz;

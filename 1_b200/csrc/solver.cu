@@ -16,7 +16,8 @@
 //  * Zi+epilogue: C2R of the three components of a row in shared memory,
 //          then the local fields, the LLG torque and the solver stage
 //          update per cell (Heun predictor/corrector, RK stage, or just
-//          the field).
+//          the field); with an open Z boundary a step's Zi goes on to the Zf
+//          of the next evaluation, which then is no pass of its own.
 // The kernel spectrum is real; it is stored as one octant (kx <= P0/2,
 // ky <= P1/2, all kz) and unfolded with the parity of each component
 // (diagonal components even, XY odd in kx,ky, XZ odd in kx, YZ odd in ky).
