@@ -192,14 +192,15 @@ static int col_tiles(int L, int ncols, int nplanes, int variant) {
   return div_up(ncols * nplanes, tk);
 }
 static int conv_blocks(int L, int ncols, bool d2) {
-  int tk = 1, per = 1;
+  int tk = 1;
+  bool split = false;
   switch (L) {
 #define C_(LL) \
-  case LL: tk = conv_tkp_narrow(LL); per = d2 && conv_split(LL, conv_tkp_narrow(LL)) ? 2 : 1; break;
+  case LL: tk = conv_tkp_narrow(LL); split = d2 && conv_split(LL, conv_tkp_narrow(LL)); break;
     FX_SIZES(C_)
 #undef C_
   }
-  return div_up(ncols, tk) * per;
+  return split ? 3 * div_up(ncols, 2 * tk) : div_up(ncols, tk);
 }
 static int zrows_per_tile(int M, int lines_per_row) {
   switch (M) {

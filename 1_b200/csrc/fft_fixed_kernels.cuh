@@ -918,15 +918,17 @@ __host__ __device__ constexpr int conv_tkp(int L) {
 __host__ __device__ constexpr size_t conv_smem(int L, int TK, bool split) {
   return n_stages(L) == 1 ? 0 : sizeof(float2) * (size_t)odd_pitch(conv_comps(split) * TK) * L;
 }
-// Films: a split block holds two thirds (one third) of the tile and of the
-// registers, and there are twice as many.  That is faster for blocks of up to
-// 256 threads (more of them resident: a field of a 1024 x 256 film with a
-// periodic 256-point line 44.9 -> 37.2 us) and for lines whose three
-// components leave no room for 4 columns (2048 x 1536 film, 3072-point lines:
-// a Heun step 1078 -> 861 us).  In between (1024 and 1536 points) a block has
-// 512 threads, two of them fit an SM only with spilled registers, and three
-// components in one block are faster (512 x 512 film, RK23 trial: 104 us
-// against 119 us split).
+// Films: a split block holds the lines of two components of TK columns, or of
+// one component of 2 TK (32-byte sectors of a long line's rows instead of 16
+// bytes of them: 2048 x 1536 film, 4 Heun steps 3446 -> 3228 us), two thirds
+// of the tile and registers of three, and there are half as many again.  That
+// is faster for blocks of up to 256 threads (more of them resident: a field of
+// a 1024 x 256 film with a periodic 256-point line 44.9 -> 36.8 us) and for
+// lines whose three components leave no room for 4 columns (3072-point lines:
+// 4 Heun steps of the film above 4131 -> 3228 us; one column per block: 4308
+// us).  In between (1024 and 1536 points) a block has 512 threads, two of them
+// fit an SM only with spilled registers, and three components in one block
+// are faster (512 x 512 film, RK23 trial: 104 us against 119 us split).
 __host__ __device__ constexpr bool conv_split(int L, int TK) { return TK < 4 || TK * conv_bf(L) <= 256; }
 __host__ __device__ constexpr int conv_threads(int L, int TK) {
   return TK * conv_bf(L) < 64 ? 64 : TK * conv_bf(L) > 512 ? 512 : (TK * conv_bf(L) + 31) / 32 * 32;

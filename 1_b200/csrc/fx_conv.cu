@@ -3,13 +3,15 @@
 #include "fx_dispatch.cuh"
 #include "fft_mixed.cuh"
 
-// the blocks of one tile: a film's split tile is two blocks, components 1 and 2 and component 0
+// A film's split blocks come in threes: components 1 and 2 of two tiles of TK
+// columns, and component 0 of both, the same number of lines in each.
 template <int L, int TK, int T, bool D2, bool HALF, bool STREAM>
 __device__ __forceinline__ void conv_block(const ConvArgs& a, int bx) {
   __shared__ float2 tw[L];
   if constexpr (D2 && conv_split(L, TK)) {
-    if (bx & 1) conv_body<L, TK, T, true, 0, 1, HALF, STREAM>(a, bx >> 1, tw);
-    else conv_body<L, TK, T, true, 1, 2, HALF, STREAM>(a, bx >> 1, tw);
+    const int g = bx / 3, r = bx - 3 * g;
+    if (r == 2) conv_body<L, 2 * TK, T, true, 0, 1, HALF, STREAM>(a, g, tw);
+    else conv_body<L, TK, T, true, 1, 2, HALF, STREAM>(a, 2 * g + r, tw);
   } else {
     conv_body<L, TK, T, D2, 0, 3, HALF, STREAM>(a, bx, tw);
   }
@@ -67,7 +69,7 @@ static cudaError_t launch_conv(const ConvArgs& a, cudaStream_t st) {
   constexpr bool split = D2 && conv_split(L, TK);
   constexpr size_t smem = conv_smem(L, TK, split);
   if (smem > 24 * 1024) cudaFuncSetAttribute(k_conv_fx<L, TK, T, D2, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  return launch_pass(k_conv_fx<L, TK, T, D2, HALF>, div_up(a.ncols, TK) * (split ? 2 : 1), T, smem, st, a);
+  return launch_pass(k_conv_fx<L, TK, T, D2, HALF>, split ? 3 * div_up(a.ncols, 2 * TK) : div_up(a.ncols, TK), T, smem, st, a);
 }
 template <int L, bool D2>
 static cudaError_t fx_launch_conv(const ConvArgs& a, cudaStream_t st) {
