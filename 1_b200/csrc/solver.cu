@@ -1167,6 +1167,8 @@ extern "C" int mmx_solver_device_control(mmx_solver* s, int on) {
     h.time = s->time;
     h.dt = s->dt;
     h.accept = 1;
+    h.torque = s->torque;  // what the state and the next table row report until a trial has run
+    h.err = s->step_error;
     // host steps may still run on any stream
     MMX_TRY(cudaDeviceSynchronize());
     MMX_TRY(cudaMemcpy(s->rkdev, &h, sizeof(h), cudaMemcpyHostToDevice));

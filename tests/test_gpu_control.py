@@ -1,0 +1,48 @@
+"""The device dt controller against the host one where the two meet: host
+steps before the switch."""
+import numpy as np
+import pytest
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+GRID = (48, 20, 3)
+
+
+def params(eng, solver, dt=1e-14, maxerror=1e-2, faithful=1, **set_):
+    p = eng.mmx_params(grid=GRID, cell=(4e-9, 4e-9, 4e-9), msat=1.1e6, aexch=1.5e-11, alpha=0.5, anis=1, k1=5e5,
+                       axis=(0, 0, 1), bext=(0.01, -0.02, 0.03), solver=solver, dt=dt, maxerror=maxerror,
+                       faithful=faithful)
+    for k, v in set_.items():
+        setattr(p, k, v)
+    return p
+
+
+@pytest.mark.parametrize("max_dt", [0.0, 1e-14])
+@pytest.mark.parametrize("solver", ["rk23", "rkdp", "rk12", "rkck"])
+def test_switch_after_host_steps(eng, cuda, solver, max_dt):
+    """Host steps, then a run: the controllers write the same rows, the first
+    one with the torque of the last host step, and take the same steps; the
+    switch keeps the torque and the error."""
+    out = []
+    for dev in (False, True):
+        s = eng.Solver(params(eng, solver, max_dt=max_dt))
+        s.set_m(O.seeded_m(GRID, 31, "random"))
+        s.step(3)
+        before = s.state()
+        assert before["torque"] > 0
+        if dev:
+            # on, off and on again: nothing is lost on the way
+            for on in (True, False, True) if solver in ("rk12", "rkck") else (True,):
+                s.device_control(on)
+                assert s.state() == before
+        rows = s.run(4.5e-14, 1e-15)
+        assert rows[0, 4] == np.float32(before["torque"])
+        out.append((rows, s.state(), s.get_m()))
+        s.close()
+    (ra, sa, ma), (rb, sb, mb) = out
+    assert sa["steps"] == sb["steps"] and ra.shape == rb.shape and len(ra) >= (4 if max_dt else 1)
+    assert np.abs(ra - rb).max() <= 1e-6 * np.abs(ra).max()
+    assert abs(sa["time"] - sb["time"]) <= 1e-6 * sa["time"]
+    assert np.abs(ma - mb).max() < 1e-6
