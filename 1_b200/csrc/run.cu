@@ -130,8 +130,6 @@ __global__ void k_energy(const float* __restrict__ m, const float* __restrict__ 
 }
 
 void solver_run_free(mmx_solver* s) {
-  if (s->rungraph) cudaGraphExecDestroy(s->rungraph);
-  s->rungraph = nullptr;
   cudaFree(s->runbuf);
   cudaFree(s->rows_dev);
   cudaFree(s->eacc);

@@ -744,13 +744,22 @@ static void free_step_graphs(mmx_solver* s) {
   s->gexec = s->gexec_carry = nullptr;
 }
 static void free_profile_graph(mmx_solver* s);
+// Every graph captured so far: steps, profiled steps, trials, the run loop.
+// Their kernels hold the solver's parameters as they were at the capture.
+static void free_graphs(mmx_solver* s) {
+  free_step_graphs(s);
+  free_profile_graph(s);
+  for (cudaGraphExec_t& g : s->dgraph) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
+  if (s->rungraph) cudaGraphExecDestroy(s->rungraph);
+  s->rungraph = nullptr;
+}
 static void solver_free(mmx_solver* s) {
   if (!s) return;
+  free_graphs(s);
   solver_run_free(s);
-  free_profile_graph(s);
-  free_step_graphs(s);
-  for (int g = 0; g < 2; g++)
-    if (s->dgraph[g]) cudaGraphExecDestroy(s->dgraph[g]);
   cudaFree(s->rkdev);
   cudaFree(s->block);
   cudaFree(s->kt_tc);
@@ -1401,7 +1410,7 @@ extern "C" int mmx_solver_state(mmx_solver* s, double* time, float* dt, float* m
 extern "C" int mmx_solver_set_hext(mmx_solver* s, const float hext[3]) {
   if (!s || !hext) { mmx_set_error("null argument"); return MMX_ERR_ARG; }
   for (int d = 0; d < 3; d++) s->p.hext[d] = hext[d];
-  free_step_graphs(s);
+  free_graphs(s);
   return MMX_OK;
 }
 

@@ -140,7 +140,7 @@ struct RunLoop {
 cudaError_t solver_device_trial(mmx_solver* s, cudaStream_t st, bool first, const RunLoop* loop = nullptr);
 // Reads the device controller's time, dt and step counts back (syncs).
 int solver_device_download(mmx_solver* s);
-// Frees the run loop's buffers and graph (run.cu).
+// Frees the run loop's buffers (run.cu).
 void solver_run_free(mmx_solver* s);
 // One solver step (host controller), as mmx_solver_step takes it.
 int solver_step_once(mmx_solver* s, cudaStream_t st);

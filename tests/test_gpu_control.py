@@ -1,5 +1,7 @@
 """The device dt controller against the host one where the two meet: host
-steps before the switch."""
+steps before the switch, a field changed between trials."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -46,3 +48,44 @@ def test_switch_after_host_steps(eng, cuda, solver, max_dt):
     assert np.abs(ra - rb).max() <= 1e-6 * np.abs(ra).max()
     assert abs(sa["time"] - sb["time"]) <= 1e-6 * sa["time"]
     assert np.abs(ma - mb).max() < 1e-6
+
+
+def test_field_changed_between_trials(eng, cuda):
+    """set_hext holds for the trials, the run and the profiled steps that
+    follow it, whatever graph was captured before it."""
+    h2 = (ctypes.c_float * 3)(0.4, -0.3, 0.2)
+    m0 = O.seeded_m(GRID, 34, "random")
+
+    def pair(solver, prepare, advance, change=True, **kw):
+        s = eng.Solver(params(eng, solver, **kw))
+        s.set_m(m0)
+        prepare(s)
+        advance(s)
+        if change:
+            assert eng.lib().mmx_solver_set_hext(s.h, h2) == 0
+        advance(s)
+        m = s.get_m()
+        # and from a new m (an FSAL solver's first trial)
+        s.set_m(m0)
+        advance(s)
+        m = np.concatenate([m, s.get_m()])
+        s.close()
+        return m
+
+    def trials(s):
+        s.step(3)
+
+    def run(s):
+        s.run(2.5e-14, 1e-15)
+
+    for solver in ("rk23", "rk12"):
+        for adv in (trials, run):
+            want = pair(solver, lambda s: s.device_control(False), adv, max_dt=1e-14)
+            got = pair(solver, lambda s: s.device_control(True), adv, max_dt=1e-14)
+            old = pair(solver, lambda s: s.device_control(False), adv, change=False, max_dt=1e-14)
+            assert np.abs(want - old).max() > 1e-4
+            assert np.abs(got - want).max() < 1e-6, (solver, adv.__name__)
+    for solver in ("heun", "rk4"):
+        want = pair(solver, lambda s: None, trials, maxerror=0.0)
+        for prepare in (lambda s: s.use_graph(True), lambda s: s.profile(2)):
+            assert np.array_equal(pair(solver, prepare, trials, maxerror=0.0), want), solver
