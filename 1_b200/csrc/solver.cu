@@ -300,7 +300,9 @@ static cudaError_t launch_zinv_fwd(mmx_solver* s, const EpiArgs& ea, cudaStream_
 bool solver_z_chain(const mmx_solver* s) {
   return s->N[2] == s->P[2] / 2 && s->p.periodic[2] == 0;
 }
-// Fixed-step Heun: the spectrum buffer holds zfwd(m) between steps (spec_ready).
+// Fixed-step Heun: the spectrum buffer holds zfwd(m) between the steps of a
+// call, and from call to call (spec_ready) as long as the program has not
+// asked for m's device address, through which it may write m (m_lent).
 static bool heun_fused(const mmx_solver* s) {
   return s->p.solver == MMX_SOLVER_HEUN && s->p.max_error == 0.f && solver_z_chain(s);
 }
@@ -373,7 +375,9 @@ EpiArgs solver_base_args(mmx_solver* s) {
 }
 
 // ------------------------------ steps ---------------------------------
-static cudaError_t heun_step(mmx_solver* s, cudaStream_t st) {
+// have_z: the spectrum buffer holds the forward Z of m; go_on: leave that of
+// the new m there (both only where heun_fused).
+static cudaError_t heun_step(mmx_solver* s, cudaStream_t st, bool have_z, bool go_on) {
   // dtGilbert = dt / (1 + alpha^2)   (torque.go:49-51)
   float dtg = f32_div(s->dt, f32_add(1.f, f32_mul(s->p.alpha, s->p.alpha)));
   cudaError_t e;
@@ -381,7 +385,7 @@ static cudaError_t heun_step(mmx_solver* s, cudaStream_t st) {
   ea.dtg = dtg;
   const bool fused = heun_fused(s);
   // predictor
-  if (!fused || !s->spec_ready) {
+  if (!have_z) {
     e = zfwd_only(s, s->m, st);
     if (e != cudaSuccess) return e;
   }
@@ -409,9 +413,7 @@ static cudaError_t heun_step(mmx_solver* s, cudaStream_t st) {
     e = cudaMemsetAsync(s->scratch, 0, sizeof(float), st);
     if (e != cudaSuccess) return e;
   }
-  e = fused ? launch_zinv_fwd<EPI_HEUN2>(s, ea, st) : launch_zinv<EPI_HEUN2>(s, ea, st);
-  s->spec_ready = fused ? 1 : 0;
-  return e;
+  return go_on ? launch_zinv_fwd<EPI_HEUN2>(s, ea, st) : launch_zinv<EPI_HEUN2>(s, ea, st);
 }
 
 // The input of RK stage i: m + dt sum_j a_ij k_j over the non-zero weights.
@@ -952,8 +954,11 @@ float solver_cell_volume(const mmx_solver* s) {
 
 static int step_once(mmx_solver* s, cudaStream_t st) {
   if (s->p.solver == MMX_SOLVER_HEUN) {
-    cudaError_t e = heun_step(s, st);
+    const bool fused = heun_fused(s), have_z = fused && s->spec_ready, go_on = fused && (s->more_steps || !s->m_lent);
+    s->spec_ready = 0;
+    cudaError_t e = heun_step(s, st, have_z, go_on);
     if (e != cudaSuccess) { mmx_set_error(cudaGetErrorString(e)); return MMX_ERR_CUDA; }
+    s->spec_ready = go_on;
     s->time += (double)s->dt;
     if (s->p.max_error != 0.f) return heun_adaptive_update(s, st);
     return MMX_OK;
@@ -1244,8 +1249,8 @@ static cudaError_t rk_fixed_launches(mmx_solver* s, cudaStream_t st, bool carry)
   return e;
 }
 
-static cudaError_t step_launches(mmx_solver* s, cudaStream_t st, bool carry = false) {
-  return s->p.solver == MMX_SOLVER_HEUN ? heun_step(s, st) : rk_fixed_launches(s, st, carry);
+static cudaError_t step_launches(mmx_solver* s, cudaStream_t st, bool carry) {
+  return s->p.solver == MMX_SOLVER_HEUN ? heun_step(s, st, carry, carry) : rk_fixed_launches(s, st, carry);
 }
 
 static void free_profile_graph(mmx_solver* s) {
@@ -1276,7 +1281,7 @@ static int profiled_graph_steps(mmx_solver* s, int nsteps, cudaStream_t st) {
       cudaGraph_t g;
       MMX_TRY(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
       s->capture_events = 1;
-      cudaError_t e = step_launches(s, cap);
+      cudaError_t e = step_launches(s, cap, heun_fused(s));
       s->capture_events = 0;
       cudaError_t e2 = cudaStreamEndCapture(cap, &g);
       if (own) cudaStreamDestroy(cap);
@@ -1305,8 +1310,14 @@ extern "C" int mmx_solver_step(mmx_solver* s, int nsteps, cudaStream_t st) {
   if (s->devctl) return rk_device_steps(s, nsteps, st);
   const bool fixed_graphable =
       ((s->p.solver == MMX_SOLVER_HEUN && s->p.max_error == 0.f) || rk_fixed(s)) && s->p.thermal_k == 0.f;
+  const bool rk = s->p.solver != MMX_SOLVER_HEUN;
+  // several steps in one call hand the forward Z of m from step to step; a
+  // call starts from m itself, but for Heun calls of a program that cannot
+  // have written m since the last one (film 64 x 16, a step a call: 20.5 us
+  // against 22.5 us)
+  if (rk || s->m_lent) s->spec_ready = 0;
   if (s->profile == 2 && fixed_graphable && !s->want_energy) {
-    if (s->p.solver != MMX_SOLVER_HEUN && s->dt_uploaded != s->dt) {
+    if (rk && s->dt_uploaded != s->dt) {
       MMX_TRY(cudaMemcpyAsync(s->scratch + 2, &s->dt, sizeof(float), cudaMemcpyHostToDevice, st));
       MMX_TRY(cudaStreamSynchronize(st));
       s->dt_uploaded = s->dt;
@@ -1314,20 +1325,16 @@ extern "C" int mmx_solver_step(mmx_solver* s, int nsteps, cudaStream_t st) {
     return profiled_graph_steps(s, nsteps, st);
   }
   bool graphable = s->use_graph && !s->profile && !s->want_energy && fixed_graphable;
-  const bool rk = s->p.solver != MMX_SOLVER_HEUN;
   if (graphable && rk && s->dt_uploaded != s->dt) {
     MMX_TRY(cudaMemcpyAsync(s->scratch + 2, &s->dt, sizeof(float), cudaMemcpyHostToDevice, st));
     MMX_TRY(cudaStreamSynchronize(st));
     s->dt_uploaded = s->dt;
   }
-  // several Runge-Kutta steps in one call hand the forward Z of m from step
-  // to step; each call starts from m itself
-  if (rk) s->spec_ready = 0;
-  const bool carry = rk && graphable && nsteps > 1 && solver_z_chain(s);
+  const bool carry = graphable && solver_z_chain(s) && (nsteps > 1 || !(rk || s->m_lent));
   cudaGraphExec_t& gexec = carry ? s->gexec_carry : s->gexec;
   cudaStream_t& gstream = carry ? s->gstream_carry : s->gstream;
   for (int k = 0; k < nsteps; k++) {
-    if (graphable && (heun_fused(s) || carry) && !s->spec_ready) {
+    if (carry && !s->spec_ready) {
       // the captured step expects the forward Z spectrum of m in S
       cudaError_t e = zfwd_only(s, s->m, st);
       if (e != cudaSuccess) { mmx_set_error(cudaGetErrorString(e)); return MMX_ERR_CUDA; }
@@ -1414,7 +1421,11 @@ extern "C" int mmx_solver_set_hext(mmx_solver* s, const float hext[3]) {
   return MMX_OK;
 }
 
-extern "C" float* mmx_solver_m_device(mmx_solver* s) { return s ? s->m : nullptr; }
+extern "C" float* mmx_solver_m_device(mmx_solver* s) {
+  if (!s) return nullptr;
+  s->m_lent = 1;
+  return s->m;
+}
 extern "C" float* mmx_solver_torque_device(mmx_solver* s) { return s ? s->scratch + 1 : nullptr; }
 
 extern "C" int mmx_solver_use_graph(mmx_solver* s, int on) {

@@ -66,6 +66,7 @@ struct mmx_solver {
   long long steps = 0;
   int fsal_init = 0;
   int spec_ready = 0;  // S holds the forward Z spectrum of m (between Heun steps; RK: within one call)
+  int m_lent = 0;      // the program has m's device address: each call starts from m itself
   int more_steps = 0;  // the caller takes another step right after this one
   float dt_uploaded = -1.f;  // dt last written to the device scalar by the graph path
   // tableau
@@ -82,7 +83,7 @@ struct mmx_solver {
   int use_graph = 0;
   cudaGraphExec_t gexec = nullptr;
   cudaStream_t gstream = nullptr;
-  cudaGraphExec_t gexec_carry = nullptr;  // fixed RK step that starts and ends with zfwd(m) in S
+  cudaGraphExec_t gexec_carry = nullptr;  // fixed step that starts and ends with zfwd(m) in S
   cudaStream_t gstream_carry = nullptr;
   // run loop with table output (run.cu)
   void* runbuf = nullptr;                 // RunDev on the device

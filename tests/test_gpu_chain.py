@@ -105,3 +105,42 @@ def test_batch_steps_in_one_call(eng, cuda, solver):
     for how in got:
         for x, y in zip(got[how], got["plain"]):
             assert np.array_equal(x, y), how
+
+
+@pytest.mark.parametrize("how", ["graph", "plain", "profile"])
+@pytest.mark.parametrize("n", [1, 2])
+def test_heun_m_written_between_calls(eng, cuda, how, n):
+    """A Heun call, too, starts from m itself once the program holds its
+    device address; the steps of solvers whose address nobody took stay the
+    same."""
+    import torch
+    c = config((48, 20, 3), (0, 0, 0), "heun")
+    m1, m2 = O.seeded_m(c["grid"], 15, "random"), O.seeded_m(c["grid"], 16, "random")
+
+    def solver():
+        s = eng.Solver(eng.mmx_params(**c))
+        s.use_graph(how == "graph")
+        s.profile(2 if how == "profile" else 0)
+        return s
+
+    a, b, other = solver(), solver(), solver()
+    a.set_m(m1)
+    a.step(3)
+    buf = torch.from_numpy(m2).cuda()
+    torch.cuda.synchronize()
+    for s in (b, other):
+        s.set_m(m2)
+    for k in range(3):
+        # m of solver a takes what the program has, the state of the others at first
+        if k:
+            buf = torch.from_numpy(b.get_m()).cuda()
+            torch.cuda.synchronize()
+        eng.lib().memcpy_on_gpu(ctypes.c_void_p(buf.data_ptr()), ctypes.c_void_p(a.m_device()), buf.numel())
+        for s in (a, b, other):
+            s.step(n)
+        if k == 0:
+            assert b.m_device()  # taken after its first steps
+        assert np.array_equal(a.get_m(), b.get_m())
+        assert np.array_equal(a.get_m(), other.get_m())
+    for s in (a, b, other):
+        s.close()
