@@ -930,6 +930,14 @@ __host__ __device__ constexpr size_t conv_smem(int L, int TK, bool split) {
 // fit an SM only with spilled registers, and three components in one block
 // are faster (512 x 512 film, RK23 trial: 104 us against 119 us split).
 __host__ __device__ constexpr bool conv_split(int L, int TK) { return TK < 4 || TK * conv_bf(L) <= 256; }
+// columns of a single-grid pass: conv_tkp, but half of them where three
+// components of so many do not fit an SM beside the twiddles (X lines of 4096
+// points: 262144 bytes)
+__host__ __device__ constexpr int conv_cols(int L, bool d2) {
+  return !(d2 && conv_split(L, conv_tkp(L))) && conv_smem(L, conv_tkp(L), false) + sizeof(float2) * L > SMEM_MOST
+             ? conv_tkp(L) / 2
+             : conv_tkp(L);
+}
 __host__ __device__ constexpr int conv_threads(int L, int TK) {
   return TK * conv_bf(L) < 64 ? 64 : TK * conv_bf(L) > 512 ? 512 : (TK * conv_bf(L) + 31) / 32 * 32;
 }
@@ -937,20 +945,23 @@ __host__ __device__ constexpr int fx_threads(int elems) {
   return elems / 16 < 64 ? 64 : (elems / 16 > 512 ? 512 : ((elems / 16 + 31) / 32) * 32);
 }
 
+// dynamic and static (twiddles; row offsets) shared memory of the tiles
+__host__ __device__ constexpr size_t col_smem(int L, int TK) { return sizeof(float2) * (size_t)odd_pitch(TK) * L; }
+__host__ __device__ constexpr size_t rows_smem(int M, int lines) { return sizeof(float2) * (size_t)lines * row_pitch(M); }
+__host__ __device__ constexpr size_t tw_smem(int L) { return sizeof(float2) * (size_t)L; }
+
 template <int L, bool INV>
 cudaError_t fx_launch_col(const float2* src, float2* dst, const ColPass& cp, cudaStream_t st) {
   constexpr int TK = fx_col_tk(L);
   constexpr int T = fx_threads(TK * L);
-  size_t smem = sizeof(float2) * (size_t)odd_pitch(TK) * L;
+  constexpr size_t smem = col_smem(L, TK);
   const int grid = div_up(cp.ncols * cp.nplanes, TK);
   const bool half = 2 * (INV ? cp.n_out : cp.n_in) == L;
-  if (half) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_col_fx<L, TK, T, INV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return launch_pass(k_col_fx<L, TK, T, INV, true>, grid, T, smem, st, src, dst, cp);
-  } else {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_col_fx<L, TK, T, INV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return launch_pass(k_col_fx<L, TK, T, INV, false>, grid, T, smem, st, src, dst, cp);
-  }
+  auto go = [&](auto kern) {
+    const cudaError_t e = smem_opt_in<smem, tw_smem(L)>(kern);
+    return e != cudaSuccess ? e : launch_pass(kern, grid, T, smem, st, src, dst, cp);
+  };
+  return half ? go(k_col_fx<L, TK, T, INV, true>) : go(k_col_fx<L, TK, T, INV, false>);
 }
 
 // rows per Z tile: 2048 elements for the forward pass (smaller blocks, more
@@ -974,8 +985,9 @@ template <int M, bool COMB>
 cudaError_t fx_launch_zr2c(const float* src, float2* dst, const ZPass& z, const ZComb& cb, cudaStream_t st) {
   constexpr int RT = fx_rows(M, 1);
   constexpr int T = fx_threads(RT * M);
-  size_t smem = sizeof(float2) * (size_t)RT * row_pitch(M);
-  if (smem > 48 * 1024) cudaFuncSetAttribute(k_zr2c_fx<M, RT, T, COMB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  constexpr size_t smem = rows_smem(M, RT);
+  const cudaError_t e = smem_opt_in<smem, tw_smem(M) + 16 * RT>(k_zr2c_fx<M, RT, T, COMB>);
+  if (e != cudaSuccess) return e;
   // 8-byte loads when every row starts at an even float offset
   int vec2 = (z.ld_real % 2 == 0) && (z.comp_stride_real % 2 == 0) && (((uintptr_t)src & 7) == 0);
   const int rt = rows_in_use(RT, z.nrows);
@@ -986,8 +998,9 @@ template <int M>
 cudaError_t fx_launch_zc2r(const float2* src, float* dst, const ZPass& z, cudaStream_t st) {
   constexpr int RT = fx_rows(M, 1);
   constexpr int T = fx_threads(RT * M);
-  size_t smem = sizeof(float2) * (size_t)RT * row_pitch(M);
-  if (smem > 16 * 1024) cudaFuncSetAttribute(k_zc2r_fx<M, RT, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  constexpr size_t smem = rows_smem(M, RT);
+  const cudaError_t e = smem_opt_in<smem, tw_smem(M) + 16 * RT>(k_zc2r_fx<M, RT, T>);
+  if (e != cudaSuccess) return e;
   // 8-byte stores when every row starts at an even float offset
   const int vec2 = z.ld_real % 2 == 0 && z.comp_stride_real % 2 == 0 && ((uintptr_t)dst & 7) == 0;
   const int rt = rows_in_use(RT, z.nrows);

@@ -1,11 +1,6 @@
 // The batch's column (Y) passes in both tile widths and its forward Z passes.
 #include "fx_dispatch.cuh"
 
-template <typename K>
-static void set_smem(K kern, size_t bytes) {
-  if (bytes > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 template <int L, int TK, int T, bool INV, bool HALF>
 __global__ void __launch_bounds__(T) kb_col(const BCol* __restrict__ a, const int* __restrict__ starts,
                                              int nseg) {
@@ -25,17 +20,15 @@ __global__ void __launch_bounds__(T) kb_zr2c(const BZr2c* __restrict__ a, const 
 template <int L, int TK>
 static cudaError_t run_col_tk(const BatchLaunch& l, cudaStream_t st) {
   constexpr int T = fx_threads(TK * L);
-  size_t smem = sizeof(float2) * (size_t)odd_pitch(TK) * L;
-#define KB_COL_(INV, HALF)                                                                        \
-  set_smem(kb_col<L, TK, T, INV, HALF>, smem);                                                    \
-  kb_col<L, TK, T, INV, HALF><<<l.blocks, T, smem, st>>>((const BCol*)l.args, l.starts, l.nseg);
-  if (l.flag) {
-    if (l.half) { KB_COL_(true, true) } else { KB_COL_(true, false) }
-  } else {
-    if (l.half) { KB_COL_(false, true) } else { KB_COL_(false, false) }
-  }
-#undef KB_COL_
-  return cudaGetLastError();
+  constexpr size_t smem = col_smem(L, TK);
+  auto go = [&](auto kern) {
+    const cudaError_t e = smem_opt_in<smem, tw_smem(L)>(kern);
+    if (e != cudaSuccess) return e;
+    kern<<<l.blocks, T, smem, st>>>((const BCol*)l.args, l.starts, l.nseg);
+    return cudaGetLastError();
+  };
+  if (l.flag) return l.half ? go(kb_col<L, TK, T, true, true>) : go(kb_col<L, TK, T, true, false>);
+  return l.half ? go(kb_col<L, TK, T, false, true>) : go(kb_col<L, TK, T, false, false>);
 }
 template <int L>
 static cudaError_t run_col(const BatchLaunch& l, cudaStream_t st) {
@@ -45,15 +38,14 @@ template <int M>
 static cudaError_t run_zr2c(const BatchLaunch& l, cudaStream_t st) {
   constexpr int RT = fx_rows(M, 1);
   constexpr int T = fx_threads(RT * M);
-  size_t smem = sizeof(float2) * (size_t)RT * row_pitch(M);
-  if (l.flag) {
-    set_smem(kb_zr2c<M, RT, T, true>, smem);
-    kb_zr2c<M, RT, T, true><<<l.blocks, T, smem, st>>>((const BZr2c*)l.args, l.starts, l.nseg);
-  } else {
-    set_smem(kb_zr2c<M, RT, T, false>, smem);
-    kb_zr2c<M, RT, T, false><<<l.blocks, T, smem, st>>>((const BZr2c*)l.args, l.starts, l.nseg);
-  }
-  return cudaGetLastError();
+  constexpr size_t smem = rows_smem(M, RT);
+  auto go = [&](auto kern) {
+    const cudaError_t e = smem_opt_in<smem, tw_smem(M) + 16 * RT>(kern);
+    if (e != cudaSuccess) return e;
+    kern<<<l.blocks, T, smem, st>>>((const BZr2c*)l.args, l.starts, l.nseg);
+    return cudaGetLastError();
+  };
+  return l.flag ? go(kb_zr2c<M, RT, T, true>) : go(kb_zr2c<M, RT, T, false>);
 }
 
 cudaError_t bx_col(const BatchLaunch& l, cudaStream_t st) {

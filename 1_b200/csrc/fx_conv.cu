@@ -20,11 +20,12 @@ __device__ __forceinline__ void conv_block(const ConvArgs& a, int bx) {
 // at least 768 resident threads per SM (6 blocks of 128 for L = 64):
 // measured faster than the unconstrained 96-register build (5 blocks) and
 // than 7 or 8 blocks (register spills).  Split blocks of a film: 1024, as far
-// as the shared memory of a block allows.
+// as the shared memory of a block allows.  A block that leaves no room for a
+// second one has the registers to itself.
 __host__ __device__ constexpr int conv_min_blocks(int L, int TK, int T, bool split) {
   const int want = (split ? 1024 : 768) / T;
   const int fit = (int)(220 * 1024 / (conv_smem(L, TK, split) + sizeof(float2) * L + 1024));
-  return want < 1 || (split && fit < 1) ? 1 : !split || want < fit ? want : fit;
+  return want < 1 || fit < 2 ? 1 : !split || want < fit ? want : fit;
 }
 template <int L, int TK, int T, bool D2, bool HALF>
 __global__ void __launch_bounds__(T, conv_min_blocks(L, TK, T, D2 && conv_split(L, TK))) k_conv_fx(ConvArgs a) {
@@ -61,14 +62,16 @@ static cudaError_t launch_conv(const ConvArgs& a, cudaStream_t st) {
     const int blocks = div_up(a.ncols, TK);
     if (blocks <= mmx_sm_count()) {
       constexpr size_t smem = conv_smem(L, TK, false);
-      if (smem > 24 * 1024) cudaFuncSetAttribute(k_conv_wide<L, TK, T, D2, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      const cudaError_t e = smem_opt_in<smem, tw_smem(L)>(k_conv_wide<L, TK, T, D2, HALF>);
+      if (e != cudaSuccess) return e;
       return launch_pass(k_conv_wide<L, TK, T, D2, HALF>, blocks, T, smem, st, a);
     }
   }
-  constexpr int TK = conv_tkp(L), T = conv_threads(L, TK);
+  constexpr int TK = conv_cols(L, D2), T = conv_threads(L, TK);
   constexpr bool split = D2 && conv_split(L, TK);
   constexpr size_t smem = conv_smem(L, TK, split);
-  if (smem > 24 * 1024) cudaFuncSetAttribute(k_conv_fx<L, TK, T, D2, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = smem_opt_in<smem, tw_smem(L)>(k_conv_fx<L, TK, T, D2, HALF>);
+  if (e != cudaSuccess) return e;
   return launch_pass(k_conv_fx<L, TK, T, D2, HALF>, split ? 3 * div_up(a.ncols, 2 * TK) : div_up(a.ncols, TK), T, smem, st, a);
 }
 template <int L, bool D2>
@@ -82,7 +85,8 @@ static cudaError_t run_conv(const BatchLaunch& l, cudaStream_t st) {
   constexpr int TK = conv_tkp_narrow(L), T = conv_threads(L, TK);
   constexpr bool split = D2 && conv_split(L, TK);
   constexpr size_t smem = conv_smem(L, TK, split);
-  if (smem > 24 * 1024) cudaFuncSetAttribute(kb_conv<L, TK, T, D2, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = smem_opt_in<smem, tw_smem(L)>(kb_conv<L, TK, T, D2, HALF>);
+  if (e != cudaSuccess) return e;
   kb_conv<L, TK, T, D2, HALF><<<l.blocks, T, smem, st>>>((const ConvArgs*)l.args, l.starts, l.nseg);
   return cudaGetLastError();
 }

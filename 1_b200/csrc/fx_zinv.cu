@@ -28,9 +28,10 @@ static cudaError_t launch(ZinvArgs za, bool fuse, cudaStream_t st) {
   constexpr int RT = fx_rows(M, 3);
   za.rt = rows_in_use(RT, za.nrows);
   constexpr int T = fx_threads(3 * RT * M);
-  size_t smem = sizeof(float2) * (size_t)3 * RT * row_pitch(M);
+  constexpr size_t smem = rows_smem(M, 3 * RT);
   auto go = [&](auto kern) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = smem_opt_in<smem, tw_smem(M) + 8 * RT>(kern);
+    if (e != cudaSuccess) return e;
     return launch_pass(kern, div_up(za.nrows, za.rt), T, smem, st, za);
   };
   if (!fuse) return go(k_zinv_fx<M, RT, T, FX_MODE>);
@@ -41,9 +42,10 @@ template <int M>
 static cudaError_t launch_batch(const BatchLaunch& l, bool fuse, cudaStream_t st) {
   constexpr int RT = fx_rows(M, 3);
   constexpr int T = fx_threads(3 * RT * M);
-  size_t smem = sizeof(float2) * (size_t)3 * RT * row_pitch(M);
+  constexpr size_t smem = rows_smem(M, 3 * RT);
   auto go = [&](auto kern) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = smem_opt_in<smem, tw_smem(M) + 8 * RT>(kern);
+    if (e != cudaSuccess) return e;
     kern<<<l.blocks, T, smem, st>>>((const ZinvArgs*)l.args, l.starts, l.nseg);
     return cudaGetLastError();
   };

@@ -73,6 +73,19 @@ static inline int div_up(int64_t a, int64_t b) { return (int)((a + b - 1) / b); 
 // Number of SMs of the current device (cached per process).
 int mmx_sm_count();
 
+// Shared memory of a block, static and dynamic together, that needs no
+// opt-in, and the most that a block can have (sm_100).
+constexpr size_t SMEM_FREE = 48 * 1024, SMEM_MOST = 227 * 1024;
+// Opts a kernel in for a launch with DYN dynamic bytes next to its STAT static
+// ones.  (The limit without opt-in is on the sum: a test of the dynamic bytes
+// alone refused columns of 2048 points, 48 KB of tile + 16 KB of twiddles.)
+template <size_t DYN, size_t STAT, typename K>
+static cudaError_t smem_opt_in(K kern) {
+  static_assert(DYN + STAT <= SMEM_MOST, "the tile does not fit an SM");
+  if (DYN + STAT <= SMEM_FREE) return cudaSuccess;
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DYN);
+}
+
 // ---------------------------------------------------------------------
 #ifndef PASS_OVERLAP_GRID
 #define PASS_OVERLAP_GRID 1
