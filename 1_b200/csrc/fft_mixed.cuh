@@ -572,9 +572,13 @@ __global__ void __launch_bounds__(T_ROW, 2) k_zinv_mix(float2* S, LineFFT fz, co
 // ---------------------------------------------------------------------
 // launch shapes
 // ---------------------------------------------------------------------
+// A kernel's opt-in is one value for the process, and launches of different
+// tiles may come from several threads: it is always the largest tile's.
+constexpr int TILE_MOST = 200 * 1024;
 template <typename K>
 static cudaError_t allow(K kern, size_t bytes) {
-  return bytes > 40 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)
+  if (bytes > TILE_MOST) return cudaErrorInvalidValue;
+  return bytes > 40 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_MOST)
                            : cudaSuccess;
 }
 // widest tile (2^lg columns, at most 16 and no more than there are, fewer
@@ -586,7 +590,7 @@ static inline int pick_columns(int L, int comps, int tiles, int64_t ncols, size_
   while (lg > 0 && (1ll << (lg - 1)) >= ncols) lg--;
   while (lg > 2 && (ncols >> lg) < mmx_sm_count()) lg--;
   while (lg > 2 && need(lg) > 72 * 1024) lg--;
-  while (lg > 0 && need(lg) > 200 * 1024) lg--;
+  while (lg > 0 && need(lg) > TILE_MOST) lg--;
   *bytes = need(lg);
   return lg;
 }
