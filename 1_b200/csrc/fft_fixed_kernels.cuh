@@ -489,7 +489,7 @@ __device__ __forceinline__ void conv_wide_body(const ConvArgs& a, int bx, float2
 
 // FULL: blocks take RT rows (the batch), else rt of them.
 template <int M, int RT, int T, bool COMB, bool FULL>
-__device__ __forceinline__ void zr2c_body(const float* __restrict__ src, float2* __restrict__ dst, const ZPass& z,
+__device__ __forceinline__ void zr2c_body(const float* src, float2* dst, const ZPass& z,
                                           const ZComb& cb, int vec2, int rt, int bx) {
   __shared__ float2 tw[M];
   __shared__ int64_t roff_s[RT], soff_s[RT];
@@ -529,7 +529,7 @@ __device__ __forceinline__ void zr2c_body(const float* __restrict__ src, float2*
 #pragma unroll
       for (int q = 0; q < R0; q++) {
         const int i0 = 2 * S0::in_idx(j, q);
-        v[q] = i0 + 1 < nreal ? __ldg(reinterpret_cast<const float2*>(cb.m0 + roff + i0)) : make_float2(0.f, 0.f);
+        v[q] = i0 + 1 < nreal ? *reinterpret_cast<const float2*>(cb.m0 + roff + i0) : make_float2(0.f, 0.f);
         // the last value of an odd row
         if (i0 + 1 == nreal) v[q].x = cb.m0[roff + i0];
       }
@@ -541,7 +541,7 @@ __device__ __forceinline__ void zr2c_body(const float* __restrict__ src, float2*
 #pragma unroll
         for (int q = 0; q < R0; q++) {
           const int i0 = 2 * S0::in_idx(j, q);
-          kk[q] = i0 + 1 < nreal ? __ldg(reinterpret_cast<const float2*>(kt + i0)) : make_float2(0.f, 0.f);
+          kk[q] = i0 + 1 < nreal ? *reinterpret_cast<const float2*>(kt + i0) : make_float2(0.f, 0.f);
           if (i0 + 1 == nreal) kk[q].x = kt[i0];
         }
 #pragma unroll
@@ -566,7 +566,7 @@ __device__ __forceinline__ void zr2c_body(const float* __restrict__ src, float2*
             if (i0 < nreal) { a = zcomb_value(cb, dt, roff + i0); cb.out[roff + i0] = a; }
             if (i0 + 1 < nreal) { b = zcomb_value(cb, dt, roff + i0 + 1); cb.out[roff + i0 + 1] = b; }
           } else if (vec2 && i0 + 1 < nreal) {
-            const float2 p = __ldg(reinterpret_cast<const float2*>(src + roff + i0));
+            const float2 p = *reinterpret_cast<const float2*>(src + roff + i0);
             a = p.x;
             b = p.y;
           } else {
@@ -602,7 +602,7 @@ __device__ __forceinline__ void zr2c_body(const float* __restrict__ src, float2*
 }
 
 template <int M, int RT, int T, bool COMB>
-__global__ void __launch_bounds__(T) k_zr2c_fx(const float* __restrict__ src, float2* __restrict__ dst, ZPass z,
+__global__ void __launch_bounds__(T) k_zr2c_fx(const float* src, float2* dst, ZPass z,
                                                ZComb cb, int vec2, int rt) {
   zr2c_body<M, RT, T, COMB, false>(src, dst, z, cb, vec2, rt, blockIdx.x);
 }
@@ -623,7 +623,7 @@ __device__ __forceinline__ float2 c2r_pre(float2 Xk, float2 Xm, int k, int M, co
 // every point read twice and all stages in shared memory, took 15.4 us where
 // this takes as long as the forward pass (128 x 128 x 16 grid: 5.3 us).
 template <int M, int RT, int T>
-__global__ void __launch_bounds__(T) k_zc2r_fx(const float2* __restrict__ src, float* __restrict__ dst, ZPass z,
+__global__ void __launch_bounds__(T) k_zc2r_fx(const float2* src, float* dst, ZPass z,
                                                int vec2, int rt) {
   __shared__ float2 tw[M];
   __shared__ int64_t roff_s[RT], soff_s[RT];

@@ -360,7 +360,7 @@ __device__ __forceinline__ float2 merge_pair(float2 Xk, float2 Xm, int k, const 
 constexpr int MAX_ROWS = 32;
 
 template <bool COMB>
-__global__ void __launch_bounds__(T_ROW) k_zr2c_mix(const float* __restrict__ src, float2* __restrict__ dst, ZPass z,
+__global__ void __launch_bounds__(T_ROW) k_zr2c_mix(const float* src, float2* dst, ZPass z,
                                                     ZComb cb, int vec2, int RT) {
   extern __shared__ float2 sm[];
   __shared__ int64_t roff_s[MAX_ROWS], soff_s[MAX_ROWS];
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(T_ROW) k_zr2c_mix(const float* __restrict__ sr
       gi[u] = roff_s[l] + 2 * n;
       two[u] = 2 * n + 1 < nreal;
       const float* s = COMB ? cb.m0 : src;
-      if (vec2 && two[u]) v[u] = __ldg(reinterpret_cast<const float2*>(s + gi[u]));
+      if (vec2 && two[u]) v[u] = *reinterpret_cast<const float2*>(s + gi[u]);
       else v[u] = make_float2(s[gi[u]], two[u] ? s[gi[u] + 1] : 0.f);
     }
     if (COMB) {
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(T_ROW) k_zr2c_mix(const float* __restrict__ sr
 #pragma unroll
         for (int u = 0; u < U; u++) {
           if (to[u] < 0) continue;
-          if (vec2 && two[u]) w[u] = __ldg(reinterpret_cast<const float2*>(kt + gi[u]));
+          if (vec2 && two[u]) w[u] = *reinterpret_cast<const float2*>(kt + gi[u]);
           else w[u] = make_float2(kt[gi[u]], two[u] ? kt[gi[u] + 1] : 0.f);
         }
 #pragma unroll
@@ -471,7 +471,7 @@ __device__ __forceinline__ void load_merged(float2* x, int lines, int M, int pit
 }
 
 template <int = 0>
-__global__ void __launch_bounds__(T_ROW) k_zc2r_mix(const float2* __restrict__ src, float* __restrict__ dst, ZPass z,
+__global__ void __launch_bounds__(T_ROW) k_zc2r_mix(const float2* src, float* dst, ZPass z,
                                                     int RT) {
   extern __shared__ float2 sm[];
   __shared__ int64_t roff_s[MAX_ROWS], soff_s[MAX_ROWS];

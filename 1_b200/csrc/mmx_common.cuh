@@ -98,6 +98,9 @@ static cudaError_t smem_opt_in(K kern) {
 // compiler from issuing the first spectrum loads before they arrive: 2% of a
 // 256 x 256 x 32 Heun step.)  Every pass ends after it has waited, so a pass
 // that has waited for its predecessor has waited for all before it.
+// What other kernels write a pass reads by plain loads: it is resident while
+// they still write, and the read-only path (__ldg, const __restrict__) is for
+// data that does not change in a kernel's lifetime (twiddles, the kernel octant).
 // ---------------------------------------------------------------------
 __device__ __forceinline__ void pass_begin() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pass_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

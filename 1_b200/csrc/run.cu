@@ -45,8 +45,6 @@ __global__ void k_run_force(RunDev* __restrict__ rd, float t) {
 // (simrun.go:27-35, simoutput.go:83-85); host-driven ones: k_run_force did.
 __global__ void k_run_row(RunDev* __restrict__ rd, const RkDev* __restrict__ dev, const float* __restrict__ m,
                           int64_t n, const float* __restrict__ torque) {
-  pass_begin();
-  pass_wait();
   float now;
   if (dev) {
     now = __fmul_rn(__double2float_rn(dev->time), rd->unit_time);
@@ -182,7 +180,8 @@ static int run_buffers(mmx_solver* s, int max_rows) {
 // the row reduction; dev: the device controller whose time decides, else k_run_force came before
 static cudaError_t row_launch(mmx_solver* s, RunDev* rd, const RkDev* dev, cudaStream_t st) {
   const float* torque = dev ? &dev->torque : s->p.solver == MMX_SOLVER_HEUN ? nullptr : s->scratch + 1;
-  return launch_pass(k_run_row, solver_grid_1d(s->n), 256, 0, st, rd, dev, s->m, s->n, torque);
+  k_run_row<<<solver_grid_1d(s->n), 256, 0, st>>>(rd, dev, s->m, s->n, torque);
+  return cudaGetLastError();
 }
 
 // outer graph: the loop condition, then a WHILE node whose body is

@@ -1023,8 +1023,6 @@ __global__ void k_rk_finish(float* __restrict__ m, const float* __restrict__ mne
                             const float* __restrict__ klast, int64_t n, float* __restrict__ scratch,
                             RkDev* __restrict__ dev, RkCtl c, int fsal, int faithful, RunDev* __restrict__ rd,
                             cudaGraphConditionalHandle h) {
-  pass_begin();
-  pass_wait();
   const float err = scratch[0];
   const bool acc = !(err > __fmul_rn(2.f, c.max_error));
   const bool copy = fsal && (acc || faithful);  // rk.go:311-315 (retry: faithful reuses the rejected k_last)
@@ -1136,9 +1134,10 @@ static cudaError_t rk_device_trial(mmx_solver* s, cudaStream_t st, bool first, c
     if ((e = rk_stage(s, i, st, dt_dev, have_z, zc && i < last)) != cudaSuccess) return e;
     have_z = zc;
   }
-  return launch_pass(k_rk_finish, solver_grid_1d(s->n), 256, 0, st, s->m, s->mnew, s->kb[0], s->kb[last], s->n,
-                     s->scratch, dev, c, s->fsal, s->p.faithful, loop ? loop->rd : (RunDev*)nullptr,
-                     loop ? loop->h : (cudaGraphConditionalHandle)0);
+  k_rk_finish<<<solver_grid_1d(s->n), 256, 0, st>>>(s->m, s->mnew, s->kb[0], s->kb[last], s->n, s->scratch, dev, c,
+                                                    s->fsal, s->p.faithful, loop ? loop->rd : nullptr,
+                                                    loop ? loop->h : 0);
+  return cudaGetLastError();
 }
 
 static int rk_device_download(mmx_solver* s) {
