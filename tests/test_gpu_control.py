@@ -1,5 +1,6 @@
 """The device dt controller against the host one where the two meet: host
-steps before the switch, a field changed between trials."""
+steps before the switch, torque-based dt bounds, rejected trials, a field
+changed between trials."""
 import ctypes
 
 import numpy as np
@@ -48,6 +49,59 @@ def test_switch_after_host_steps(eng, cuda, solver, max_dt):
     assert np.abs(ra - rb).max() <= 1e-6 * np.abs(ra).max()
     assert abs(sa["time"] - sb["time"]) <= 1e-6 * sa["time"]
     assert np.abs(ma - mb).max() < 1e-6
+
+
+# a step's largest change dm = dt max|k0| is some 0.01 at dt = 1e-14 s here
+@pytest.mark.parametrize("bounds", [dict(max_dm=2e-3), dict(min_dm=3e-2), dict(min_dt=1.5e-14), dict(max_dt=4e-15),
+                                    dict(min_dm=1e-3, max_dm=4e-3, min_dt=1e-17, max_dt=5e-15)])
+@pytest.mark.parametrize("solver", ["rk23", "rkdp", "rk12", "rkck"])
+def test_dt_bounds(eng, cuda, solver, bounds):
+    """min_dm, max_dm, min_dt and max_dt give both controllers the same dt,
+    another one than without them."""
+    out = []
+    for dev, b in ((False, {}), (False, bounds), (True, bounds)):
+        s = eng.Solver(params(eng, solver, **b))
+        s.set_m(O.seeded_m(GRID, 32, "random"))
+        s.device_control(dev)
+        s.step(3)
+        out.append((s.state(), s.get_m()))
+        s.close()
+    (free, _), (h, mh), (d, md) = out
+    assert h["steps"] == d["steps"] == 3
+    assert abs(h["time"] - free["time"]) > 1e-2 * free["time"]
+    for k in ("time", "dt", "torque"):
+        assert abs(h[k] - d[k]) <= 1e-6 * abs(h[k]), k
+    assert np.abs(mh - md).max() < 1e-6
+
+
+@pytest.mark.parametrize("max_dm", [0.0, 0.8])
+@pytest.mark.parametrize("faithful", [0, 1])
+@pytest.mark.parametrize("solver", ["rk23", "rkdp", "rk12", "rkck"])
+def test_rejected_trials(eng, cuda, solver, faithful, max_dm):
+    """A start dt that is far too large: the first trials are rejected, m
+    stays, and both controllers end at the same accepted steps.  faithful
+    restarts an FSAL trial from the rejected one's last torque."""
+    kw = dict(dt=8e-13, maxerror=1e-5, faithful=faithful, max_dm=max_dm)
+    m0 = O.seeded_m(GRID, 33, "random")
+    h = eng.Solver(params(eng, solver, **kw))
+    h.set_m(m0)
+    h.step(3)
+    d = eng.Solver(params(eng, solver, **kw))
+    d.set_m(m0)
+    d.device_control(True)
+    trials = 0
+    while d.state()["steps"] < 3 and trials < 40:
+        d.step(1)
+        trials += 1
+        if d.state()["steps"] == 0:
+            assert np.array_equal(d.get_m(), m0)
+    sh, sd = h.state(), d.state()
+    assert sh["steps"] == sd["steps"] == 3 and trials > 3
+    for k in ("time", "dt", "torque"):
+        assert abs(sh[k] - sd[k]) <= 1e-5 * abs(sh[k]), k
+    assert np.abs(h.get_m() - d.get_m()).max() < 1e-6
+    h.close()
+    d.close()
 
 
 def test_field_changed_between_trials(eng, cuda):
