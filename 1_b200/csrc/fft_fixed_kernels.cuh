@@ -684,8 +684,8 @@ struct ZinvArgs {
   EpiArgs ea;
 };
 
-// FUSE (Heun modes, open Z boundary): after the epilogue the block's new
-// magnetisation rows (the next evaluation's input) are still in its shared
+// FUSE (a step's modes, open Z boundary): after the epilogue the block's new
+// rows (the next evaluation's input) are still in its shared
 // tile, so the block also runs the next forward Z transform on them and
 // writes the same spectrum rows it read -- the next evaluation needs no
 // separate forward Z pass and never re-reads m.
@@ -889,7 +889,7 @@ __host__ __device__ constexpr int conv_tk_raw(int L) {
 // butterflies per column in the last forward stage (one thread each)
 __host__ __device__ constexpr int conv_bf(int L) { return L / fwd_radix(L, n_stages(L) - 1); }
 // Lines whose last stage has fewer than 8 butterflies per column (L = 2, 4,
-// 8, 16 in one stage; 6, 12 in two) take 128 / conv_bf columns, so that a
+// 6, 8, 12, 16 in one stage; 24 in two) take 128 / conv_bf columns, so that a
 // block still has 128 busy threads: a 16-column tile of L = 8 left 48 of
 // its 64 threads idle.
 __host__ __device__ constexpr int conv_tkp_narrow(int L) {

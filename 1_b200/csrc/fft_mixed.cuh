@@ -10,12 +10,12 @@
 // barrier; the first stage of a column reads global memory and the last one
 // writes it, so two-stage columns keep a single tile.  The inverse
 // transform is the forward one with real and imaginary parts exchanged on
-// the way in and out.
+// the way in and out.  Blocks have 256 threads for rows, and for columns what
+// pick_threads says.
 //
-// These kernels replace ones whose stages were limited to radix 8 (four
-// stages for 250 points), divided by run-time values several times per
-// element and passed through shared memory in place with two barriers a
-// stage.  Blocks have 256 threads for rows, and for columns what pick_threads says.
+// Several units include this header.  What is not a template by nature is one
+// of a defaulted parameter (template <int = 0>): a unit then compiles only the
+// kernels that it launches, and the units' copies are one function.
 #pragma once
 #include "epilogue.cuh"
 #include "fft_dft.cuh"
@@ -102,7 +102,7 @@ __host__ __device__ constexpr int odd_up(int n) { return n | 1; }
 // ---------------------------------------------------------------------
 constexpr int T_COL = 256;  // at most
 
-template <int = 0>  // instantiated where it is launched
+template <int = 0>
 __global__ void __launch_bounds__(T_COL, 2) k_col_mix(const float2* src, float2* dst, ColPass cp, int lg) {
   extern __shared__ float2 sm[];
   pass_begin();

@@ -87,9 +87,6 @@ static cudaError_t smem_opt_in(K kern) {
 }
 
 // ---------------------------------------------------------------------
-#ifndef PASS_OVERLAP_GRID
-#define PASS_OVERLAP_GRID 1
-#endif
 // Programmatic dependent launch of passes that are queued one by one.  A pass
 // lets its successor start at once (pass_begin) and waits for its
 // predecessor's memory (pass_wait) before its first access; where the launch
@@ -123,7 +120,7 @@ cudaError_t launch_pass(void (*kern)(P...), int grid, int block, size_t smem, cu
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = st == nullptr && grid <= PASS_OVERLAP_GRID * mmx_sm_count() ? 1 : 0;
+  cfg.numAttrs = st == nullptr && grid <= mmx_sm_count() ? 1 : 0;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, P(args)...);
   return e != cudaSuccess ? e : cudaGetLastError();
 }

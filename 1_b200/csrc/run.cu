@@ -12,9 +12,9 @@
 //    row, one row {t, <m> (user x,y,z), the last maximum torque, min and max
 //    of the user's m_z} is reduced on the device.  With the device dt
 //    controller (mmx_solver_device_control) the whole run is ONE CUDA graph
-//    launch: a WHILE conditional node repeats {row check and reduction,
-//    one RK trial, loop condition} until the device time reaches the stop
-//    time, so no step, trial or row synchronises with the host.
+//    launch: a WHILE conditional node repeats {a row where one is due, one
+//    RK trial, which sets the loop condition} until the device time reaches
+//    the stop time, so no step, trial or row synchronises with the host.
 #include <math.h>
 #include <string.h>
 

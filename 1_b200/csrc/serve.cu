@@ -73,17 +73,21 @@ struct mmx_server {
 };
 
 // resident solves at or below which a batched server steps each solve on
-// its own graph (measured per step, RK4: one solve 0.129 ms alone vs 0.141
-// ms as a batch of one; two solves 0.238 ms one after the other vs 0.159 ms
-// batched)
+// its own graph (measured per step, RK4, grids of 96 x 96 x 2 and 64 x 48 x 4:
+// one solve 0.068 ms alone vs 0.094 ms as a batch of one; two solves 0.131 ms
+// one after the other vs 0.107 ms batched)
 static const int SOLO_MAX = 1;
 
 static double sv_clock(const mmx_server* sv) {
   return std::chrono::duration<double>(std::chrono::steady_clock::now() - sv->t0).count();
 }
 
-// Device bytes mmx_solver_create holds for these parameters, plus the
-// transient real-space kernel and spectrum it builds the octant from.
+// Device bytes that admission counts for these parameters: the spectrum
+// buffer, the state vectors and the kernel octant, plus the transient
+// real-space kernel and spectrum that the octant is built from.  Of a fixed
+// Runge-Kutta solver this is 12 bytes a cell more than mmx_solver_create
+// holds (it keeps no m_new); the rounding of each array to 256 bytes is not
+// counted.
 extern "C" int mmx_server_footprint(const mmx_params* p, size_t* bytes) {
   if (!p || !bytes) { mmx_set_error("null argument"); return MMX_ERR_ARG; }
   int64_t N[3], P[3];
@@ -98,7 +102,7 @@ extern "C" int mmx_server_footprint(const mmx_params* p, size_t* bytes) {
   int64_t ocs = (P[0] / 2 + 1) * (P[1] / 2 + 1) * HZ;
   int vecs = 2;  // m, m1
   if (p->solver == MMX_SOLVER_HEUN) vecs += 1;
-  else if (p->solver == MMX_SOLVER_RK4) vecs += 5;
+  else if (p->solver == MMX_SOLVER_RK4) vecs += 5;  // four stages, and one counted in reserve
   else if (p->solver == MMX_SOLVER_RK23) vecs += 5;
   else vecs += 8;
   int64_t persistent = 3 * cs * 8 + n3 * 4 * vecs + 64 + 6 * ocs * 4;

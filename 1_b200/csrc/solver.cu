@@ -794,7 +794,7 @@ extern "C" int mmx_solver_create(const mmx_params* p, mmx_solver** out) {
   s->is2d = s->P[0] == 1;
   s->n = (int64_t)s->N[0] * s->N[1] * s->N[2];
   int rc = box_plan_init(&s->bp, s->N, s->P);
-  if (rc != MMX_OK) { delete s; mmx_set_error("unsupported padded size (radices 2,3,5,7; <= 16384)"); return rc; }
+  if (rc != MMX_OK) { delete s; mmx_set_error("unsupported padded size (products of 2, 3, 5 and 7; X and Y <= 8192, Z <= 16384)"); return rc; }
   s->HZ = s->bp.HZ;
   s->CS = (int64_t)s->N[0] * s->P[1] * s->HZ;
   set_tableau(s);

@@ -130,8 +130,9 @@ int mmx_solver_energy(mmx_solver* s, double* energy, cudaStream_t stream);
  * their count; successive calls continue the output schedule.  Fixed-step
  * and host-controlled solvers step from the host (no read-back except the
  * adaptive controller's own); with mmx_solver_device_control the whole run
- * is one CUDA graph launch (a WHILE conditional node over {row check, one
- * RK trial, loop condition}) with no host synchronisation until it ends.
+ * is one CUDA graph launch (a WHILE conditional node over {a table row where
+ * one is due, one RK trial, which sets the loop condition}) with no host
+ * synchronisation until it ends.
  * max_steps > 0 caps the steps (device controller: 16 x max_steps trials;
  * MMX_ERR_STATE if the cap ends the run early); 0 = no cap.  Synchronous. */
 int mmx_solver_run(mmx_solver* s, double seconds, float period, float* rows, int max_rows, int* nrows,
