@@ -168,10 +168,13 @@ int mmx_write_odt(const char* path, const float* rows, int nrows, const char* ti
 int mmx_solver_state(mmx_solver* s, double* time, float* dt, float* max_torque, float* step_error, long long* steps);
 /* Sets the applied field (internal units and order) for following steps. */
 int mmx_solver_set_hext(mmx_solver* s, const float hext[3]);
-/* Device pointer of the resident magnetisation (3*N floats).  The program
- * may read and write m through it between calls (ordered with the step's
- * stream): every later call starts from m itself.  Until it is asked for,
- * fixed-step Heun calls take over the transform of m from one another. */
+/* Device pointer of the resident magnetisation (3*N floats), to be read, and
+ * written, between calls (ordered with the step's stream).  Every later call
+ * transforms m itself; until the pointer is asked for, fixed-step Heun calls
+ * take over the transform of m from one another.  rk23 and rkdp take the
+ * first torque of a step from the last stage of the step before (FSAL, as the
+ * reference does): give them a new m with mmx_solver_set_m, which ends that
+ * chain. */
 float* mmx_solver_m_device(mmx_solver* s);
 /* Device address of the solver's last maximum torque (one float). */
 float* mmx_solver_torque_device(mmx_solver* s);
